@@ -346,14 +346,15 @@ mgr_status mgr_level_create(const mgr_level_desc *desc, int device, void *stream
         L->ref.alloc(L->N, L->stream);
         L->warped.alloc(L->N, L->stream);
         L->minmax.alloc(2, L->stream);
-        L->mmpart.alloc(1024, L->stream);
+        L->mmpart.alloc(prefilter_x_blocks(d.dim, L->n[0], L->n[1], L->n[2]), L->stream);
         L->params.alloc(L->nparams, L->stream);
         if (d.dim == 3) L->params_f.alloc(L->nparams, L->stream);
         L->grad_total.alloc(L->nparams, L->stream);
         L->scalars.alloc(SC_NSLOTS, L->stream);
         L->costs.alloc(2, L->stream);
         L->means.alloc(2, L->stream);
-        L->mpart.alloc(2 * 1024, L->stream);
+        ck(cudaMemsetAsync(L->means.p, 0, 2 * sizeof(double), L->stream), "memset");
+        if (d.cost == MGR_COST_NCC) L->mpart.alloc(2 * 1024, L->stream);
         L->counters.alloc(8, L->stream);
         ck(cudaMemsetAsync(L->counters.p, 0, 8 * sizeof(unsigned), L->stream), "memset");
         ck(cudaMemsetAsync(L->scalars.p, 0, SC_NSLOTS * sizeof(double), L->stream), "memset");
@@ -391,47 +392,23 @@ mgr_status mgr_level_csize(const mgr_level *lvl, int csize[3], size_t *nparams)
 
 }  // extern "C"
 
-// means of the two images in double (NCC provisional centres): per-block
-// partial sums (blockIdx.y selects the image), then a fixed-order final sum
-__global__ void __launch_bounds__(256) k_mean_part(const float *__restrict__ a, const float *__restrict__ b, size_t n,
-                                                   double *part)
-{
-    __shared__ double red[8];
-    const float *img = blockIdx.y ? b : a;
-    double v[1] = {0.0};
-    for (size_t i = blockIdx.x * size_t(256) + threadIdx.x; i < n; i += size_t(gridDim.x) * 256) v[0] += img[i];
-    block_sum<1>(v, red);
-    if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = v[0];
-}
-
-__global__ void __launch_bounds__(256) k_mean_final(const double *part, int nb, size_t n, double *out)
-{
-    __shared__ double red[8];
-    double v[1] = {0.0};
-    for (int i = threadIdx.x; i < nb; i += 256) v[0] += part[blockIdx.x * nb + i];
-    block_sum<1>(v, red);
-    if (threadIdx.x == 0) out[blockIdx.x] = v[0] / double(n);
-}
-
 namespace mgr {
 
-// copy the images into the level, clamp bounds, centres and the prefilter,
-// all queued on the level's stream (the sources must stay valid until the
-// stream reaches them)
+// the images into the level: the source's coefficients and clamp bounds, the
+// reference and (for NCC, whose sums are taken about them) both means, all
+// queued on the level's stream (the sources must stay valid until the stream
+// reaches them)
 void level_set_images_async(mgr_level *L, const float *d_src, const float *d_ref)
 {
     ck(cudaSetDevice(L->device), "cudaSetDevice");
     cudaStream_t st = L->stream;
-    ck(cudaMemcpyAsync(L->coef.p, d_src, L->N * sizeof(float), cudaMemcpyDeviceToDevice, st), "copy src");
-    if (d_ref != L->ref.p)
-        ck(cudaMemcpyAsync(L->ref.p, d_ref, L->N * sizeof(float), cudaMemcpyDeviceToDevice, st), "copy ref");
-    const int nb = int(std::min<size_t>(1024, (L->N + 255) / 256));
-    launch_minmax(L->coef.p, L->N, L->mmpart.p, nb, L->counters.p + 4, L->minmax.p, st);
-    k_mean_part<<<dim3(nb, 2), 256, 0, st>>>(L->coef.p, L->ref.p, L->N, L->mpart.p);
-    k_mean_final<<<2, 256, 0, st>>>(L->mpart.p, nb, L->N, L->means.p);
-    count_launch(2);
-    launch_prefilter(L->coef.p, L->d.dim, L->n[0], L->n[1], L->n[2], st);
-    launch_pad_mirror(L->coef.p, L->coef_pad.p, L->d.dim, L->n[0], L->n[1], L->n[2], st);
+    float *ref_out = d_ref != L->ref.p ? L->ref.p : nullptr;
+    if (L->d.cost == MGR_COST_NCC)
+        launch_image_means(d_src, d_ref, ref_out, L->N, L->mpart.p, L->counters.p + 5, L->means.p, st);
+    else if (ref_out)
+        ck(cudaMemcpyAsync(ref_out, d_ref, L->N * sizeof(float), cudaMemcpyDeviceToDevice, st), "copy ref");
+    launch_prefilter(d_src, L->coef.p, L->coef_pad.p, L->d.dim, L->n[0], L->n[1], L->n[2], L->mmpart.p,
+                     L->counters.p + 4, L->minmax.p, st);
     check_launch("set_images kernels");
     L->images_set = true;
 }

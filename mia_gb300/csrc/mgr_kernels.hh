@@ -33,13 +33,18 @@ cudaError_t host_malloc_pinned(void **p, size_t bytes);
 // evaluation then makes no driver call for it
 void raise_smem_limit(const void *kernel, size_t bytes);
 
-void launch_prefilter(float *img, int dim, int nx, int ny, int nz, cudaStream_t st);
-// padded copy with the mirror fold applied in the halo (layout of coef_pad)
-void launch_pad_mirror(const float *img, float *pad, int dim, int nx, int ny, int nz, cudaStream_t st);
+// the B-spline coefficients of src and their mirror-padded copy (layout of
+// coef_pad), and src's minimum and maximum: minmax[0..1], mmpart holds
+// prefilter_x_blocks() entries, *counter is 0 before and after
+void launch_prefilter(const float *src, float *coef, float *pad, int dim, int nx, int ny, int nz, float2 *mmpart,
+                      unsigned *counter, float *minmax, cudaStream_t st);
+int prefilter_x_blocks(int dim, int nx, int ny, int nz);
+// the means of src and ref in out[0..1] (part: 2 x 1024 doubles, *counter as
+// above), ref copied to ref_out when given
+void launch_image_means(const float *src, const float *ref, float *ref_out, size_t n, double *part, unsigned *counter,
+                        double *out, cudaStream_t st);
 // the padded image's size in floats
 size_t pad_floats(int dim, int nx, int ny, int nz);
-void launch_minmax(const float *img, size_t n, float2 *part, int nblocks, unsigned int *counter,
-                   float *out, cudaStream_t st);
 
 // 3D: tensor map of the padded copy (box 64 x 16 x 1 floats, the
 // warp kernel's shared-memory ring planes); false if the driver offers no
@@ -71,7 +76,7 @@ struct EvalArgs {
     float *partial;        // per tile adjoint footprint partials
     int slot;              // floats per tile slot
     double *tile_sums;     // per warp tile: 5 doubles
-    unsigned int *counters;// [0] warp, [1] gather, [2] penalty value
+    unsigned int *counters;// [0] warp, [1] gather, [4] [5] image set-up, [6] [7] status flags
     double *scalars;       // SC_* slots
     // penalty
     int has_penalty;

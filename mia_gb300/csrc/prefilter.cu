@@ -5,7 +5,7 @@
 // (mia/core/boundary_conditions.cc:62-103) and CMirrorOnBoundary
 // (mia/core/splinebc/bc.cc:67-88): x lines, then y lines, then z lines, each
 // line filtered with the reference's operations (in float, see
-// k_prefilter_lines) and stored back as float.
+// prefilter_line) and stored back as float.
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -14,180 +14,400 @@
 
 namespace mgr {
 
-// One block of PF_NT threads owns up to `lb` (<= 64) lines of length n,
-// staged in shared memory (odd pitch) by independent coalesced loads: along
-// the line for x lines, across the lines (consecutive x) for y and z lines.
-// One thread per line runs the recursion, then the block stores the lines
-// back the way it loaded them.  The reference filters each line in a double
-// buffer; FP64 arithmetic runs at a small fraction of the FP32 rate on this
-// GPU, so the recursion runs in float with the same operations: the pole's
-// magnitude (0.268) damps the rounding of every step, and the result differs
-// from the double filter by a few float ulp of the coefficient (the parity
-// tests bound the warped image and costs, which read these coefficients, at
-// 1e-5 / 1e-4).
-// axis 0: lines along x (rows, consecutive rows per block);
-// axis 1/2: lines along y/z (columns of consecutive x per block).
+// One pass filters the lines of one axis; a block of PF_NT threads owns lb
+// (<= 32) of them, staged in shared memory.  The loads come scaled by lambda
+// (the filter's first step) and cover whole rows: along the line for x lines
+// (a warp per line), across the lines (consecutive x) for y and z lines.  One
+// thread per line then runs the recursion in two sweeps with the running
+// value in a register, and the block stores the lines back.
+//
+// The passes also take what used to be passes of their own over the images:
+// the first (x) reads the caller's image (no copy of it is made) and finds
+// its minimum and maximum, the last writes the mirror-padded copy beside the
+// coefficients.  What bounds a pass is the latency of load, recursion and
+// store, one after the other in a block; blocks of 32 lines keep three to
+// five of them on an SM.  New images on a kept level and the evaluation
+// after them, 192x192x128 SSD: 325 us with a kernel each for copy, bounds,
+// means, three passes and padding, 188 us so.
+//
+// The reference filters each line in a double buffer; FP64 arithmetic runs
+// at a small fraction of the FP32 rate on this GPU, so the recursion runs in
+// float with the same operations: the pole's magnitude (0.268) damps the
+// rounding of every step, and the result differs from the double filter by a
+// few float ulp of the coefficient (the parity tests bound the warped image
+// and costs, which read these coefficients, at 1e-5 / 1e-4).
 constexpr int PF_NT = 256;
+constexpr int PF_NW = PF_NT / 32;
+constexpr int PF_BATCH = 8;   // line values a thread holds in registers at a time
 
-__global__ void __launch_bounds__(PF_NT) k_prefilter_lines(float *__restrict__ img, int nx, int ny, int nz,
-                                                           int axis, int lb)
+struct PrefilterPass {
+    const float *in;
+    float *out;
+    int n;               // line length
+    int nlines;          // x pass: all lines; y and z passes: the image's x size
+    int lb;              // lines per block, a power of two <= 32
+    size_t estride;      // elements between neighbours of a line
+    size_t bstride;      // y and z passes: elements between blockIdx.y groups
+    // x pass: minimum and maximum of the input
+    float2 *mmpart;      // one per block
+    unsigned *counter;
+    float *minmax;
+    // last pass: the mirror-padded copy (null: none)
+    float *pad;
+    size_t pad_estride;  // its elements between neighbours of a line
+    int pad_pitch;
+    int ny;              // 3D: rows of a plane, blockIdx.y is the row; 2D: 0
+};
+
+// the line at c (elements s apart), already scaled by lambda
+__device__ __forceinline__ void prefilter_line(float *c, int n, int s)
+{
+    const float p = float(1.7320508075688772 - 2.0);   // sqrt(3) - 2
+    // mirror initial value: sum of (p^k + p^(2n-2-k)) c[k], k ascending; the
+    // terms whose powers are below the float range add nothing, and from the
+    // first of them on all following ones (short lines have no such term)
+    float zn = p;
+    const float iz = 1.0f / p;
+    float z2n = powf(p, float(n - 1));
+    float sum = c[0] + z2n * c[(n - 1) * s];
+    z2n *= z2n * iz;
+    for (int k0 = 1; k0 < n - 1; k0 += PF_BATCH) {
+        float v[PF_BATCH];
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 + j < n - 1 ? c[(k0 + j) * s] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j)
+            if (k0 + j < n - 1) {
+                sum += (zn + z2n) * v[j];
+                zn *= p;
+                z2n *= iz;
+            }
+        if (zn == 0.0f && z2n == 0.0f) break;
+    }
+    float prev = sum / (1.0f - zn * zn), before = prev;
+    c[0] = prev;
+    for (int k0 = 1; k0 < n; k0 += PF_BATCH) {
+        float v[PF_BATCH];
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 + j < n ? c[(k0 + j) * s] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j)
+            if (k0 + j < n) {
+                before = prev;
+                prev = v[j] + p * prev;
+                v[j] = prev;
+            }
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j)
+            if (k0 + j < n) c[(k0 + j) * s] = v[j];
+    }
+    float next = (p / (p * p - 1.0f)) * (p * before + prev);
+    c[(n - 1) * s] = next;
+    for (int k0 = n - 2; k0 >= 0; k0 -= PF_BATCH) {
+        float v[PF_BATCH];
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 - j >= 0 ? c[(k0 - j) * s] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j)
+            if (k0 - j >= 0) {
+                next = p * (next - v[j]);
+                v[j] = next;
+            }
+#pragma unroll
+        for (int j = 0; j < PF_BATCH; ++j)
+            if (k0 - j >= 0) c[(k0 - j) * s] = v[j];
+    }
+}
+
+__device__ __forceinline__ float prefilter_scale(float v)
+{
+    return v * float(2.0 - (1.7320508075688772 - 2.0) - 1.0 / (1.7320508075688772 - 2.0));
+}
+
+// x lines.  The minimum and maximum follow the reference's rule that the
+// lower clamp bound is at most 0 (interpolator.cxx:109-112); the last block
+// to finish reduces the blocks' values.
+__global__ void __launch_bounds__(PF_NT) k_prefilter_x(PrefilterPass a)
 {
     extern __shared__ float sl[];
-    const int t = threadIdx.x;
-    const size_t nxy = size_t(nx) * ny;
-    int n, nl;
-    size_t base, lstride, estride;
-    if (axis == 0) {
-        n = nx;
-        const int l0 = blockIdx.x * lb;
-        nl = min(lb, ny * nz - l0);
-        base = size_t(l0) * nx;
-        lstride = size_t(nx);
-        estride = 1;
-    } else {
-        const int xb = blockIdx.x * lb;
-        const int other = blockIdx.y;
-        n = (axis == 1) ? ny : nz;
-        base = (axis == 1) ? size_t(other) * nxy + xb : size_t(other) * nx + xb;
-        lstride = 1;
-        estride = (axis == 1) ? size_t(nx) : nxy;
-        nl = min(lb, nx - xb);
-    }
-    const int pitch = n | 1;
-    const bool along = axis == 0;
-#pragma unroll 4
-    for (int e = t; e < nl * n; e += PF_NT) {
-        const int l = along ? e / n : e % nl, k = along ? e % n : e / nl;
-        sl[l * pitch + k] = img[base + l * lstride + k * estride];
-    }
-    __syncthreads();
-    if (t < nl && n >= 2) {
-        float *c = sl + t * pitch;
-        const float p = float(1.7320508075688772 - 2.0);   // sqrt(3) - 2
-        const float lambda = float(2.0 - (1.7320508075688772 - 2.0) - 1.0 / (1.7320508075688772 - 2.0));
-        for (int k = 0; k < n; ++k) c[k] *= lambda;
-        // mirror initial value: sum of (p^k + p^(2n-2-k)) c[k]; the powers
-        // below the float range contribute nothing
-        float zn = p;
-        const float iz = 1.0f / p;
-        float z2n = powf(p, float(n - 1));
-        float sum = c[0] + z2n * c[n - 1];
-        z2n *= z2n * iz;
-        for (int k = 1; k < n - 1; ++k) {
-            sum += (zn + z2n) * c[k];
-            zn *= p;
-            z2n *= iz;
-        }
-        c[0] = sum / (1.0f - zn * zn);
-        for (int k = 1; k < n; ++k) c[k] += p * c[k - 1];
-        c[n - 1] = (p / (p * p - 1.0f)) * (p * c[n - 2] + c[n - 1]);
-        for (int k = n - 2; k >= 0; --k) c[k] = p * (c[k + 1] - c[k]);
-    }
-    __syncthreads();
-    for (int e = t; e < nl * n; e += PF_NT) {
-        const int l = along ? e / n : e % nl, k = along ? e % n : e / nl;
-        img[base + l * lstride + k * estride] = sl[l * pitch + k];
-    }
-}
-
-// min/max of the source image with the reference's rule that the lower
-// clamp bound is at most 0 (interpolator.cxx:109-112).  Per-block results
-// go to `part`; the last block to finish reduces them in a fixed order.
-__global__ void __launch_bounds__(256) k_minmax(const float *__restrict__ img, size_t n, float2 *part,
-                                                unsigned int *counter, float *out_minmax)
-{
-    __shared__ float smin[256], smax[256];
+    __shared__ float2 wmm[PF_NW];
     __shared__ bool last;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int n = a.n, pitch = n | 1;
+    const int l0 = blockIdx.x * a.lb, nl = min(a.lb, a.nlines - l0);
+    const float *src = a.in + size_t(l0) * n;
     float mn = INFINITY, mx = -INFINITY;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const float v = img[i];
-        mn = fminf(mn, v);
-        mx = fmaxf(mx, v);
-    }
-    smin[threadIdx.x] = mn;
-    smax[threadIdx.x] = mx;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            smin[threadIdx.x] = fminf(smin[threadIdx.x], smin[threadIdx.x + o]);
-            smax[threadIdx.x] = fmaxf(smax[threadIdx.x], smax[threadIdx.x + o]);
+    for (int l = w; l < nl; l += PF_NW) {
+        const float *row = src + size_t(l) * n;
+        float *c = sl + l * pitch;
+        for (int k0 = lane; k0 < n; k0 += 32 * PF_BATCH) {
+            float v[PF_BATCH];
+#pragma unroll
+            for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 + 32 * j < n ? __ldg(row + k0 + 32 * j) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < PF_BATCH; ++j)
+                if (k0 + 32 * j < n) {
+                    mn = fminf(mn, v[j]);
+                    mx = fmaxf(mx, v[j]);
+                    c[k0 + 32 * j] = prefilter_scale(v[j]);
+                }
         }
-        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = make_float2(smin[0], smax[0]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane == 0) wmm[w] = make_float2(mn, mx);
+    __syncthreads();
+    if (t < nl) prefilter_line(sl + t * pitch, n, 1);
+    if (t == PF_NT - 1) {   // a thread without a line (lb <= 32)
+        for (int k = 0; k < PF_NW; ++k) {
+            mn = fminf(mn, wmm[k].x);
+            mx = fmaxf(mx, wmm[k].y);
+        }
+        a.mmpart[blockIdx.x] = make_float2(mn, mx);
         __threadfence();
-        last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+        last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        float a = INFINITY, b = -INFINITY;
-        for (unsigned i = 0; i < gridDim.x; ++i) {
-            const volatile float *v = reinterpret_cast<volatile float *>(part) + 2 * i;
-            a = fminf(a, v[0]);
-            b = fmaxf(b, v[1]);
+    float *dst = a.out + size_t(l0) * n;
+    for (int l = w; l < nl; l += PF_NW) {
+        float *row = dst + size_t(l) * n;
+        const float *c = sl + l * pitch;
+#pragma unroll 4
+        for (int k = lane; k < n; k += 32) row[k] = c[k];
+    }
+    if (!last) return;
+    __threadfence();
+    mn = INFINITY;
+    mx = -INFINITY;
+    for (unsigned i = t; i < gridDim.x; i += PF_NT) {
+        const float2 v = __ldcg(a.mmpart + i);
+        mn = fminf(mn, v.x);
+        mx = fmaxf(mx, v.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane == 0) wmm[w] = make_float2(mn, mx);
+    __syncthreads();
+    if (t == 0) {
+        for (int k = 0; k < PF_NW; ++k) {
+            mn = fminf(mn, wmm[k].x);
+            mx = fmaxf(mx, wmm[k].y);
         }
-        if (0.0f < a) a = 0.0f;
-        out_minmax[0] = a;
-        out_minmax[1] = b;
-        *counter = 0;
+        if (0.0f < mn) mn = 0.0f;
+        a.minmax[0] = mn;
+        a.minmax[1] = mx;
+        *a.counter = 0;
     }
 }
 
-// lines per block: at most 64 and 64 KB of staged lines, fewer while the
+// y or z lines of lb consecutive x, in place; PAD: the mirror-padded copy is
+// written from the staged lines, every image of a line's elements along the
+// line, of the row across the plane's rows (3D) and of the columns within
+// PAD_H of the image's x borders
+template <bool PAD>
+__global__ void __launch_bounds__(PF_NT) k_prefilter_cols(PrefilterPass a)
+{
+    extern __shared__ float sl[];
+    __shared__ int images[2 * PAD_H + 1];   // PAD, 3D: the padded rows that hold this row
+    __shared__ int nimages;
+    const int t = threadIdx.x, n = a.n, lb = a.lb;
+    const int xb = blockIdx.x * lb, nl = min(lb, a.nlines - xb);
+    const int l = t & (lb - 1), g = t / lb, ng = PF_NT / lb;
+    const size_t base = size_t(blockIdx.y) * a.bstride + xb + l;
+    if (l < nl)
+        for (int k0 = g; k0 < n; k0 += ng * PF_BATCH) {
+            float v[PF_BATCH];
+#pragma unroll
+            for (int j = 0; j < PF_BATCH; ++j)
+                v[j] = k0 + ng * j < n ? __ldcg(a.in + base + size_t(k0 + ng * j) * a.estride) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < PF_BATCH; ++j)
+                if (k0 + ng * j < n) sl[(k0 + ng * j) * lb + l] = prefilter_scale(v[j]);
+        }
+    if (PAD && t >= PF_NT - 32) {   // the last warp has no line
+        const int j = t & 31, yp = j < PAD_H ? j - PAD_H : a.ny + j - PAD_H;
+        const bool hit = a.ny > 0 && mirror_fold(yp, a.ny) == int(blockIdx.y);
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) images[1 + __popc(m & ((1u << j) - 1u))] = yp + PAD_H;
+        if (j == 0) {
+            images[0] = a.ny > 0 ? int(blockIdx.y) + PAD_H : 0;
+            nimages = 1 + __popc(m);
+        }
+    }
+    __syncthreads();
+    if (t < nl) prefilter_line(sl + t, n, lb);
+    __syncthreads();
+    if (l < nl) {
+#pragma unroll 4
+        for (int k = g; k < n; k += ng) a.out[base + size_t(k) * a.estride] = sl[k * lb + l];
+    }
+    if (!PAD) return;
+    const int nimg = nimages, np = n + 2 * PAD_H, nx = a.nlines;
+    if (l < nl)
+#pragma unroll 2
+        for (int kp = g; kp < np; kp += ng) {
+            const float v = sl[mirror_fold(kp - PAD_H, n) * lb + l];
+            float *row = a.pad + size_t(kp) * a.pad_estride + PAD_H + xb + l;
+            for (int r = 0; r < nimg; ++r) row[size_t(images[r]) * a.pad_pitch] = v;
+        }
+    // the x halo's columns whose source lies in this block, and the zeros
+    // that fill the padded rows to their pitch (written by the last block)
+    const int j = t & 31, w = t >> 5;
+    const int xp = j < PAD_H ? j - PAD_H : nx + j - PAD_H;
+    const int xs = mirror_fold(xp, nx) - xb;
+    const bool hit = unsigned(xs) < unsigned(nl);
+    const int xz = nx + 2 * PAD_H + j;
+    const bool zero = xb + nl == nx && xz < a.pad_pitch;
+    if (!__any_sync(0xffffffffu, hit || zero)) return;
+    for (int kp = w; kp < np; kp += PF_NW) {
+        const float v = hit ? sl[mirror_fold(kp - PAD_H, n) * lb + xs] : 0.0f;
+        float *row = a.pad + size_t(kp) * a.pad_estride;
+        for (int r = 0; r < nimg; ++r) {
+            float *q = row + size_t(images[r]) * a.pad_pitch;
+            if (hit) q[xp + PAD_H] = v;
+            if (zero) q[xz] = 0.0f;
+        }
+    }
+}
+
+// lines per block: at most 32 and 64 KB of staged lines, fewer while the
 // launch would have less than two blocks per SM (the recursion of the
 // block's lines is its critical path)
 static int lines_per_block(int n, int lines_total, int blocks_per_line_group)
 {
-    int lb = 64;
+    int lb = 32;
     while (lb > 1 && size_t(lb) * (n | 1) * sizeof(float) > 64 * 1024) lb >>= 1;
     const int nsm = device_sm_count();
     while (lb > 8 && size_t((lines_total + lb - 1) / lb) * blocks_per_line_group < size_t(2 * nsm)) lb >>= 1;
     return lb;
 }
 
-void launch_prefilter(float *img, int dim, int nx, int ny, int nz, cudaStream_t st)
+int prefilter_x_blocks(int dim, int nx, int ny, int nz)
+{
+    const int nlines = ny * (dim == 3 ? nz : 1);
+    const int lb = lines_per_block(nx, nlines, 1);
+    return (nlines + lb - 1) / lb;
+}
+
+void launch_prefilter(const float *src, float *coef, float *pad, int dim, int nx, int ny, int nz, float2 *mmpart,
+                      unsigned *counter, float *minmax, cudaStream_t st)
 {
     if (dim == 2) nz = 1;
-    // (a per-device setting: set on every call, once per level)
-    cudaFuncSetAttribute(k_prefilter_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    {
-        const int nlines = ny * nz;
-        const int lb = lines_per_block(nx, nlines, 1);
-        const size_t sm = size_t(lb) * (nx | 1) * sizeof(float);
-        k_prefilter_lines<<<(nlines + lb - 1) / lb, PF_NT, sm, st>>>(img, nx, ny, nz, 0, lb);
-        count_launch();
-    }
-    {
-        const int lb = lines_per_block(ny, nx, nz);
-        const size_t sm = size_t(lb) * (ny | 1) * sizeof(float);
-        k_prefilter_lines<<<dim3((nx + lb - 1) / lb, nz), PF_NT, sm, st>>>(img, nx, ny, nz, 1, lb);
-        count_launch();
-    }
-    if (dim == 3 && nz > 1) {
-        const int lb = lines_per_block(nz, nx, ny);
-        const size_t sm = size_t(lb) * (nz | 1) * sizeof(float);
-        k_prefilter_lines<<<dim3((nx + lb - 1) / lb, ny), PF_NT, sm, st>>>(img, nx, ny, nz, 2, lb);
+    PrefilterPass a = {};
+    a.in = src;
+    a.out = coef;
+    a.n = nx;
+    a.nlines = ny * nz;
+    a.lb = lines_per_block(nx, a.nlines, 1);
+    a.mmpart = mmpart;
+    a.counter = counter;
+    a.minmax = minmax;
+    size_t sm = size_t(a.lb) * (nx | 1) * sizeof(float);
+    raise_smem_limit(reinterpret_cast<const void *>(k_prefilter_x), sm);
+    k_prefilter_x<<<(a.nlines + a.lb - 1) / a.lb, PF_NT, sm, st>>>(a);
+    count_launch();
+    const size_t nxy = size_t(nx) * ny;
+    for (int axis = 1; axis < dim; ++axis) {
+        const bool last = axis == dim - 1;
+        const int other = axis == 1 ? nz : ny;
+        a.in = coef;
+        a.n = axis == 1 ? ny : nz;
+        a.nlines = nx;
+        a.lb = lines_per_block(a.n, nx, other);
+        a.estride = axis == 1 ? size_t(nx) : nxy;
+        a.bstride = axis == 1 ? nxy : size_t(nx);
+        sm = size_t(a.lb) * a.n * sizeof(float);
+        const dim3 grid((nx + a.lb - 1) / a.lb, other);
+        if (last) {
+            a.pad = pad;
+            a.pad_pitch = pad_pitch(nx);
+            a.ny = dim == 3 ? ny : 0;
+            a.pad_estride = dim == 3 ? size_t(a.pad_pitch) * (ny + 2 * PAD_H) : size_t(a.pad_pitch);
+            raise_smem_limit(reinterpret_cast<const void *>(k_prefilter_cols<true>), sm);
+            k_prefilter_cols<true><<<grid, PF_NT, sm, st>>>(a);
+        } else {
+            raise_smem_limit(reinterpret_cast<const void *>(k_prefilter_cols<false>), sm);
+            k_prefilter_cols<false><<<grid, PF_NT, sm, st>>>(a);
+        }
         count_launch();
     }
 }
 
-__global__ void k_pad_mirror(const float *__restrict__ img, float *__restrict__ pad, int nx, int ny, int nz,
-                             int pitch, int rows, int hz, size_t total)
+// The means of the two images in double (NCC provisional centres), and the
+// copy of the reference into the level in the same pass.  Per-block partial
+// sums in a fixed order, added by the last block.  FP64 instructions bound
+// it (two additions per voxel at 1/64 of the FP32 rate), so a value is
+// widened to double with integer instructions instead of a conversion on the
+// same pipe.
+__device__ __forceinline__ double widen(float x)
 {
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const int px = int(i % pitch);
-        const size_t r = i / pitch;
-        const int py = int(r % rows), pz = int(r / rows);
-        const int x = px - PAD_H, y = py - PAD_H, z = pz - hz;
-        float v = 0.0f;
-        if (x < nx + PAD_H) {
-            const int gx = mirror_fold(x, nx), gy = mirror_fold(y, ny), gz = mirror_fold(z, nz);
-            v = img[(size_t(gz) * ny + gy) * nx + gx];
+    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    if (m - 0x00800000u < 0x7f000000u)   // a normal number: the exponent's bias moves by 1023 - 127
+        return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), int(u << 29));
+    return m == 0u ? __hiloint2double(int(u), 0) : double(x);
+}
+
+__global__ void __launch_bounds__(256) k_image_means(const float *__restrict__ src, const float *__restrict__ ref,
+                                                     float *__restrict__ ref_out, size_t n, double *part,
+                                                     unsigned *counter, double *out)
+{
+    __shared__ double red[16];
+    __shared__ bool last;
+    double v[2] = {0.0, 0.0};
+    const size_t step = size_t(gridDim.x) * 256;
+    for (size_t i0 = blockIdx.x * size_t(256) + threadIdx.x; i0 < n; i0 += 4 * step) {
+        float a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const size_t i = i0 + j * step;
+            a[j] = i < n ? __ldg(src + i) : 0.0f;
+            b[j] = i < n ? __ldcg(ref + i) : 0.0f;
         }
-        pad[i] = v;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const size_t i = i0 + j * step;
+            if (i < n) {
+                v[0] += widen(a[j]);
+                v[1] += widen(b[j]);
+                if (ref_out) ref_out[i] = b[j];
+            }
+        }
     }
+    block_sum<2>(v, red);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = v[0];
+        part[gridDim.x + blockIdx.x] = v[1];
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    v[0] = v[1] = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += 256) {
+        v[0] += __ldcg(part + i);
+        v[1] += __ldcg(part + gridDim.x + i);
+    }
+    block_sum<2>(v, red);
+    if (threadIdx.x == 0) {
+        out[0] = v[0] / double(n);
+        out[1] = v[1] / double(n);
+        *counter = 0;
+    }
+}
+
+void launch_image_means(const float *src, const float *ref, float *ref_out, size_t n, double *part, unsigned *counter,
+                        double *out, cudaStream_t st)
+{
+    const int nb = int(std::min<size_t>(1024, (n + 255) / 256));
+    k_image_means<<<nb, 256, 0, st>>>(src, ref, ref_out, n, part, counter, out);
+    count_launch();
 }
 
 bool encode_pad_tmap(CUtensorMap *map, const float *pad, int nx, int ny, int nz)
@@ -217,23 +437,6 @@ size_t pad_floats(int dim, int nx, int ny, int nz)
 {
     const int planes = dim == 3 ? nz + 2 * PAD_H : 1;
     return size_t(pad_pitch(nx)) * (ny + 2 * PAD_H) * planes;
-}
-
-void launch_pad_mirror(const float *img, float *pad, int dim, int nx, int ny, int nz, cudaStream_t st)
-{
-    if (dim == 2) nz = 1;
-    const size_t total = pad_floats(dim, nx, ny, nz);
-    const int nb = int(std::min<size_t>(4096, (total + 255) / 256));
-    k_pad_mirror<<<nb, 256, 0, st>>>(img, pad, nx, ny, nz, pad_pitch(nx), ny + 2 * PAD_H, dim == 3 ? PAD_H : 0,
-                                     total);
-    count_launch();
-}
-
-void launch_minmax(const float *img, size_t n, float2 *part, int nblocks, unsigned int *counter,
-                   float *out, cudaStream_t st)
-{
-    k_minmax<<<nblocks, 256, 0, st>>>(img, n, part, counter, out);
-    count_launch();
 }
 
 }  // namespace mgr
