@@ -130,7 +130,7 @@ mgr_status mgr_level_evaluate(mgr_level *lvl, const double *params, double *grad
 /* How mgr_level_evaluate moves the caller's host data.  *in_place = 1: the
    level's device reads and writes pageable host memory coherently through
    the host's page tables (Grace-based systems such as GB300) and the level
-   is a 3D split-path level; the kernels read `params` and write the
+   is a split-path level; the kernels read `params` and write the
    gradients where the caller holds them, with no staged copy.  *in_place =
    0: the call stages them through device buffers.  MGR_HOST_COPY=1 in the
    environment when the level is created keeps the staged copies.  The

@@ -228,7 +228,7 @@ void level_set_grid(mgr_level *L, const int csize[3], const int tile[3])
     L->grad_image.release();
     L->grad_penalty.release();
     L->params.alloc(L->nparams, L->stream);
-    if (D == 3) L->params_f.alloc(L->nparams, L->stream);
+    L->params_f.alloc(L->nparams, L->stream);
     L->grad_total.alloc(L->nparams, L->stream);
     L->partial.release();
     L->tile_sums.release();
@@ -263,7 +263,7 @@ mgr_level *level_create_on_images(const mgr_level *S, const int csize[3], cudaSt
     L->images_from = S;
     L->images_set = true;
     L->params.alloc(L->nparams, st);
-    if (D == 3) L->params_f.alloc(L->nparams, st);
+    L->params_f.alloc(L->nparams, st);
     L->grad_total.alloc(L->nparams, st);
     L->scalars.alloc(SC_NSLOTS, st);
     L->costs.alloc(2, st);
@@ -348,7 +348,7 @@ mgr_status mgr_level_create(const mgr_level_desc *desc, int device, void *stream
         L->minmax.alloc(2, L->stream);
         L->mmpart.alloc(prefilter_x_blocks(d.dim, L->n[0], L->n[1], L->n[2]), L->stream);
         L->params.alloc(L->nparams, L->stream);
-        if (d.dim == 3) L->params_f.alloc(L->nparams, L->stream);
+        L->params_f.alloc(L->nparams, L->stream);
         L->grad_total.alloc(L->nparams, L->stream);
         L->scalars.alloc(SC_NSLOTS, L->stream);
         L->costs.alloc(2, L->stream);
@@ -449,7 +449,7 @@ static void upload_params(mgr_level *L, const double *params)
 static void run_image_term(mgr_level *L, EvalArgs &a, bool with_gradient);
 
 // Evaluation on a device that reads and writes the caller's host memory
-// coherently (3D split path): the parameter conversion reads the caller's
+// coherently (split path): the parameter conversion reads the caller's
 // parameters, the gather writes the gradients into the caller's buffers and
 // the costs and status flags into the level's pinned buffer; no staged copy
 // and one synchronisation.  Non-finite parameters are found by the
@@ -527,8 +527,8 @@ static void run_image_term(mgr_level *L, EvalArgs &a, bool with_gradient)
         return;
     }
     L->record(0);
-    // 3D: the cost is finalised after the warp kernel (its blocks end earlier)
-    a.defer_cost = L->d.dim == 3;
+    // the cost is finalised after the warp kernel (its blocks end earlier)
+    a.defer_cost = L->can_defer();
     {
         NvtxRange r(L->d.dim == 3 ? "k_warp3" : "k_warp (2D)");
         launch_warp(a, st);
@@ -594,7 +594,7 @@ mgr_status mgr_level_evaluate(mgr_level *lvl, const double *params, double *grad
     return guarded([&] {
         if (!lvl->images_set) throw StateError("set_images must be called before evaluate");
         ck(cudaSetDevice(lvl->device), "cudaSetDevice");
-        if (lvl->coherent && lvl->d.dim == 3 && lvl->path == MGR_PATH_SPLIT) {
+        if (lvl->coherent && lvl->path == MGR_PATH_SPLIT) {
             evaluate_in_place(lvl, params, grad_total, grad_image, grad_penalty, cost_image, cost_penalty);
             return;
         }
@@ -633,7 +633,7 @@ mgr_status mgr_level_evaluate(mgr_level *lvl, const double *params, double *grad
 mgr_status mgr_level_host_access(const mgr_level *lvl, int *in_place)
 {
     if (!lvl || !in_place) return fail(MGR_ERR_ARG, "null argument");
-    *in_place = lvl->coherent && lvl->d.dim == 3 && lvl->path == MGR_PATH_SPLIT ? 1 : 0;
+    *in_place = lvl->coherent && lvl->path == MGR_PATH_SPLIT ? 1 : 0;
     return MGR_OK;
 }
 
@@ -646,7 +646,7 @@ mgr_status mgr_level_value(mgr_level *lvl, const double *params, double *cost_im
         ck(cudaSetDevice(lvl->device), "cudaSetDevice");
         upload_params(lvl, params);
         EvalArgs a = lvl->args();
-        a.defer_cost = lvl->d.dim == 3;   // the cost is finalised after the warp kernel
+        a.defer_cost = lvl->can_defer();   // the cost is finalised after the warp kernel
         launch_warp(a, lvl->stream);
         launch_gather(a, 0, lvl->stream);
         check_launch("value kernels");

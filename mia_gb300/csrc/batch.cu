@@ -6,7 +6,7 @@
 // All pairs advance in lock step.  One step evaluates the cost+gradient of
 // every unfinished pair at the point its minimizer proposes:
 //   k_min_propose  (blocks x pairs) the minimizer's next evaluation point
-//                  (and, in 3D, its float copy that the warp kernel reads)
+//                  (and its float copy that the warp kernel reads)
 //   warp, adjoint, gather of the split path over a work list of
 //                  (pair, tile) / (pair, block) items covering all pairs
 //   k_min_update   (blocks x pairs) the minimizer's decision
@@ -62,7 +62,7 @@ struct PairVec {
     double *x, *g, *xt, *gt;
     const double *costs;   // {image, penalty} at xt
     int n;
-    float *xf;             // 3D: the level's float copy of xt (written with xt), else null
+    float *xf;             // the level's float copy of xt (written with xt)
 };
 
 // The minimizer kernels spread each pair's vectors over blocks of MCH
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(MT) k_min_propose(MinState *st, const PairVec 
         for (int i = i0 + tid; i < i1; i += MT) {
             const double xi = v.x[i];
             v.xt[i] = xi;
-            if (v.xf) v.xf[i] = float(xi);
+            v.xf[i] = float(xi);
         }
         if (lead) active[p] = 1;
         return;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(MT) k_min_propose(MinState *st, const PairVec 
         for (int i = i0 + tid; i < i1; i += MT) {
             const double x1 = __dadd_rn(v.x[i], __dmul_rn(a, v.g[i]));
             v.xt[i] = x1;
-            if (v.xf) v.xf[i] = float(x1);
+            v.xf[i] = float(x1);
             if (x1 != v.x[i]) mv = 1;
         }
         mv = __syncthreads_or(mv);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(MT) k_min_propose(MinState *st, const PairVec 
         for (int i = i0 + tid; i < i1; i += MT) {
             const double xi = __dadd_rn(v.xt[i], __dmul_rn(ms, v.g[i]));
             v.xt[i] = xi;
-            if (v.xf) v.xf[i] = float(xi);
+            v.xf[i] = float(xi);
         }
         double d0 = 0.0, d1 = 0.0, d2 = 0.0;
         if (!pair_totals(m, p, nb, d0, d1, d2, red)) return;
@@ -426,8 +426,11 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         a.grad_image = nullptr;
         a.grad_penalty = nullptr;
         a.costs = r.costs.p;
+        a.convert = 0;   // k_min_propose writes the float copy
+        // 2D SSD: the gather's last block finalises the cost
+        a.defer_cost = dim == 2 && a.cost == MGR_COST_SSD;
         args[k] = a;
-        vecs[k] = PairVec{r.x.p, r.g.p, r.xt.p, r.gt.p, r.costs.p, int(n), dim == 3 ? a.params_f : nullptr};
+        vecs[k] = PairVec{r.x.p, r.g.p, r.xt.p, r.gt.p, r.costs.p, int(n), a.params_f};
         MinState s{};
         s.step = mz.step;
         states[k] = s;

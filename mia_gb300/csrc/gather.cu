@@ -1,18 +1,24 @@
-// gather.cu — per-coefficient gather of the tile partials, the divcurl
-// penalty (value and gradient) and the final weighted costs.
+// gather.cu — 2D: per-coefficient gather of the tile partials, the divcurl
+// penalty (value and gradient) and the final weighted costs (3D: k_gather3 in
+// split3.cu).
 //
 // One block owns 32 consecutive coefficients (lane = coefficient, so
 // neighbour loads coalesce along x).  The eight warps split the work of
-// those 32 coefficients: the (dz, dy) rows of the 3D penalty stencil
-// (C3DPPDivcurlMatrixImpl::evaluate / multiply, mia/3d/ppmatrix.cc:292-599;
-// the P cell of an offset is read as a broadcast), the cells of the 2D
-// boundary-clipped CSR row (mia/2d/ppmatrix.cc:328-352), and the partial
-// slots of the split path that hold the coefficient.  Warp 0 combines the
-// per-warp sums in a fixed order (deterministic, no atomics), applies the
-// penalty weight and sign (C3DSplineTransformPenalty::value_and_gradient,
+// those 32 coefficients: the cells of the boundary-clipped CSR row
+// (mia/2d/ppmatrix.cc:328-352), and the partial slots of the split path that
+// hold the coefficient.  The per-warp sums are combined in a fixed order
+// (deterministic, no atomics), the penalty weight and sign
+// (C3DSplineTransformPenalty::value_and_gradient,
 // mia/3d/splinetransformpenalty.cc:60-71) and the full-cost weight
-// (mia/template/fullcost.cxx:37-45), and the last block finalises the costs.
+// (mia/template/fullcost.cxx:37-45) applied, and the last block finalises
+// the costs.
+//
+// A few blocks with a chain of dependent loads (row range, cell, parameter;
+// tile range, tile start, slot): latency bounds it, so the loads of a step
+// are issued together and everything but the slots is done before the wait
+// for the adjoint kernel.
 #include "mgr_cost.cuh"
+#include "mgr_launch.hh"
 
 namespace mgr {
 
@@ -20,138 +26,141 @@ namespace {
 constexpr int GT = 256;   // threads per block
 constexpr int GW = GT / 32;
 constexpr int GC = 32;    // coefficients per block
-constexpr int NPART = 12; // per warp: penalty g[3], r[6]; image s[3]
+constexpr int NPART = 7;  // per warp: penalty g[2], r[3]; image s[2]
+constexpr int GCELLS = 7; // cells a warp loads at a time: a row has at most 49
+constexpr int GSLOTS = 4; // partial slots a warp loads at a time
 }  // namespace
 
 // block `blk` of the pair's `nblk` gather blocks
-template <int D>
-__device__ __forceinline__ void gather_body(const EvalArgs &a, int with_gradient, int image_from_dense, int blk,
-                                            int nblk)
+__device__ __forceinline__ void gather2_body(const EvalArgs &a, int with_gradient, int image_from_dense, int blk,
+                                             int nblk)
 {
-    extern __shared__ float sm[];            // 3D: P table (9^3 x 6)
     __shared__ float part[GW][NPART][GC];
-    __shared__ double red[GW];
+    __shared__ double red[2 * GW];
     __shared__ bool is_last;
-    const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
-    const int ncx = a.nc[0], ncy = a.nc[1], ncz = (D == 3) ? a.nc[2] : 1;
-    const size_t ncoef = size_t(ncx) * ncy * ncz;
+    const Axis &X = a.ax[0], &Y = a.ax[1];
+    const int ncx = a.nc[0], ncy = a.nc[1];
+    const size_t ncoef = size_t(ncx) * ncy;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    if (D == 3 && a.has_penalty) {
-        for (int e = tid; e < 9 * 9 * 9 * 6; e += GT) sm[e] = a.ptable[e];
-        __syncthreads();
-    }
     const size_t i = size_t(blk) * GC + lane;
     const bool valid = i < ncoef;
     const int cx = valid ? int(i % ncx) : 0;
-    const int cy = valid ? int((i / ncx) % ncy) : 0;
-    const int cz = (D == 3 && valid) ? int(i / (size_t(ncx) * ncy)) : 0;
+    const int cy = valid ? int(i / ncx) : 0;
 
-    float g[3] = {0.0f, 0.0f, 0.0f};
-    float r[6] = {0, 0, 0, 0, 0, 0};
-    float s[3] = {0.0f, 0.0f, 0.0f};
+    // the slots that hold the coefficient: entries k = w, w + GW, ... of the
+    // tiles [gx, gy]
+    const bool img = valid && with_gradient && !image_from_dense;
+    int2 gx = make_int2(0, -1), gy = gx;
+    if (img) {
+        gx = X.gtile[cx];
+        gy = Y.gtile[cy];
+    }
+    const int nX = gx.y - gx.x + 1, nY = gy.y - gy.x + 1;
+    const int total = (nX > 0 && nY > 0) ? nX * nY : 0;
+    auto slot = [&](int k) -> const float * {
+        const int jy = k / nX, tx = gx.x + (k - jy * nX), ty = gy.x + jy;
+        const int lx = cx - X.atile0[tx], ly = cy - Y.atile0[ty];
+        return a.partial + (size_t(ty) * X.nt + tx) * a.slot + (size_t(ly) * X.ac + lx) * 2;
+    };
+    const float *sp[GSLOTS];
+#pragma unroll
+    for (int u = 0; u < GSLOTS; ++u) sp[u] = w + u * GW < total ? slot(w + u * GW) : nullptr;
+
+    // The float copy of the parameters is complete before any block of this
+    // kernel starts, except right after the warp kernel that makes it (the
+    // value alone, no adjoint kernel between them); it is read through the
+    // L2, never from a line an earlier kernel left in L1.
+    if (!with_gradient) pdl_wait();
+    float g[2] = {0.0f, 0.0f}, r[3] = {0, 0, 0}, s[2] = {0.0f, 0.0f};
     if (valid && a.has_penalty) {
-        if (D == 3) {
-            for (int p = w; p < 49; p += GW) {
-                const int dz = p / 7 - 3, dy = p % 7 - 3;
-                const int zj = cz - dz, yj = cy - dy;
-                if (zj < 0 || zj >= ncz || yj < 0 || yj >= ncy) continue;
-                const double *row = a.params + ((size_t(zj) * ncy + yj) * ncx) * 3;
-                const float *Prow = sm + (((dz + 4) * 9 + (dy + 4)) * 9 + 4) * 6;
+        const int e1 = a.pen_rowptr[i + 1];
+        for (int e0 = a.pen_rowptr[i] + w; e0 < e1; e0 += GW * GCELLS) {
+            float4 v[GCELLS];
+            int j[GCELLS];
+            float2 c[GCELLS];
 #pragma unroll
-                for (int dx = -3; dx <= 3; ++dx) {
-                    const int xj = cx - dx;
-                    if (xj < 0 || xj >= ncx) continue;
-                    const float *P = Prow + dx * 6;
-                    const float cjx = float(row[xj * 3]), cjy = float(row[xj * 3 + 1]), cjz = float(row[xj * 3 + 2]);
-                    const float vxx = P[0], vxy = P[1], vyy = P[2], vyz = P[3], vzz = P[4], vxz = P[5];
-                    if (with_gradient) {
-                        const float ax = vxx * cjx, az = vxz * cjx;
-                        const float bxy = vxy * cjy, byy = vyy * cjy;
-                        const float cyz = vyz * cjz, czz = vzz * cjz;
-                        r[0] += ax; r[1] += bxy; r[2] += byy; r[3] += cyz; r[4] += czz; r[5] += az;
-                        g[0] += cjz * vxz + (2.0f * ax + bxy);
-                        g[1] += cjx * vxy + (2.0f * byy + cyz);
-                        g[2] += cjy * vyz + (2.0f * czz + az);
-                    } else {
-                        // operator*: ci.x cj.y vxy, ci.x cj.z vxz, ci.y cj.z vyz
-                        r[0] += cjx * vxx; r[2] += cjy * vyy; r[4] += cjz * vzz;
-                        r[1] += cjy * vxy; r[5] += cjz * vxz; r[3] += cjz * vyz;
-                    }
+            for (int u = 0; u < GCELLS; ++u) {
+                const bool in = e0 + u * GW < e1;
+                j[u] = in ? a.pen_col[e0 + u * GW] : -1;
+                v[u] = in ? a.pen_val[e0 + u * GW] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < GCELLS; ++u)
+                c[u] = j[u] >= 0 ? __ldcg(reinterpret_cast<const float2 *>(a.params_f) + j[u])
+                                 : make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int u = 0; u < GCELLS; ++u)
+                if (j[u] >= 0) {
+                    const float cjx = c[u].x, cjy = c[u].y;
+                    const float aa = cjx * v[u].x, bb = cjy * v[u].y, cxx = cjx * v[u].z, cyy = cjy * v[u].z;
+                    g[0] += aa + aa + cyy;
+                    g[1] += bb + bb + cxx;
+                    r[0] += aa;
+                    r[1] += cyy;
+                    r[2] += bb;
                 }
-            }
-        } else {
-            for (int e = a.pen_rowptr[i] + w; e < a.pen_rowptr[i + 1]; e += GW) {
-                const int j = a.pen_col[e];
-                const float4 v = a.pen_val[e];
-                const float cjx = float(a.params[size_t(j) * 2]), cjy = float(a.params[size_t(j) * 2 + 1]);
-                const float aa = cjx * v.x, bb = cjy * v.y, cxx = cjx * v.z, cyy = cjy * v.z;
-                g[0] += aa + aa + cyy;
-                g[1] += bb + bb + cxx;
-                r[0] += aa;
-                r[1] += cyy;
-                r[2] += bb;
-            }
         }
     }
-    if (valid && with_gradient && !image_from_dense) {
-        const int2 gx = X.gtile[cx], gy = Y.gtile[cy];
-        const int2 gz = (D == 3) ? Z.gtile[cz] : make_int2(0, 0);
-        const int nX = gx.y - gx.x + 1, nY = gy.y - gy.x + 1, nZ = gz.y - gz.x + 1;
-        const int total = (nX > 0 && nY > 0 && nZ > 0) ? nX * nY * nZ : 0;
-        for (int k = w; k < total; k += GW) {
-            const int tx = gx.x + k % nX, ty = gy.x + (k / nX) % nY, tz = gz.x + k / (nX * nY);
-            const int lx = cx - X.atile0[tx], ly = cy - Y.atile0[ty];
-            const int lz = (D == 3) ? cz - Z.atile0[tz] : 0;
-            const size_t t = (size_t(tz) * Y.nt + ty) * X.nt + tx;
-            const float *p = a.partial + t * a.slot + ((size_t(lz) * Y.ac + ly) * X.ac + lx) * D;
+    float2 ci = make_float2(0.0f, 0.0f);
+    if (w == 0 && valid && a.has_penalty) ci = __ldcg(reinterpret_cast<const float2 *>(a.params_f) + i);
+    if (with_gradient) pdl_wait();
+    pdl_trigger();
+    {
+        float2 v[GSLOTS];
 #pragma unroll
-            for (int c = 0; c < D; ++c) s[c] += p[c];
-        }
+        for (int u = 0; u < GSLOTS; ++u)
+            v[u] = sp[u] ? __ldcg(reinterpret_cast<const float2 *>(sp[u])) : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < GSLOTS; ++u)
+            if (sp[u]) {
+                s[0] += v[u].x;
+                s[1] += v[u].y;
+            }
     }
+    for (int k = w + GSLOTS * GW; k < total; k += GW) {
+        const float2 v = __ldcg(reinterpret_cast<const float2 *>(slot(k)));
+        s[0] += v.x;
+        s[1] += v.y;
+    }
+    part[w][0][lane] = g[0];
+    part[w][1][lane] = g[1];
+    part[w][2][lane] = r[0];
+    part[w][3][lane] = r[1];
+    part[w][4][lane] = r[2];
+    part[w][5][lane] = s[0];
+    part[w][6][lane] = s[1];
+    __syncthreads();
+    // the warps' sums of each quantity in warp order, quantity k by warp k
+    if (w < NPART) {
+        float t = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) part[w][k][lane] = g[k];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) part[w][3 + k][lane] = r[k];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) part[w][9 + k][lane] = s[k];
+        for (int p = 0; p < GW; ++p) t += part[p][w][lane];
+        part[0][w][lane] = t;
+    }
     __syncthreads();
     if (w == 0) {
         double pval = 0.0;
+        // parameters the warp kernel found non-finite: nothing is written to
+        // the caller's buffers (uniform over the block)
+        const bool bad = a.params_host && *(volatile unsigned *)&a.counters[7] != 0u;
         if (valid) {
-            float G[3] = {0.0f, 0.0f, 0.0f}, R[6] = {0, 0, 0, 0, 0, 0}, S[3] = {0.0f, 0.0f, 0.0f};
-            for (int p = 0; p < GW; ++p) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) G[k] += part[p][k][lane];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) R[k] += part[p][3 + k][lane];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) S[k] += part[p][9 + k][lane];
-            }
-            double gp[3] = {0.0, 0.0, 0.0};
+            const float G[2] = {part[0][0][lane], part[0][1][lane]};
+            const float R[3] = {part[0][2][lane], part[0][3][lane], part[0][4][lane]};
+            const float S[2] = {part[0][5][lane], part[0][6][lane]};
+            double gp[2] = {0.0, 0.0};
             if (a.has_penalty) {
-                float ci[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int k = 0; k < D; ++k) ci[k] = float(a.params[i * D + k]);
-                float v;
-                if (D == 3) {
-                    if (with_gradient)
-                        v = ci[0] * R[0] + ci[0] * R[1] + ci[1] * R[2] + ci[1] * R[3] + ci[2] * R[4] + ci[2] * R[5];
-                    else
-                        v = ci[0] * R[0] + ci[1] * R[2] + ci[2] * R[4] + ci[0] * R[1] + ci[0] * R[5] + ci[1] * R[3];
-                } else {
-                    v = ci[0] * R[0] + ci[0] * R[1] + ci[1] * R[2];
-                }
+                const float v = ci.x * R[0] + ci.x * R[1] + ci.y * R[2];
                 pval = v;
 #pragma unroll
-                for (int k = 0; k < D; ++k) gp[k] = (a.pen_grad_sign * a.pen_weight) * double(G[k]);
+                for (int k = 0; k < 2; ++k) gp[k] = (a.pen_grad_sign * a.pen_weight) * double(G[k]);
             }
-            if (with_gradient) {
+            if (with_gradient && !bad) {
 #pragma unroll
-                for (int k = 0; k < D; ++k) {
-                    const double gi = image_from_dense ? a.grad_image[i * D + k] : a.cost_weight * (-double(S[k]));
-                    a.grad_total[i * D + k] = gi + gp[k];
-                    if (a.grad_image && !image_from_dense) a.grad_image[i * D + k] = gi;
-                    if (a.grad_penalty) a.grad_penalty[i * D + k] = gp[k];
+                for (int k = 0; k < 2; ++k) {
+                    const double gi = image_from_dense ? a.grad_image[i * 2 + k] : a.cost_weight * (-double(S[k]));
+                    a.grad_total[i * 2 + k] = gi + gp[k];
+                    if (a.grad_image && !image_from_dense) a.grad_image[i * 2 + k] = gi;
+                    if (a.grad_penalty) a.grad_penalty[i * 2 + k] = gp[k];
                 }
             }
         }
@@ -165,39 +174,60 @@ __device__ __forceinline__ void gather_body(const EvalArgs &a, int with_gradient
     __syncthreads();
     if (is_last) {
         __threadfence();
-        double sv[1] = {0.0};
-        for (unsigned b = tid; b < unsigned(nblk); b += GT) sv[0] += ((volatile double *)a.pen_part)[b];
-        block_sum<1>(sv, red);
+        // v[0]: a deferred SSD cost from the warp kernel's tile sums (the
+        // order of reduce_tile_sums); v[1]: the blocks' penalty partials
+        const bool fin = a.defer_cost && a.cost == 0;
+        double v2[2] = {0.0, 0.0};
+        if (fin) {
+            const int nt = X.nt * Y.nt;
+            for (int t = tid; t < nt; t += GT) v2[0] += __ldcg(a.tile_sums + size_t(t) * 5);
+        }
+        for (unsigned b = tid; b < unsigned(nblk); b += GT) v2[1] += ((volatile double *)a.pen_part)[b];
+        block_sum<2>(v2, red);
         if (tid == 0) {
+            if (fin) {
+                const double s5[5] = {v2[0], 0.0, 0.0, 0.0, 0.0};
+                finalise_cost(a, s5, size_t(a.n[0]) * a.n[1]);
+            }
             double *sc = a.scalars;
-            const double pen = a.has_penalty ? sv[0] : 0.0;
+            const double pen = a.has_penalty ? v2[1] : 0.0;
             sc[SC_PEN] = pen;
-            const double img = (D == 2 && with_gradient) ? sc[SC_FORCE_COST] : sc[SC_VALUE];
-            sc[SC_COST_IMG] = a.cost_weight * img;
+            const double im = with_gradient ? sc[SC_FORCE_COST] : sc[SC_VALUE];
+            sc[SC_COST_IMG] = a.cost_weight * im;
             sc[SC_COST_PEN] = a.has_penalty ? a.pen_weight * pen : 0.0;
             if (a.costs) {
                 a.costs[0] = sc[SC_COST_IMG];
                 a.costs[1] = sc[SC_COST_PEN];
+            }
+            if (a.host_out) {
+                // the costs and both status flags to the caller's host
+                // memory; the non-finite flag is cleared for the next call
+                // (every block has read it before its arrival above)
+                a.host_out[0] = sc[SC_COST_IMG];
+                a.host_out[1] = sc[SC_COST_PEN];
+                unsigned *hf = reinterpret_cast<unsigned *>(a.host_out + 2);
+                hf[0] = *(volatile unsigned *)&a.counters[6];
+                hf[1] = *(volatile unsigned *)&a.counters[7];
+                a.counters[7] = 0;
             }
             a.counters[1] = 0;
         }
     }
 }
 
-template <int D>
-__global__ void __launch_bounds__(GT) k_gather_b(EvalArgs a, int with_gradient, int image_from_dense)
+__global__ void __launch_bounds__(GT) k_gather2(const __grid_constant__ EvalArgs a, int with_gradient,
+                                                int image_from_dense)
 {
-    gather_body<D>(a, with_gradient, image_from_dense, blockIdx.x, gridDim.x);
+    gather2_body(a, with_gradient, image_from_dense, blockIdx.x, gridDim.x);
 }
 
 // batch: work list of (pair, block) items; finished pairs are skipped
-template <int D>
-__global__ void __launch_bounds__(GT) k_gather_batch(const EvalArgs *__restrict__ args, const int2 *__restrict__ items,
-                                                     const int *__restrict__ active, const int *__restrict__ nblocks)
+__global__ void __launch_bounds__(GT) k_gather2_batch(const EvalArgs *__restrict__ args, const int2 *__restrict__ items,
+                                                      const int *__restrict__ active, const int *__restrict__ nblocks)
 {
     const int2 it = items[blockIdx.x];
     if (!active[it.x]) return;
-    gather_body<D>(args[it.x], 1, 0, it.y, nblocks[it.x]);
+    gather2_body(args[it.x], 1, 0, it.y, nblocks[it.x]);
 }
 
 void launch_gather_batch(int dim, const EvalArgs *args, const int2 *items, int nitems, const int *active,
@@ -208,7 +238,7 @@ void launch_gather_batch(int dim, const EvalArgs *args, const int2 *items, int n
         launch_gather3_batch(args, items, nitems, active, nblocks, st);
         return;
     }
-    k_gather_batch<2><<<nitems, GT, 0, st>>>(args, items, active, nblocks);
+    k_gather2_batch<<<nitems, GT, 0, st>>>(args, items, active, nblocks);
     count_launch();
 }
 
@@ -225,7 +255,7 @@ void launch_gather_mode(const EvalArgs &a, int with_gradient, int dense, cudaStr
         launch_gather3(a, with_gradient, dense, st);
         return;
     }
-    k_gather_b<2><<<gather_blocks(a), GT, 0, st>>>(a, with_gradient, dense);
+    launch_pdl(a.pdl != 0, k_gather2, dim3(gather_blocks(a)), dim3(GT), 0, st, a, with_gradient, dense);
     count_launch();
 }
 

@@ -164,6 +164,8 @@ struct mgr_level {
     // 1: events around every kernel (launched one after another); 2: events
     // around the whole evaluation only (kernels overlap as in untimed runs)
     int timing_mode = 0, ev_mode = 0;
+    // a deferred cost finalisation (EvalArgs::defer_cost) is possible
+    bool can_defer() const { return d.dim == 3 || d.cost == MGR_COST_SSD; }
     // programmatic dependent launch of the split path's kernels (MGR_PDL=0
     // in the environment at level creation turns it off)
     bool pdl = true;
@@ -238,6 +240,7 @@ struct mgr_level {
         a.minmax = I.minmax.p;
         a.params = params.p;
         a.params_f = params_f.p;
+        a.convert = d.dim == 2;
         a.cost = d.cost;
         a.ssd_norm = d.ssd_norm;
         a.cost_weight = d.cost_weight;

@@ -46,28 +46,6 @@ __host__ __device__ inline int pad_pitch(int nx)
     return ((nx + 2 * PAD_H + 31) / 32) * 32;
 }
 
-// Shared-memory box in which the warp kernel stages the moving image's tap
-// footprint of one tile: rows of stage_bx floats (a multiple of 32, so that
-// the bank of a tap depends only on its x position and lanes on different
-// rows do not conflict), stage_by rows per plane, stage_bz planes.  A tile
-// whose footprint does not fit reads its taps from global memory.
-__host__ __device__ constexpr int stage_bx(int tx)
-{
-    return ((tx + 24 + 31) / 32) * 32;
-}
-__host__ __device__ constexpr int stage_by(int ty)
-{
-    return ty + 10;
-}
-__host__ __device__ constexpr int stage_bz(int dim, int tz)
-{
-    return dim == 3 ? tz + 10 : 1;
-}
-__host__ __device__ constexpr int stage_floats(int dim, int tx, int ty, int tz)
-{
-    return stage_bx(tx) * stage_by(ty) * stage_bz(dim, tz);
-}
-
 // Mirror boundary index folding with period 2w-2
 // (mia/core/splinebc/bc.cc:52-64).
 __device__ __forceinline__ int mirror_fold(int i, int w)
@@ -173,35 +151,10 @@ __device__ __forceinline__ float sample2(const float *__restrict__ c, int nx, in
     return clamp_ref(acc, mn, mx);
 }
 
-// Tricubic / bicubic sample from a shared-memory footprint of the
-// prefiltered image whose elements already hold the mirror-folded values:
-// `base` points at the first tap (fx-1, fy-1, fz-1) and rows / planes are
-// `sy` / `sz` floats apart.  Same weights and summation order as sample3 /
+// Bicubic sample whose first tap (fx-1, fy-1) is at `base`, rows `sy` floats
+// apart, no index folding needed.  Same weights and summation order as
 // sample2.
-__device__ __forceinline__ float staged_sample3(const float *base, int sy, int sz, float px, float py, float pz,
-                                                int fx, int fy, int fz, float mn, float mx)
-{
-    float wx[4], wy[4], wz[4];
-    bspline3_weights(px - float(fx), wx);
-    bspline3_weights(py - float(fy), wy);
-    bspline3_weights(pz - float(fz), wz);
-    float acc = 0.0f;
-#pragma unroll
-    for (int kz = 0; kz < 4; ++kz) {
-        const float *pl = base + kz * sz;
-        float ay = 0.0f;
-#pragma unroll
-        for (int ky = 0; ky < 4; ++ky) {
-            const float *row = pl + ky * sy;
-            const float r = wx[0] * row[0] + wx[1] * row[1] + wx[2] * row[2] + wx[3] * row[3];
-            ay += wy[ky] * r;
-        }
-        acc += wz[kz] * ay;
-    }
-    return clamp_ref(acc, mn, mx);
-}
-
-__device__ __forceinline__ float staged_sample2(const float *base, int sy, float px, float py, int fx, int fy,
+__device__ __forceinline__ float sample2_at(const float *base, int sy, float px, float py, int fx, int fy,
                                                 float mn, float mx)
 {
     float wx[4], wy[4];
@@ -218,13 +171,61 @@ __device__ __forceinline__ float staged_sample2(const float *base, int sy, float
 }
 
 // ---------------------------------------------------------------------
+// programmatic dependent launch
+// ---------------------------------------------------------------------
+// A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization
+// may start while the kernel before it in the stream is still running;
+// pdl_wait returns once that kernel has completed and its writes are visible
+// (at once for a kernel launched without the attribute).  Before it a kernel
+// reads only the level's fixed tables.  pdl_trigger, issued by every block
+// after its pdl_wait, lets the next kernel be launched: so no kernel starts
+// before the one two places back in the stream has completed.
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// ---------------------------------------------------------------------
 // reductions
 // ---------------------------------------------------------------------
+// double(x) with integer instructions: conversions to double share the FP64
+// pipe, which runs at a small fraction of the FP32 rate
+__device__ __forceinline__ double widen(float x)
+{
+    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    if (m - 0x00800000u < 0x7f000000u)   // a normal number: the exponent's bias moves by 1023 - 127
+        return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), int(u << 29));
+    return m == 0u ? __hiloint2double(int(u), 0) : double(x);
+}
+
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// The sums over the warp of five floats per lane in double, each with
+// warp_sum's tree (the same bits): lanes exchange halves of four of the
+// values, so that a step adds each pair once instead of in both lanes (11
+// FP64 additions per lane instead of 25).  v[k] of lane warp_sum5_lane(k)
+// holds sum k.
+__device__ __forceinline__ double warp_sum5(const float (&x)[5], int lane)
+{
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const double x0 = widen(x[0]), x1 = widen(x[1]), x2 = widen(x[2]), x3 = widen(x[3]);
+    double a = (h16 ? x2 : x0) + __shfl_xor_sync(0xffffffffu, h16 ? x0 : x2, 16);
+    const double b = (h16 ? x3 : x1) + __shfl_xor_sync(0xffffffffu, h16 ? x1 : x3, 16);
+    a = (h8 ? b : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+    a += __shfl_xor_sync(0xffffffffu, a, 4);
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    const double e = warp_sum(widen(x[4]));
+    return lane & 1 ? e : a;   // even lanes: sum 2 * h16 + h8, odd lanes: sum 4
 }
 
 // Block-wide sum of K doubles per thread into red[0..K-1] (thread 0 holds

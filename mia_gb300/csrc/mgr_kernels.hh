@@ -66,7 +66,8 @@ struct EvalArgs {
     float *warped;         // warped moving image (N)
     const float *minmax;   // device {min, max} clamp bounds
     const double *params;  // spline parameters, interleaved, device
-    float *params_f;       // 3D: their float copy (launch_params_f32), read by the warp and gather kernels
+    float *params_f;       // their float copy (3D: launch_params_f32), read by the warp and gather kernels
+    int convert;           // 2D: 1, the warp kernel makes the float copy; 0, it is there
     int cost;              // MGR_COST_SSD / NCC
     int ssd_norm;
     double cost_weight;
@@ -94,9 +95,9 @@ struct EvalArgs {
     double *grad_penalty;  // optional
     double *costs;         // optional {cost_image, cost_penalty}
     // caller's host memory read and written in place (a device with
-    // coherent access to pageable host memory, 3D split path): params_host
-    // is read by the parameter conversion (launch_params_f32), and the
-    // gather's last block writes {cost_image, cost_penalty, status flags}
+    // coherent access to pageable host memory, split path): params_host
+    // is read by the parameter conversion (3D: launch_params_f32, 2D: the
+    // warp kernel), and the gather's last block writes {cost_image, cost_penalty, status flags}
     // to host_out; the gradient pointers above may then be host memory too
     const double *params_host;
     double *host_out;
@@ -104,11 +105,11 @@ struct EvalArgs {
     // (the warp blocks then end without a device-wide fence and last-block
     // reduction): an SSD cost by the gather's last block (the adjoint takes
     // its force scale from the settings), an NCC cost by k_finalise3, which
-    // launch_warp3 queues right after the warp kernel; 0: the warp kernel's
-    // last block finalises the cost
+    // launch_warp3 queues right after the warp kernel (2D: SSD only); 0: the
+    // warp kernel's last block finalises the cost
     int defer_cost;
-    // 1: the 3D split path's warp, adjoint and gather kernels are launched
-    // with programmatic stream serialisation (each may start while the one
+    // 1: the split path's adjoint and gather kernels (3D: the warp kernel,
+    // too) are launched with programmatic stream serialisation (each may start while the one
     // before it finishes, and waits for it before reading its outputs)
     int pdl;
 };

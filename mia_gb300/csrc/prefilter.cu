@@ -342,17 +342,8 @@ void launch_prefilter(const float *src, float *coef, float *pad, int dim, int nx
 // The means of the two images in double (NCC provisional centres), and the
 // copy of the reference into the level in the same pass.  Per-block partial
 // sums in a fixed order, added by the last block.  FP64 instructions bound
-// it (two additions per voxel at 1/64 of the FP32 rate), so a value is
-// widened to double with integer instructions instead of a conversion on the
-// same pipe.
-__device__ __forceinline__ double widen(float x)
-{
-    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
-    if (m - 0x00800000u < 0x7f000000u)   // a normal number: the exponent's bias moves by 1023 - 127
-        return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), int(u << 29));
-    return m == 0u ? __hiloint2double(int(u), 0) : double(x);
-}
-
+// it (two additions per voxel at 1/64 of the FP32 rate), so values are widened
+// beside that pipe (widen).
 __global__ void __launch_bounds__(256) k_image_means(const float *__restrict__ src, const float *__restrict__ ref,
                                                      float *__restrict__ ref_out, size_t n, double *part,
                                                      unsigned *counter, double *out)

@@ -42,6 +42,7 @@
 
 #include "../../include/mgr.h"
 #include "mgr_cost.cuh"
+#include "mgr_launch.hh"
 #include "warp3_common.cuh"
 
 #include <type_traits>
@@ -68,23 +69,6 @@ constexpr int NT3 = 256;   // threads per tile block: 8 warps
 constexpr int TX3 = 32;    // tile x (lanes)
 constexpr int TY3 = 8;     // tile y (warps)
 constexpr unsigned FULL = 0xffffffffu;
-
-// Programmatic dependent launch.  A kernel launched with
-// cudaLaunchAttributeProgrammaticStreamSerialization may start while the
-// kernel before it in the stream is still running; pdl_wait returns once
-// that kernel has completed and its writes are visible (at once for a
-// kernel launched without the attribute).  Before it a kernel reads only
-// the level's fixed tables.  pdl_trigger, issued by every block after its
-// pdl_wait, lets the next kernel be launched: so no kernel starts before the
-// one two places back in the stream has completed.
-__device__ __forceinline__ void pdl_wait()
-{
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-__device__ __forceinline__ void pdl_trigger()
-{
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
 
 }  // namespace
 
@@ -1291,26 +1275,6 @@ __global__ void __launch_bounds__(256) k_params_f32(const double *__restrict__ p
 // ---------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------
-// A launch that may start while the kernel before it in the stream is still
-// running (programmatic stream serialisation; the kernel waits in pdl_wait
-// before it reads that kernel's outputs), or a plain stream-ordered launch.
-template <typename... KArgs, typename... Args>
-static void launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                       Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // The parameters read where the caller holds them (host memory that the
 // device reads coherently): the device keeps a double and a float copy.  A
 // non-finite value is stored as 0 in both and raises counters[7], so that
@@ -1335,7 +1299,7 @@ __global__ void __launch_bounds__(256) k_params_host(const double *__restrict__ 
 
 void launch_params_f32(const EvalArgs &a, cudaStream_t st)
 {
-    const size_t n = size_t(a.nc[0]) * a.nc[1] * a.nc[2] * 3;
+    const size_t n = size_t(a.nc[0]) * a.nc[1] * a.nc[2] * a.dim;
     const int nb = int(std::min<size_t>(1024, (n + 255) / 256));
     if (a.params_host)
         k_params_host<<<nb, 256, 0, st>>>(a.params_host, const_cast<double *>(a.params), a.params_f, n,
