@@ -410,6 +410,7 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     std::vector<int> nblocks(np);
     size_t sm_warp = 0, sm_adj = 0, max_params = 0;
     int has_pen = 0;
+    const int cost = pairs[members[0]]->full.cost;   // (the same for all pairs of a batch)
     for (int k = 0; k < np; ++k) {
         PairRun &r = *pairs[members[k]];
         const size_t n = r.params.size();
@@ -492,22 +493,22 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     const bool queue = persistent && dim == 3;
     int qgrid[2] = {0, 0};
     if (queue) {
-        prepare_split_batch(dim, tile[0], tile[1], tile[2], sm_warp, sm_adj);
-        qgrid[0] = std::min(int(titems.size()), split3_queue_grid(tile[2], 0, sm_warp));
-        qgrid[1] = std::min(int(titems.size()), split3_queue_grid(tile[2], 1, sm_adj));
+        prepare_split_batch(dim, cost, tile[0], tile[1], tile[2], sm_warp, sm_adj);
+        qgrid[0] = std::min(int(titems.size()), split3_queue_grid(cost, 0, sm_warp));
+        qgrid[1] = std::min(int(titems.size()), split3_queue_grid(cost, 1, sm_adj));
     }
     auto step = [&]() {
         k_min_propose<<<mgrid, MT, 0, st>>>(d_states, d_vecs, mz, d_active, msc);
         if (queue) {
-            launch_split3_queue(tile[2], d_args, d_titems, int(titems.size()), d_active, d_queue, qgrid[0], sm_warp,
+            launch_split3_queue(cost, d_args, d_titems, int(titems.size()), d_active, d_queue, qgrid[0], sm_warp,
                                 0, st);
-            launch_split3_queue(tile[2], d_args, d_titems, int(titems.size()), d_active, d_queue + 2, qgrid[1], sm_adj,
+            launch_split3_queue(cost, d_args, d_titems, int(titems.size()), d_active, d_queue + 2, qgrid[1], sm_adj,
                                 1, st);
         } else {
-            if (!launch_split_batch(dim, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
+            if (!launch_split_batch(dim, cost, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
                                     d_active, sm_warp, 0, st))
                 throw std::invalid_argument("tile shape not compiled in");
-            launch_split_batch(dim, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
+            launch_split_batch(dim, cost, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
                                d_active, sm_adj, 1, st);
         }
         launch_gather_batch(dim, d_args, d_gitems, int(gitems.size()), d_active, d_nblocks, has_pen, st);
@@ -517,7 +518,7 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     const int chunk = 8;
     const int max_steps = 1 + (mz.maxiter + 2) * 64;   // bounded: GSL trials shrink the step geometrically
     // kernel attributes are set outside the capture
-    prepare_split_batch(dim, tile[0], tile[1], tile[2], sm_warp, sm_adj);
+    prepare_split_batch(dim, cost, tile[0], tile[1], tile[2], sm_warp, sm_adj);
     cudaGraphExec_t exec = nullptr;
     const unsigned kernels_per_chunk = unsigned(chunk) * 5 + 1;
     tr_setup.stop();

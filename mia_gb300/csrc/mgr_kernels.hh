@@ -128,8 +128,9 @@ bool tile_supported(int dim, int tx, int ty, int tz);
 // (pair, tile) items (which = 0 warp, 1 adjoint) or (pair, block) items
 // (gather); pairs with active[pair] == 0 are skipped
 size_t split_smem(const EvalArgs &a, int which);
-void prepare_split_batch(int dim, int tx, int ty, int tz, size_t sm_warp, size_t sm_adj);
-bool launch_split_batch(int dim, int tx, int ty, int tz, const EvalArgs *args, const int2 *items, int nitems,
+// (all pairs of a batch have the same cost)
+void prepare_split_batch(int dim, int cost, int tx, int ty, int tz, size_t sm_warp, size_t sm_adj);
+bool launch_split_batch(int dim, int cost, int tx, int ty, int tz, const EvalArgs *args, const int2 *items, int nitems,
                         const int *active, size_t smem, int which, cudaStream_t st);
 void launch_gather_batch(int dim, const EvalArgs *args, const int2 *items, int nitems, const int *active,
                          const int *nblocks, int has_penalty, cudaStream_t st);
@@ -146,8 +147,8 @@ void launch_adjoint3(const EvalArgs &a, cudaStream_t st);
 // persistent batched 3D warp (which = 0) and adjoint (1) kernels: `grid`
 // resident blocks draw the items from the device queue queue[0..1] (zero
 // before the first launch; the last block resets it)
-int split3_queue_grid(int tz, int which, size_t sm);
-void launch_split3_queue(int tz, const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue,
+int split3_queue_grid(int cost, int which, size_t sm);
+void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue,
                          int grid, size_t sm, int which, cudaStream_t st);
 // the fused SSD kernel (fused3.cu): warp, force and adjoint in one pass per
 // 30 x 8 x TZ tile; with_gradient = 0 sums the cost only
@@ -156,8 +157,8 @@ size_t fused3_smem(const EvalArgs &a);
 void launch_fused3(const EvalArgs &a, int with_gradient, cudaStream_t st);
 int gather3_blocks(const EvalArgs &a);
 void launch_gather3(const EvalArgs &a, int with_gradient, int dense, cudaStream_t st);
-void prepare_split3_batch(int tz, size_t sm_warp, size_t sm_adj);
-void launch_split3_batch(int tz, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
+void prepare_split3_batch(int cost, size_t sm_warp, size_t sm_adj);
+void launch_split3_batch(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
                          int which, cudaStream_t st);
 void launch_gather3_batch(const EvalArgs *args, const int2 *items, int nitems, const int *active, const int *nblocks,
                           cudaStream_t st);

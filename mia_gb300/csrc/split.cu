@@ -473,10 +473,10 @@ static void prepare_batch_tile(size_t sm_warp, size_t sm_adj)
     cudaFuncSetAttribute(k_adjoint2_batch<TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_adj));
 }
 
-void prepare_split_batch(int dim, int tx, int ty, int tz, size_t sm_warp, size_t sm_adj)
+void prepare_split_batch(int dim, int cost, int tx, int ty, int tz, size_t sm_warp, size_t sm_adj)
 {
     if (dim == 3) {
-        prepare_split3_batch(tz, sm_warp, sm_adj);
+        if (tile_supported3_batch(tx, ty, tz)) prepare_split3_batch(cost, sm_warp, sm_adj);
         return;
     }
 #define MGR_PTILE2(X_, Y_) \
@@ -489,12 +489,12 @@ void prepare_split_batch(int dim, int tx, int ty, int tz, size_t sm_warp, size_t
 #undef MGR_PTILE2
 }
 
-bool launch_split_batch(int dim, int tx, int ty, int tz, const EvalArgs *args, const int2 *items, int nitems,
+bool launch_split_batch(int dim, int cost, int tx, int ty, int tz, const EvalArgs *args, const int2 *items, int nitems,
                         const int *active, size_t sm, int which, cudaStream_t st)
 {
     if (dim == 3) {
         if (!tile_supported3_batch(tx, ty, tz)) return false;
-        launch_split3_batch(tz, args, items, nitems, active, sm, which, st);
+        launch_split3_batch(cost, args, items, nitems, active, sm, which, st);
         return true;
     }
 #define MGR_BTILE2(X_, Y_)                                                      \

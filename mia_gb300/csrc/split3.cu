@@ -75,23 +75,42 @@ constexpr unsigned FULL = 0xffffffffu;
 // ---------------------------------------------------------------------
 // warp
 // ---------------------------------------------------------------------
-// COST: the image cost when known at compile time (MGR_COST_SSD / NCC; the
-// one-pair kernels are compiled per cost), -1 to read it from a
+// What bounds it: a sample takes 64 taps from shared memory, a wavefront
+// each for the 32 lanes of a warp (about 106 wavefronts per warp step with
+// bank conflicts, the tap planes' arrival and the tile's set-up), and the
+// instructions around them.  So the walk is kept lean: two planes per step
+// whose arithmetic runs on register pairs (one instruction for both), the
+// point's integer part from two additions rounded down, a tap address from
+// three integer instructions and the ring's wrap from a minimum.  No check
+// per voxel: the box that the ring holds contains the taps of every voxel of
+// the tile.  192x192x128 SSD, against a walk with scalar arithmetic, a check
+// and an index computation per voxel: 435 -> 313 instructions per warp step
+// and 77 -> 71 us cold, the shared-memory path 74 -> 81 % busy; evaluations
+// one after another 99.3 -> 92.2 us, 256^3 NCC 431 -> 396 us.
+//
+// COST: the image cost (MGR_COST_SSD / NCC); compiled per cost, the SSD
+// kernel keeps one sum and no branch on it
 template <int TZ, int COST>
 __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, int bz, int ntiles, int tile)
 {
-    const int cost = COST >= 0 ? COST : a.cost;
-    extern __shared__ __align__(16) float sm3[];
-    __shared__ double red[5 * (NT3 / 32)];
-    __shared__ float wsum[5][NT3 / 32];
+    constexpr int NW = NT3 / 32;
+    constexpr int NPAIR = RING_N / 2;                      // the ring's slots are filled in pairs of planes
+    constexpr unsigned PLANE_B = RING_PLANE * 4u, RING_B = RING_N * PLANE_B;
+    static_assert(RING_N % 2 == 0, "pairs of planes");
+    constexpr int cost = COST;
+    // [RING_N][RING_Y][RING_X] ring (the tensor copies want a 128-byte
+    // aligned destination), then C and Tx
+    extern __shared__ __align__(128) float sm3[];
+    __shared__ double red[5 * NW];
+    __shared__ float wsum[5][NW];
     __shared__ float csc[2];   // NCC centres (converted once per block)
     __shared__ int zs[TZ];
-    __shared__ float4 zw[TZ];
-    __shared__ float urng[NT3 / 32][6];   // per warp: footprint min / max per component
-    __shared__ int boxs[8];               // staged, xs, ylo, zbase, nplanes, span, w4, rows
-    __shared__ __align__(8) unsigned long long mbar[RING_N];
-    __shared__ unsigned rdone[RING_N];    // warps done with the ring slot's current plane
-    __shared__ int nissued;               // planes whose copies were issued
+    __shared__ float4 zw[TZ][2];          // the weights, each twice: {x, x, y, y}, {z, z, w, w}
+    __shared__ float urng[6][NW];         // per warp: displacement min / max per component
+    __shared__ int boxs[NW][3];           // per warp: the box's xs, ylo, zbase
+    __shared__ __align__(8) unsigned long long mbar[NPAIR];
+    __shared__ unsigned rdone[NPAIR];     // warps done with the slots' current planes
+    __shared__ int nissued;               // pairs of planes whose copies were issued
     __shared__ volatile int ring_failed;  // a wait of this block gave up
     __shared__ bool is_last;
     const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
@@ -116,80 +135,63 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
         fwz = Z.fw[z];
     }
     const float mn = a.minmax[0], mxv = a.minmax[1];
-    if (tid == 0) {
-        csc[0] = float(a.centers[0]);
-        csc[1] = float(a.centers[1]);
-    }
+    if (tid < 2) csc[tid] = cost == 0 ? 0.0f : float(a.centers[tid]);
 
     // the parameters' float copy comes from the kernel before this one
     pdl_wait();
     pdl_trigger();
-    float *C = sm3;                        // [3][FZ][FY][FX]
+    float *C = sm3 + RING_N * RING_PLANE;  // [3][FZ][FY][FX]
     float *Tx = C + 3 * FZ * FY * FX;      // [3][FZ][FY][32]
-    // [RING_N][RING_Y][RING_X]: the tensor copies want a 128-byte aligned
-    // destination, so the ring starts at the next 128-byte boundary of the
-    // shared window after Tx (the launch reserves the 128 bytes of slack)
-    float *ring;
-    {
-        const int off = 3 * FZ * FY * (FX + 32);
-        const unsigned ra = smem_u32(sm3 + off);
-        ring = sm3 + off + ((((ra + 127u) & ~127u) - ra) >> 2);
-    }
     // coefficient footprint: rows (iz, iy) of 3 FX consecutive floats
-    // (parameters are interleaved per node); each thread issues its loads
-    // as one batch before storing
-    {
-        const int w3 = 3 * FX, nel = FZ * FY * w3;
-        auto src = [&](int e, int &dst) -> const float * {
-            const int r = e / w3, j = e - r * w3;
-            const int ix = j / 3, c = j - 3 * ix;
-            const int iz = r / FY, iy = r - iz * FY;
-            dst = (c * FZ * FY + r) * FX + ix;
-            if (cx0 + ix >= ncx || cy0 + iy >= ncy || cz0 + iz >= ncz) return nullptr;
-            return a.params_f + ((size_t(cz0 + iz) * ncy + (cy0 + iy)) * ncx + cx0) * 3 + j;
-        };
-        constexpr int K = 4;
-        float v[K];
-        int dst[K];
+    // (parameters are interleaved per node), a warp per row, each thread's
+    // loads issued as one batch before storing
+    for (int j = lane; j < 3 * FX; j += 32) {
+        const int ix = j / 3, c = j - 3 * ix;
+        const bool inx = cx0 + ix < ncx;
+        const float *p = a.params_f + size_t(cx0) * 3 + j;
+        float *q = C + c * FZ * FY * FX + ix;
+        constexpr int K = 6;
+        const int nr = FZ * FY;
+        int iz = 0, iy = wy;
+        for (int r0 = wy; r0 < nr; r0 += K * NW) {
+            float v[K];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int e = tid + k * NT3;
-            v[k] = 0.0f;
-            dst[k] = -1;
-            if (e < nel) {
-                const float *p = src(e, dst[k]);
-                if (p) v[k] = *p;
+            for (int k = 0; k < K; ++k) {
+                while (iy >= FY) {
+                    iy -= FY;
+                    ++iz;
+                }
+                const bool in = inx && r0 + k * NW < nr && cy0 + iy < ncy && cz0 + iz < ncz;
+                v[k] = in ? p[(size_t(cz0 + iz) * ncy + (cy0 + iy)) * ncx * 3] : 0.0f;
+                iy += NW;
             }
-        }
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (dst[k] >= 0) C[dst[k]] = v[k];
-        for (int e = tid + K * NT3; e < nel; e += NT3) {
-            int d;
-            const float *p = src(e, d);
-            C[d] = p ? *p : 0.0f;
+            for (int k = 0; k < K; ++k)
+                if (r0 + k * NW < nr) q[(r0 + k * NW) * FX] = v[k];
         }
     }
     if (tid < TZ) {
         zs[tid] = fsz - cz0;
-        zw[tid] = fwz;
+        zw[tid][0] = make_float4(fwz.x, fwz.x, fwz.y, fwz.y);
+        zw[tid][1] = make_float4(fwz.z, fwz.z, fwz.w, fwz.w);
+    }
+    // the ring's barriers: one thread initialises them all (mbarrier and
+    // bulk-copy instructions are issued by single threads here)
+    if (tid == 0) {
+        for (int k = 0; k < NPAIR; ++k) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mbar[k])) : "memory");
+            rdone[k] = 0;
+        }
+        ring_failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
     // x stage: Tx[c][kz][jy][lane]
     {
         const int sx = fsx - cx0;
-        for (int r = wy; r < 3 * FZ * FY; r += NT3 / 32) {
+        for (int r = wy; r < 3 * FZ * FY; r += NW) {
             const float *c = C + r * FX + sx;
             Tx[r * 32 + lane] = fwx.x * c[0] + fwx.y * c[1] + fwx.z * c[2] + fwx.w * c[3];
-        }
-        // the ring's barriers: one thread initialises them all (mbarrier and
-        // bulk-copy instructions are issued by single threads here)
-        if (tid == 0) {
-            for (int k = 0; k < RING_N; ++k) {
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mbar[k])) : "memory");
-                rdone[k] = 0;
-            }
-            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
     }
     __syncthreads();
@@ -199,195 +201,166 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
         const float *t = Tx + ((c * FZ + kz) * FY + sy) * 32 + lane;
         return wyv.x * t[0] + wyv.y * t[32] + wyv.z * t[64] + wyv.w * t[96];
     };
-    float q[3][4];
+    // the window of four z coefficients, components 0 and 1 as pairs
+    float2x q01[4];
+    float q2[4];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) q[c][m] = qat(c, m);
+    for (int m = 0; m < 4; ++m) {
+        q01[m] = pack2(qat(0, m), qat(1, m));
+        q2[m] = qat(2, m);
+    }
     int cur = 0;   // the window's first z coefficient (zs[0] == 0)
     auto advance = [&](int t) {   // the window moves to the coefficients of plane z0 + t (uniform)
         const int s = zs[t];
         while (cur < s) {
             ++cur;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                q[c][0] = q[c][1];
-                q[c][1] = q[c][2];
-                q[c][2] = q[c][3];
-                q[c][3] = qat(c, cur + 3);
+            for (int m = 0; m < 3; ++m) {
+                q01[m] = q01[m + 1];
+                q2[m] = q2[m + 1];
             }
+            q01[3] = pack2(qat(0, cur + 3), qat(1, cur + 3));
+            q2[3] = qat(2, cur + 3);
         }
     };
-    const bool inxy_t = (x0 + lane < nx) && (y0 + wy < ny);
+    auto displacement = [&](int t, float &u0, float &u1, float &u2) {
+        const float4 wa = zw[t][0], wb = zw[t][1];
+        const float2x u01 = fma2(pack2(wb.z, wb.w), q01[3],
+                                 fma2(pack2(wb.x, wb.y), q01[2],
+                                      fma2(pack2(wa.x, wa.y), q01[0], mul2(pack2(wa.z, wa.w), q01[1]))));
+        unpack2(u01, u0, u1);
+        u2 = __fmaf_rn(wb.z, q2[3], __fmaf_rn(wb.x, q2[2], __fmaf_rn(wa.x, q2[0], __fmul_rn(wa.z, q2[1]))));
+    };
+    const bool inxy = (x0 + lane < nx) && (y0 + wy < ny);
     {
         // the range of u over the tile: along z, u is a combination of this
         // thread's q values over the window range 0 .. zs[ez-1] + 3 with
         // non-negative weights summing to 1 (to less than 1 on the last
-        // plane of the image, where 0 joins the range)
+        // plane of the image, where 0 joins the range).  A NaN stays in the
+        // range (the tile is then not staged).
         float lo[3], hi[3];
+        float m0[4], m1[4];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {   // the window's q values are kz = 0..3
-            lo[c] = fminf(fminf(q[c][0], q[c][1]), fminf(q[c][2], q[c][3]));
-            hi[c] = fmaxf(fmaxf(q[c][0], q[c][1]), fmaxf(q[c][2], q[c][3]));
+        for (int m = 0; m < 4; ++m) unpack2(q01[m], m0[m], m1[m]);   // the window's q values are kz = 0..3
+        const float *const w4[3] = {m0, m1, q2};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = min_nan(min_nan(w4[c][0], w4[c][1]), min_nan(w4[c][2], w4[c][3]));
+            hi[c] = max_nan(max_nan(w4[c][0], w4[c][1]), max_nan(w4[c][2], w4[c][3]));
         }
         const int kend = zs[ez - 1] + 3;
         for (int kz = 4; kz <= kend; ++kz)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float v = qat(c, kz);
-                lo[c] = fminf(lo[c], v);
-                hi[c] = fmaxf(hi[c], v);
+                lo[c] = min_nan(lo[c], v);
+                hi[c] = max_nan(hi[c], v);
             }
         const bool last_plane = z0 + ez == nz;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             if (last_plane) {
-                lo[c] = fminf(lo[c], 0.0f);
-                hi[c] = fmaxf(hi[c], 0.0f);
+                lo[c] = min_nan(lo[c], 0.0f);
+                hi[c] = max_nan(hi[c], 0.0f);
             }
-            if (!inxy_t) {
+            if (!inxy) {
                 lo[c] = 3.0e38f;
                 hi[c] = -3.0e38f;
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                lo[c] = fminf(lo[c], __shfl_xor_sync(FULL, lo[c], o));
-                hi[c] = fmaxf(hi[c], __shfl_xor_sync(FULL, hi[c], o));
+            const float l = warp_min_nan(lo[c]), h = warp_max_nan(hi[c]);
+            if (lane == 0) {
+                urng[c][wy] = l;
+                urng[3 + c][wy] = h;
             }
         }
-        if (lane == 0)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                urng[wy][c] = lo[c];
-                urng[wy][3 + c] = hi[c];
-            }
     }
     __syncthreads();
-    // tap box of the tile: x from xs (16-byte aligned in the padded rows),
-    // rows from ylo, planes zbase .. zbase + nplanes - 1 of which step t
-    // needs t .. t + span - 1; the ring is filled by bulk copies, one per
-    // row, completion counted on the plane's mbarrier
+    // tap box of the tile, the same in every thread: x from xs (16-byte
+    // aligned in the padded rows), rows from ylo, planes zbase .. zbase +
+    // nplanes - 1 of which step t needs t .. t + span - 1
     constexpr int H = PAD_H;
-    auto issue_plane = [&](int k) {   // one thread: plane k of the box into its ring slot, one tensor copy
-        const int slot = ring_slot(k);
-        const unsigned mb = smem_u32(&mbar[slot]);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mb),
-                     "r"(unsigned(RING_PLANE) * 4u)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-            "[%5];\n" ::"r"(smem_u32(ring + slot * RING_PLANE)),
-            "l"(reinterpret_cast<unsigned long long>(&a.tmap)), "r"(boxs[1] + H), "r"(boxs[2] + H), "r"(boxs[3] + k + H),
-            "r"(mb)
-            : "memory");
-    };
-    // the displacement range of the tile: lane k < 6 of warp 0 reduces bound
-    // k over the warps (lanes 0-2 the minima, 3-5 the maxima), lane 0 then
-    // sets the box
-    float urange = 0.0f;
-    if (wy == 0 && lane < 6) {
-        urange = urng[0][lane];
-        for (int w = 1; w < NT3 / 32; ++w)
-            urange = lane < 3 ? fminf(urange, urng[w][lane]) : fmaxf(urange, urng[w][lane]);
-    }
-    float ulo[3], uhi[3];
+    bool staged;
+    int xs, ylo, zbase, nplanes, span;
+    {
+        float ulo[3], uhi[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        ulo[c] = __shfl_sync(FULL, urange, c);
-        uhi[c] = __shfl_sync(FULL, urange, 3 + c);
-    }
-    if (tid == 0) {
-        // taps of a voxel at p = v - u: floor(p) - 1 .. floor(p) + 2; the
-        // fixed-point floor may round p up to the next integer, one more
-        // row / column / plane on the upper side
+        for (int c = 0; c < 3; ++c) {
+            ulo[c] = warp_min_nan(urng[c][lane & (NW - 1)]);
+            uhi[c] = warp_max_nan(urng[3 + c][lane & (NW - 1)]);
+        }
+        // taps of a voxel at p = v - u: floor(p) - 1 .. floor(p) + 2.  The
+        // fixed-point floor may round p up to the next integer: one more
+        // row / column / plane on the upper side, which also covers the
+        // rounding of u and p there; on the lower side the margin m covers
+        // it (u: a few roundings of 2^-24 relative; p: one).
         const float big = 1.0e6f;
         // once a wait of this launch has given up (the flag the host reads
         // afterwards), later blocks read their taps from global memory, so
         // that a stalled copy engine costs one wait limit per launch, not
         // one per block
-        bool ok = a.has_tmap != 0 && *(volatile unsigned *)&a.counters[6] == 0u;
+        bool ok = a.has_tmap != 0 && *(volatile unsigned *)&a.counters[6] == 0u && (smem_u32(sm3) & 127u) == 0u;
+        float m = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) ok = ok && fabsf(ulo[c]) < big && fabsf(uhi[c]) < big;
-        int xs = 0, xe = 0, ylo = 0, yhi = 0, dzl = 0, dzh = 0;
+        for (int c = 0; c < 3; ++c) {
+            ok = ok && fabsf(ulo[c]) < big && fabsf(uhi[c]) < big;
+            m = fmaxf(m, fmaxf(fabsf(ulo[c]), fabsf(uhi[c])));
+        }
+        m = 1.0e-4f + 1.0e-6f * (m + float(max(nx, max(ny, nz))));
+        xs = ylo = zbase = nplanes = span = 0;
         if (ok) {
-            const int xlo = int(floorf(float(x0) - uhi[0])) - 1;
-            xe = int(floorf(float(x0 + TX3 - 1) - ulo[0])) + 3;
+            const int xlo = int(floorf(float(x0) - uhi[0] - m)) - 1;
+            const int xe = int(floorf(float(x0 + TX3 - 1) - ulo[0])) + 3;
             xs = ((xlo + H) & ~3) - H;
-            ylo = int(floorf(float(y0) - uhi[1])) - 1;
-            yhi = int(floorf(float(y0 + ey - 1) - ulo[1])) + 3;
-            dzl = int(floorf(-uhi[2])) - 1;
-            dzh = int(floorf(-ulo[2])) + 3;
+            ylo = int(floorf(float(y0) - uhi[1] - m)) - 1;
+            const int yhi = int(floorf(float(y0 + ey - 1) - ulo[1])) + 3;
+            const int dzl = int(floorf(-uhi[2] - m)) - 1;
+            const int dzh = int(floorf(-ulo[2])) + 3;
             ok = xs >= -H && xe <= nx + H - 1 && xe - xs + 1 <= RING_X && ylo >= -H && yhi <= ny + H - 1 &&
                  yhi - ylo + 1 <= RING_Y && z0 + dzl >= -H && z0 + ez - 1 + dzh <= nz + H - 1 &&
                  dzh - dzl + 1 <= RING_N - 2;
+            zbase = z0 + dzl;
+            span = dzh - dzl + 1;
+            nplanes = ez + span - 1;
         }
-        boxs[0] = ok;
-        boxs[1] = xs;
-        boxs[2] = ylo;
-        boxs[3] = z0 + dzl;
-        boxs[4] = ez + dzh - dzl;
-        boxs[5] = dzh - dzl + 1;
-        boxs[6] = RING_X;
-        boxs[7] = yhi - ylo + 1;
-        ring_failed = 0;
-        nissued = ok ? min(boxs[4], RING_N) : 0;
+        staged = ok;
     }
-    __syncthreads();
-    // the box's first planes, issued by thread 0 after the barrier: the
-    // other warps start their walks meanwhile, their waits on a plane end
-    // once its copy has been issued and has landed
-    if (tid == 0)
-        for (int k = 0; k < nissued; ++k) issue_plane(k);
+    if (lane == 0) {   // for the refills this lane may issue
+        boxs[wy][0] = xs + H;
+        boxs[wy][1] = ylo + H;
+        boxs[wy][2] = zbase + H;
+    }
+    // one thread: pair k of the box's planes into its ring slots, one tensor
+    // copy a plane, completion counted on the pair's mbarrier
+    auto issue_pair = [&](int k) {
+        const int slot = k % NPAIR;
+        const unsigned mb = smem_u32(&mbar[slot]);
+        const int np = min(2, nplanes - 2 * k);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mb), "r"(PLANE_B * unsigned(np))
+                     : "memory");
+        for (int j = 0; j < np; ++j)
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+                "%4}], [%5];\n" ::"r"(smem_u32(sm3) + unsigned(2 * slot + j) * PLANE_B),
+                "l"(reinterpret_cast<unsigned long long>(&a.tmap)), "r"(boxs[wy][0]), "r"(boxs[wy][1]),
+                "r"(boxs[wy][2] + 2 * k + j), "r"(mb)
+                : "memory");
+    };
+    // the box's first planes, issued by thread 0: the other warps start
+    // their walks meanwhile, their waits on a plane end once its copy has
+    // been issued and has landed
+    if (tid == 0) {
+        const int n0 = staged ? min((nplanes + 1) / 2, NPAIR) : 0;
+        nissued = n0;
+        // (a persistent block's ring was read for the item before)
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        for (int k = 0; k < n0; ++k) issue_pair(k);
+    }
 
-    const bool inxy = (x0 + lane < nx) && (y0 + wy < ny);
     const float px0 = float(x0 + lane), py0 = float(y0 + wy);
     const float ca = csc[0], cb = csc[1];
     const size_t nxy = size_t(nx) * ny;
-    const size_t col = size_t(min(y0 + wy, ny - 1)) * nx + min(x0 + lane, nx - 1) + size_t(z0) * nxy;
-    float *wout = a.warped + col;
-    const float *rin = a.ref + col;
+    const size_t col = size_t(y) * nx + x + size_t(z0) * nxy;
     float acc[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    const bool staged = boxs[0] != 0;
-    const int bxs = boxs[1], bylo = boxs[2], bzbase = boxs[3], nplanes = boxs[4], span = boxs[5];
-    const int brows = boxs[7];
-    bool ring_ok = staged;
-    // planes (bit t) of this thread's voxels whose taps are not read from
-    // the ring: all of them when the tile was not staged, else the rare
-    // voxel outside the box and, after a wait gave up, the rest of the walk.
-    // They are sampled from global memory after the walk, so that the walk
-    // itself makes no call (a call site costs the loop register spills).
-    unsigned defer = 0u;
-    int kwait = 0;      // planes below kwait have arrived
-    // the reference is streamed three planes ahead of its use (registers
-    // r0..r2), so the walk does not wait on its memory latency
-    // two planes per step: the two voxels' tap gathers are independent
-    // chains, so a warp keeps twice the loads in flight; the waits, the
-    // displacement window and the refills are done per pair.  Per voxel the
-    // arithmetic and the order of the sums are those of one plane per step.
-    float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, r3 = 0.0f;
-    if (inxy) {
-        r0 = __ldg(rin);
-        if (ez > 1) r1 = __ldg(rin + nxy);
-        if (ez > 2) r2 = __ldg(rin + 2 * nxy);
-        if (ez > 3) r3 = __ldg(rin + 3 * nxy);
-    }
-    // the sample at plane t from the ring; ok = false when its taps are
-    // not there (the voxel is deferred)
-    auto sample_ring = [&](int t, int st, const float u[3], bool &ok) -> float {
-        const int z = z0 + t;
-        const float px = px0 - u[0], py = py0 - u[1], pz = float(z) - u[2];
-        const int fx = ffloor16(px), fy = ffloor16(py), fz = ffloor16(pz);
-        const int col = fx - 1 - bxs, row = fy - 1 - bylo, dk = fz - 1 - bzbase - t;
-        ok = ring_ok && unsigned(col) < unsigned(RING_X - 3) && unsigned(row) < unsigned(brows - 3) &&
-             unsigned(dk) < unsigned(span - 3);
-        // a voxel whose taps are not in the ring reads the ring's first taps
-        // instead (the sample is discarded and the voxel deferred), so that
-        // no branch separates the step's two tap chains
-        const int c = ok ? col : 0, r = ok ? row : 0, d = ok ? dk : 0;
-        // the slot of plane t + d: st is plane t's, d < RING_N
-        const int sl = st + d >= RING_N ? st + d - RING_N : st + d;
-        return taps3_ring(ring, sl, r, c, px - float(fx), py - float(fy), pz - float(fz), mn, mxv);
-    };
     auto add_cost = [&](float wv, float b) {
         if (cost == 0) {
             const float d = wv - b;
@@ -401,123 +374,156 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             acc[4] += da * db;
         }
     };
-    // this warp is done with planes t and t + 1 (t even: the pair's slots
-    // st, st + 1 share the counter of slot st); the last warp refills both
-    auto release = [&](int t, int st) {
-        if (staged && t + RING_N < nplanes) {
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence_block();
-                if (atomicAdd(&rdone[st], 1u) == unsigned(NT3 / 32 - 1)) {
-                    rdone[st] = 0;
-                    if (ring_ok && !ring_failed) {
-                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                        issue_plane(t + RING_N);
-                        const bool second = t + 1 + RING_N < nplanes;
-                        if (second) issue_plane(t + 1 + RING_N);
-                        atomicAdd(&nissued, second ? 2 : 1);
-                    }
-                }
-            }
+    int tdone = 0;   // planes walked (a warp whose wait gives up stops)
+    int kw = 0;      // pairs of planes that have arrived (thread 0 drains from here)
+    if (staged) {
+        float *wout = a.warped + col;
+        const float *rin = a.ref + col;
+        // the reference is streamed two steps ahead of its use, so the walk
+        // does not wait on its memory latency
+        float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, r3 = 0.0f;
+        if (inxy) {
+            r0 = __ldg(rin);
+            if (ez > 1) r1 = __ldg(rin + nxy);
+            if (ez > 2) r2 = __ldg(rin + 2 * nxy);
+            if (ez > 3) r3 = __ldg(rin + 3 * nxy);
         }
-    };
-    if (!staged && inxy) defer = ez >= 32 ? ~0u : (1u << ez) - 1u;
-    static_assert(RING_N % 2 == 0, "the walk releases the ring's slots in pairs");
-    for (int t = 0, st = 0; staged && t < ez; t += 2, st = st + 2 == RING_N ? 0 : st + 2) {
-        const bool two = t + 1 < ez;
-        float ua[3], ub[3] = {0.0f, 0.0f, 0.0f};
-        advance(t);
-        {
-            const float4 wz = zw[t];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) ua[c] = wz.x * q[c][0] + wz.y * q[c][1] + wz.z * q[c][2] + wz.w * q[c][3];
-        }
-        if (two) {
-            advance(t + 1);
-            const float4 wz = zw[t + 1];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) ub[c] = wz.x * q[c][0] + wz.y * q[c][1] + wz.z * q[c][2] + wz.w * q[c][3];
-        }
-        if (ring_ok) {
-            const int need = t + span - (two ? 0 : 1);
-            while (kwait <= need) {
-                if (!mbar_wait(smem_u32(&mbar[ring_slot(kwait)]), unsigned(kwait / RING_N) & 1u) || ring_failed) {
-                    if (!ring_failed) {
-                        ring_failed = 1;
-                        atomicOr(&a.counters[6], 1u);
-                    }
-                    ring_ok = false;
+        // byte offset of a point's first tap in the ring from the bits of its
+        // integer parts (floor2): 4 (fx - 1 - xs) + 256 (fy - 1 - ylo) + the
+        // plane fz - 1 - zbase; koff also takes off the ring's whole turns
+        unsigned koff = 0u - (FLOOR_BITS + 1u + unsigned(xs)) * 4u - (FLOOR_BITS + 1u + unsigned(ylo)) * (RING_X * 4u) -
+                        (FLOOR_BITS + 1u + unsigned(zbase)) * PLANE_B;
+        // (the last minimum only keeps a wild offset inside the ring)
+        auto tap0 = [&](unsigned ix, unsigned iy, unsigned iz) {
+            const unsigned o = ix * 4u + iy * (RING_X * 4u) + iz * PLANE_B + koff;
+            return min(min(o, o - RING_B), RING_B - 4u);
+        };
+        auto next_plane = [](unsigned o) { return min(o + PLANE_B, o + PLANE_B - RING_B); };
+        unsigned wmb = smem_u32(mbar), wpar = 0;   // the barrier and parity of pair kw
+        float zf = float(z0);
+        int st = 0;   // the ring slot of plane t
+#pragma unroll 1
+        for (int t = 0; t < ez; t += 2) {
+            const bool two = t + 1 < ez;
+            const int tb = two ? t + 1 : t;   // an odd last plane is sampled twice, the second discarded
+            float ua0, ua1, ua2, ub0, ub1, ub2;
+            advance(t);
+            displacement(t, ua0, ua1, ua2);
+            advance(tb);
+            displacement(tb, ub0, ub1, ub2);
+            const int need = min((t + span) >> 1, (nplanes - 1) >> 1);
+            bool failed = false;
+            while (kw <= need) {
+                if (!mbar_wait(wmb, wpar) || ring_failed) {
+                    failed = true;
                     break;
                 }
-                ++kwait;
-            }
-        }
-        if (inxy) {
-            bool oka, okb = true;
-            const float wa = sample_ring(t, st, ua, oka);
-            float wb = 0.0f;
-            if (two) wb = sample_ring(t + 1, st + 1, ub, okb);
-            if (oka) {
-                wout[0] = wa;
-                add_cost(wa, r0);
-            } else {
-                defer |= 1u << t;
-            }
-            if (two) {
-                if (okb) {
-                    wout[nxy] = wb;
-                    add_cost(wb, r1);
-                } else {
-                    defer |= 1u << (t + 1);
+                ++kw;
+                wmb += 8;
+                if (wmb == smem_u32(mbar) + 8 * NPAIR) {
+                    wmb = smem_u32(mbar);
+                    wpar ^= 1u;
                 }
             }
+            if (failed) {
+                if (!ring_failed) {
+                    ring_failed = 1;
+                    atomicOr(&a.counters[6], 1u);
+                }
+                break;
+            }
+            const float2x px = pack2(px0 - ua0, px0 - ub0), py = pack2(py0 - ua1, py0 - ub1);
+            const float2x pz = pack2(zf - ua2, (two ? zf + 1.0f : zf) - ub2);
+            unsigned xa, xb, ya, yb, za, zb;
+            const float2x fx = floor2(px, xa, xb), fy = floor2(py, ya, yb), fz = floor2(pz, za, zb);
+            unsigned oa = tap0(xa, ya, za), ob = tap0(xb, yb, zb);
+            float2x wx[4], wyp[4], wz[4];
+            bspline3_weights2(sub2(px, fx), wx);
+            bspline3_weights2(sub2(py, fy), wyp);
+            bspline3_weights2(sub2(pz, fz), wz);
+            float2x sum;
+#pragma unroll
+            for (int kz = 0; kz < 4; ++kz) {
+                const float *pa = reinterpret_cast<const float *>(reinterpret_cast<const char *>(sm3) + oa);
+                const float *pb = reinterpret_cast<const float *>(reinterpret_cast<const char *>(sm3) + ob);
+                float2x ay;
+#pragma unroll
+                for (int ky = 0; ky < 4; ++ky) {
+                    const float *ra = pa + ky * RING_X, *rb = pb + ky * RING_X;
+                    float2x r = mul2(wx[1], pack2(ra[1], rb[1]));
+                    r = fma2(wx[0], pack2(ra[0], rb[0]), r);
+                    r = fma2(wx[2], pack2(ra[2], rb[2]), r);
+                    r = fma2(wx[3], pack2(ra[3], rb[3]), r);
+                    ay = ky == 0 ? mul2(wyp[0], r) : fma2(wyp[ky], r, ay);
+                }
+                sum = kz == 0 ? mul2(wz[0], ay) : fma2(wz[kz], ay, sum);
+                oa = next_plane(oa);
+                ob = next_plane(ob);
+            }
+            if (inxy) {
+                float wa, wb;
+                unpack2(sum, wa, wb);
+                wa = fminf(fmaxf(wa, mn), mxv);
+                wb = fminf(fmaxf(wb, mn), mxv);
+                wout[0] = wa;
+                add_cost(wa, r0);
+                if (two) {
+                    wout[nxy] = wb;
+                    add_cost(wb, r1);
+                }
+            }
+            r0 = r2;
+            r1 = r3;
+            if (inxy && t + 4 < ez) r2 = __ldg(rin + 4 * nxy);
+            if (inxy && t + 5 < ez) r3 = __ldg(rin + 5 * nxy);
+            wout += 2 * nxy;
+            rin += 2 * nxy;
+            zf += 2.0f;
+            tdone = tb + 1;
+            // this warp is done with planes t and t + 1; the last warp
+            // refills their slots
+            if (t + RING_N < nplanes) {
+                __syncwarp();
+                if (lane == 0) {
+                    __threadfence_block();
+                    if (atomicAdd(&rdone[st >> 1], 1u) == unsigned(NW - 1)) {
+                        rdone[st >> 1] = 0;
+                        if (!ring_failed) {
+                            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                            issue_pair((t + RING_N) >> 1);
+                            atomicAdd(&nissued, 1);
+                        }
+                    }
+                }
+            }
+            st += 2;
+            if (st == RING_N) {
+                st = 0;
+                koff -= RING_B;
+            }
         }
-        r0 = r2;
-        r1 = r3;
-        r2 = (inxy && t + 4 < ez) ? __ldg(rin + 4 * nxy) : 0.0f;
-        r3 = (inxy && t + 5 < ez) ? __ldg(rin + 5 * nxy) : 0.0f;
-        wout += 2 * nxy;
-        rin += 2 * nxy;
-        release(t, st);
     }
-    // the deferred voxels, in plane order: the displacement from the y
-    // stage's window at plane t (the walk's values: the window then starts
-    // at coefficient zs[t]) and the taps from global memory
-    if (defer) {
-        float *const w0p = a.warped + col;
-        const float *const r0p = a.ref + col;
-        do {
-            const int t = __ffs(defer) - 1;
-            defer &= defer - 1u;
+    // the planes not walked (a tile whose taps do not fit the ring, or the
+    // rest of a walk whose wait gave up): the displacement from the y stage's
+    // window at plane t (the walk's values: the window then starts at
+    // coefficient zs[t]) and the taps from global memory.  They come after
+    // the walk, so that the walk itself makes no call (a call site costs the
+    // loop register spills).
+    if (inxy)
+        for (int t = tdone; t < ez; ++t) {
             const int s = zs[t];
-            const float4 wz = zw[t];
+            const float4 wa = zw[t][0], wb = zw[t][1];
             float u[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                u[c] = wz.x * qat(c, s) + wz.y * qat(c, s + 1) + wz.z * qat(c, s + 2) + wz.w * qat(c, s + 3);
+                u[c] = wa.x * qat(c, s) + wa.z * qat(c, s + 1) + wb.x * qat(c, s + 2) + wb.z * qat(c, s + 3);
             const float wv = taps3_global(a, px0 - u[0], py0 - u[1], float(z0 + t) - u[2], mn, mxv);
-            w0p[size_t(t) * nxy] = wv;
-            add_cost(wv, __ldg(r0p + size_t(t) * nxy));
-        } while (defer);
-    }
-    if (staged) __syncthreads();   // every warp is done with the ring
-    if (staged && tid == 0) {
-        // copies still in flight (only after a wait gave up) are waited for
-        // before the block's shared memory is released: only the planes that
-        // were issued, and within one wait limit in total (a plane whose
-        // wait gives up ends the drain)
-        const int issued = nissued;
-        while (kwait < issued) {
-            if (!mbar_wait(smem_u32(&mbar[ring_slot(kwait)]), unsigned(kwait / RING_N) & 1u)) {
-                atomicOr(&a.counters[6], 1u);
-                break;
-            }
-            ++kwait;
+            a.warped[col + size_t(t) * nxy] = wv;
+            add_cost(wv, __ldg(a.ref + col + size_t(t) * nxy));
         }
-    }
     // tile sums: a float tree within each warp (5 levels), the warps' sums
-    // added in double in a fixed order by thread 0 (FP64 is slow here, so
-    // it is kept off the per-thread path)
+    // added in double in a fixed order, one thread per sum (FP64 is slow
+    // here, so it is kept off the per-thread path)
     const int ncomp = cost == 0 ? 1 : 5;
 #pragma unroll
     for (int k = 0; k < 5; ++k)
@@ -526,23 +532,32 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(FULL, acc[k], o);
             if (lane == 0) wsum[k][wy] = acc[k];
         }
-    __syncthreads();
+    __syncthreads();   // also: every warp is done with the ring
+    if (staged && tid == 0) {
+        // copies still in flight (only after a wait gave up) are waited for
+        // before the block's shared memory is released: only the planes that
+        // were issued, and within one wait limit in total (a pair whose
+        // wait gives up ends the drain)
+        const int issued = nissued;
+        for (; kw < issued; ++kw)
+            if (!mbar_wait(smem_u32(&mbar[kw % NPAIR]), unsigned(kw / NPAIR) & 1u)) {
+                atomicOr(&a.counters[6], 1u);
+                break;
+            }
+    }
+    if (tid < 5) {
+        double v = 0.0;
+        if (tid < ncomp)
+            for (int w = 0; w < NW; ++w) v += widen(wsum[tid][w]);
+        a.tile_sums[size_t(tile) * 5 + tid] = v;
+    }
     // a deferred finalisation (the gather's for SSD, k_finalise3's for NCC)
     // needs no last-block pass here
-    const bool finalise_here = !a.defer_cost;
+    if (a.defer_cost) return;
+    __syncthreads();
     if (tid == 0) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            double v = 0.0;
-            if (k < ncomp)
-                for (int w = 0; w < NT3 / 32; ++w) v += double(wsum[k][w]);
-            a.tile_sums[size_t(tile) * 5 + k] = v;
-        }
-        is_last = false;
-        if (finalise_here) {
-            __threadfence();
-            is_last = (atomicAdd(&a.counters[0], 1u) == unsigned(ntiles - 1));
-        }
+        __threadfence();
+        is_last = (atomicAdd(&a.counters[0], 1u) == unsigned(ntiles - 1));
     }
     __syncthreads();
     if (is_last) {
@@ -1167,7 +1182,7 @@ __device__ __forceinline__ void decode_tile3(const EvalArgs &a, int t, int &bx, 
     nt = ntx * nty * ntz;
 }
 
-template <int TZ>
+template <int TZ, int COST>
 __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_batch(const EvalArgs *__restrict__ args,
                                                                     const int2 *__restrict__ items,
                                                                     const int *__restrict__ active)
@@ -1177,7 +1192,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_batch(const EvalAr
     const EvalArgs &a = args[it.x];
     int bx, by, bz, nt;
     decode_tile3(a, it.y, bx, by, bz, nt);
-    warp3_body<TZ, -1>(a, bx, by, bz, nt, it.y);
+    warp3_body<TZ, COST>(a, bx, by, bz, nt, it.y);
 }
 
 template <int TZ>
@@ -1220,7 +1235,7 @@ __device__ __forceinline__ void queue_done(int *queue)
     }
 }
 
-template <int TZ>
+template <int TZ, int COST>
 __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_queue(const EvalArgs *__restrict__ args,
                                                                     const int2 *__restrict__ items, int nitems,
                                                                     const int *__restrict__ active, int *queue)
@@ -1232,7 +1247,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_queue(const EvalAr
         const EvalArgs &a = args[it.x];
         int bx, by, bz, nt;
         decode_tile3(a, it.y, bx, by, bz, nt);
-        warp3_body<TZ, -1>(a, bx, by, bz, nt, it.y);
+        warp3_body<TZ, COST>(a, bx, by, bz, nt, it.y);
     }
     queue_done(queue);
 }
@@ -1312,8 +1327,7 @@ size_t split3_smem(const EvalArgs &a, int which)
 {
     const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
     if (which == 0)
-        return size_t(3) * Z.fc * Y.fc * (X.fc + TX3) * sizeof(float) + 128 +
-               size_t(RING_N) * RING_PLANE * sizeof(float);
+        return size_t(3) * Z.fc * Y.fc * (X.fc + TX3) * sizeof(float) + size_t(RING_N) * RING_PLANE * sizeof(float);
     return size_t(3) * Z.ac * TY3 * (TX3 + 1 + X.ac) * sizeof(float);
 }
 
@@ -1340,20 +1354,6 @@ bool with_tz(int tz, Fn &&fn)
     }
 }
 
-// the z-tile lengths of the batched and persistent kernels (the
-// registration drivers run 16-plane tiles)
-template <typename Fn>
-bool with_tz_batch(int tz, Fn &&fn)
-{
-    switch (tz) {
-    case 4: fn(std::integral_constant<int, 4>{}); return true;
-    case 8: fn(std::integral_constant<int, 8>{}); return true;
-    case 16: fn(std::integral_constant<int, 16>{}); return true;
-    case 32: fn(std::integral_constant<int, 32>{}); return true;
-    default: return false;
-    }
-}
-
 }  // namespace
 
 bool tile_supported3(int tx, int ty, int tz)
@@ -1361,9 +1361,13 @@ bool tile_supported3(int tx, int ty, int tz)
     return tx == TX3 && ty == TY3 && with_tz(tz, [](auto) {});
 }
 
+// the batched and persistent kernels are compiled for the tile that the
+// registration drivers run (registration_tile)
+constexpr int BATCH_TZ = 16;
+
 bool tile_supported3_batch(int tx, int ty, int tz)
 {
-    return tx == TX3 && ty == TY3 && with_tz_batch(tz, [](auto) {});
+    return tx == TX3 && ty == TY3 && tz == BATCH_TZ;
 }
 
 namespace {
@@ -1388,47 +1392,6 @@ void launch_adjoint3_z(const EvalArgs &a, size_t sm, cudaStream_t st)
 {
     raise_smem_limit(reinterpret_cast<const void *>(k_adjoint3<TZ>), sm);
     launch_pdl(a.pdl != 0, k_adjoint3<TZ>, dim3(a.ax[0].nt, a.ax[1].nt, a.ax[2].nt), dim3(NT3), sm, st, a);
-}
-
-template <int TZ>
-void batch3_z(const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm, int which,
-              cudaStream_t st)
-{
-    if (which == 0)
-        k_warp3_batch<TZ><<<nitems, NT3, sm, st>>>(args, items, active);
-    else
-        k_adjoint3_batch<TZ><<<nitems, NT3, sm, st>>>(args, items, active);
-}
-
-template <int TZ>
-void prepare3_z(size_t sm_warp, size_t sm_adj)
-{
-    cudaFuncSetAttribute(k_warp3_batch<TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_warp));
-    cudaFuncSetAttribute(k_adjoint3_batch<TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_adj));
-    cudaFuncSetAttribute(k_warp3_queue<TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_warp));
-    cudaFuncSetAttribute(k_adjoint3_queue<TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_adj));
-}
-
-// resident blocks of the persistent kernels (blocks per SM x SMs)
-template <int TZ>
-int queue_grid_z(int which, size_t sm)
-{
-    int per_sm = 0;
-    if (which == 0)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_warp3_queue<TZ>, NT3, sm);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint3_queue<TZ>, NT3, sm);
-    return std::max(1, per_sm) * device_sm_count();
-}
-
-template <int TZ>
-void queue3_z(const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue, int grid, size_t sm,
-              int which, cudaStream_t st)
-{
-    if (which == 0)
-        k_warp3_queue<TZ><<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
-    else
-        k_adjoint3_queue<TZ><<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
 }
 
 }  // namespace
@@ -1463,29 +1426,56 @@ void launch_gather3(const EvalArgs &a, int with_gradient, int dense, cudaStream_
     count_launch();
 }
 
-void prepare_split3_batch(int tz, size_t sm_warp, size_t sm_adj)
+namespace {
+
+// the batch's warp kernel by cost
+auto warp3_batch_kernel(int cost)
 {
-    with_tz_batch(tz, [&](auto z) { prepare3_z<decltype(z)::value>(sm_warp, sm_adj); });
+    return cost == MGR_COST_SSD ? k_warp3_batch<BATCH_TZ, MGR_COST_SSD> : k_warp3_batch<BATCH_TZ, MGR_COST_NCC>;
+}
+auto warp3_queue_kernel(int cost)
+{
+    return cost == MGR_COST_SSD ? k_warp3_queue<BATCH_TZ, MGR_COST_SSD> : k_warp3_queue<BATCH_TZ, MGR_COST_NCC>;
 }
 
-void launch_split3_batch(int tz, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
+}  // namespace
+
+void prepare_split3_batch(int cost, size_t sm_warp, size_t sm_adj)
+{
+    raise_smem_limit(reinterpret_cast<const void *>(warp3_batch_kernel(cost)), sm_warp);
+    raise_smem_limit(reinterpret_cast<const void *>(warp3_queue_kernel(cost)), sm_warp);
+    raise_smem_limit(reinterpret_cast<const void *>(k_adjoint3_batch<BATCH_TZ>), sm_adj);
+    raise_smem_limit(reinterpret_cast<const void *>(k_adjoint3_queue<BATCH_TZ>), sm_adj);
+}
+
+void launch_split3_batch(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
                          int which, cudaStream_t st)
 {
-    with_tz_batch(tz, [&](auto z) { batch3_z<decltype(z)::value>(args, items, nitems, active, sm, which, st); });
+    if (which == 0)
+        warp3_batch_kernel(cost)<<<nitems, NT3, sm, st>>>(args, items, active);
+    else
+        k_adjoint3_batch<BATCH_TZ><<<nitems, NT3, sm, st>>>(args, items, active);
     count_launch();
 }
 
-int split3_queue_grid(int tz, int which, size_t sm)
+// resident blocks of the persistent kernels (blocks per SM x SMs)
+int split3_queue_grid(int cost, int which, size_t sm)
 {
-    int g = 0;
-    with_tz_batch(tz, [&](auto z) { g = queue_grid_z<decltype(z)::value>(which, sm); });
-    return g;
+    int per_sm = 0;
+    if (which == 0)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, warp3_queue_kernel(cost), NT3, sm);
+    else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint3_queue<BATCH_TZ>, NT3, sm);
+    return std::max(1, per_sm) * device_sm_count();
 }
 
-void launch_split3_queue(int tz, const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue,
+void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue,
                          int grid, size_t sm, int which, cudaStream_t st)
 {
-    with_tz_batch(tz, [&](auto z) { queue3_z<decltype(z)::value>(args, items, nitems, active, queue, grid, sm, which, st); });
+    if (which == 0)
+        warp3_queue_kernel(cost)<<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
+    else
+        k_adjoint3_queue<BATCH_TZ><<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
     count_launch();
 }
 

@@ -46,6 +46,112 @@ __device__ __noinline__ float taps3_global(const EvalArgs &a, float px, float py
     return sample3(a.coef_img, nx, ny, nz, px, py, pz, mn, mx);
 }
 
+// ---------------------------------------------------------------------
+// Pairs of floats in a 64-bit register pair: one instruction does the
+// arithmetic of both, each rounded as its scalar form rounds.
+// ---------------------------------------------------------------------
+typedef unsigned long long float2x;
+
+__device__ __forceinline__ float2x pack2(float a, float b)
+{
+    float2x r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(float2x v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ float2x add2(float2x a, float2x b)
+{
+    float2x r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x add2_down(float2x a, float2x b)
+{
+    float2x r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x sub2(float2x a, float2x b)
+{
+    float2x r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x mul2(float2x a, float2x b)
+{
+    float2x r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c)
+{
+    float2x r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// ffloor16 of two coordinates below 2^22 in magnitude: rounding to the
+// nearest multiple of 2^-16 before the floor is adding half of one before it,
+// and a sum rounded down at 1.5 * 2^23 has the floor in its low bits: returns
+// the floors as floats, ia / ib the bits of those sums (the integer plus
+// FLOOR_BITS).  Both additions round down, so that neither carries a
+// coordinate over an integer that it does not reach.  A coordinate out of
+// range, infinite or NaN gives some other integer.
+constexpr unsigned FLOOR_BITS = 0x4B400000u;   // 1.5 * 2^23
+__device__ __forceinline__ float2x floor2(float2x p, unsigned &ia, unsigned &ib)
+{
+    const float half = 1.0f / 131072.0f, big = 12582912.0f;
+    const float2x s = add2_down(add2_down(p, pack2(half, half)), pack2(big, big));
+    float a, b;
+    unpack2(s, a, b);
+    ia = __float_as_uint(a);
+    ib = __float_as_uint(b);
+    return sub2(s, pack2(big, big));
+}
+
+// bspline3_weights of two offsets
+__device__ __forceinline__ void bspline3_weights2(float2x f, float2x w[4])
+{
+    const float o6 = 1.0f / 6.0f;
+    const float2x ob6 = pack2(o6, o6);
+    const float2x xm1 = sub2(pack2(1.0f, 1.0f), f);
+    const float2x w0 = mul2(mul2(xm1, xm1), mul2(xm1, ob6));
+    const float2x w3 = mul2(mul2(f, f), mul2(f, ob6));
+    w[0] = w0;
+    w[3] = w3;
+    w[1] = add2(sub2(sub2(xm1, w0), w0), w3);
+    w[2] = add2(sub2(sub2(f, w3), w3), w0);
+}
+
+// minimum and maximum that keep a NaN, of two values and over the warp
+__device__ __forceinline__ float min_nan(float a, float b)
+{
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float warp_min_nan(float v)
+{
+    float r;
+    asm volatile("redux.sync.min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(0xffffffffu));
+    return r;
+}
+__device__ __forceinline__ float warp_max_nan(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(0xffffffffu));
+    return r;
+}
+
 // Shared-memory ring of tap planes of the 3D warp kernel: RING_N planes of
 // RING_Y rows of RING_X floats (a row holds the x extent of a tile's taps
 // plus the alignment of the copies; its pitch is a multiple of the 32

@@ -1,0 +1,70 @@
+"""The 3D warp kernel's walk where it can go wrong: tiles whose last step has
+one plane, one plane in all, taps that just fit the shared-memory ring, just
+do not, or leave the padded copy, and displacements that are not numbers.
+
+Tolerance: as for every warped image (tests/test_gpu_parity.py), 1e-5 of the
+largest value against the oracle at reference precision, costs 1e-5.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _level(size, rate, cost):
+    import mia_gb300 as M
+    from mia_gb300 import synth
+    ref = synth.blob_phantom(size[::-1], 10, sigma=(4.0, 8.0), seed=4)
+    mov = np.roll(ref, 2, axis=2).astype(np.float32)
+    lv = M.Level(size, rate=rate, cost=cost, penalty_weight=1.0)
+    lv.set_images(mov, ref)
+    return lv, mov, ref
+
+
+@pytest.mark.parametrize("size", [(40, 33, 21), (33, 9, 33), (70, 16, 13)])
+@pytest.mark.parametrize("amplitude", [0.0, 1.0, 4.0, 8.0, 14.0, 30.0])
+def test_walk_against_the_oracle(size, amplitude):
+    from oracle import oracle as O
+    from mia_gb300 import synth
+    lv, mov, ref = _level(size, 4.0, "ssd")
+    o = O.Level(size, rate=4.0, cost="ssd", penalty_weight=1.0)
+    o.set_images(mov, ref)
+    # smooth: what varies over a tile grows with the amplitude, up to past
+    # the ring's 10 planes, 16 rows and 64 columns
+    p = synth.smooth_params(lv.csize, amplitude, seed=9)
+    wo, co = o.warp(p), o.evaluate(p)[0]
+    first = None
+    for tz in (4, 8, 12, 16, 20, 24, 32):
+        lv.set_path("split", (32, 8, tz))
+        w = lv.warp(p)
+        assert np.max(np.abs(w - wo)) <= 1e-5 * np.max(np.abs(mov)), tz
+        # a voxel's sample does not depend on the tile that holds it
+        first = w if first is None else first
+        np.testing.assert_array_equal(w, first)
+        assert abs(lv.evaluate(p)[0] - co) <= 1e-5 * co, tz
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 1e30, -3e6])
+def test_displacements_that_are_not_numbers(value):
+    """the device entry point takes parameters as they are: a coefficient
+    that is not a usable number affects its voxels only, and the split path
+    gives the plain path's image cost"""
+    import torch
+    size = (70, 20, 24)
+    lv, mov, ref = _level(size, 6.0, "ssd")
+    p = np.random.default_rng(3).normal(0.0, 1.0, lv.nparams)
+    # in the middle of the grid, the z component
+    c = [n // 2 for n in lv.csize]
+    p[((c[2] * lv.csize[1] + c[1]) * lv.csize[0] + c[0]) * 3 + 2] = value
+    d_p = torch.from_numpy(p).cuda()
+    d_g = torch.empty(lv.nparams, dtype=torch.float64, device="cuda")
+    d_c = torch.empty(2, dtype=torch.float64, device="cuda")
+    cost = []
+    for path in ("plain", "split"):
+        lv.set_path(path)
+        torch.cuda.synchronize()
+        lv.evaluate_device(d_p.data_ptr(), d_g.data_ptr(), d_c.data_ptr())
+        lv.sync()
+        cost.append(d_c.cpu().numpy()[0])
+    assert np.isfinite(cost[0])
+    assert abs(cost[1] - cost[0]) <= 1e-5 * cost[0]
