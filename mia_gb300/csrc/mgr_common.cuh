@@ -292,6 +292,7 @@ constexpr int WARP_RING_PLANES = MGR_RING_PLANES;
 enum {
     SC_VALUE = 0,      // image cost value() (unweighted), NCC with the 1e-10 threshold
     SC_FORCE_COST = 1, // force-pass cost (2D full cost returns this)
+    // the force constants, SC_K1 .. SC_FSCALE, are read as one range
     SC_K1 = 2,         // NCC: 2*cov/(var_a*var_b)  (gradient helper, 1e-5 threshold)
     SC_K2 = 3,         // NCC: cov/var_a
     SC_MA = 4,         // NCC: mean of the warped image

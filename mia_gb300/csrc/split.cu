@@ -259,10 +259,9 @@ __device__ __forceinline__ void adjoint2_body(const EvalArgs &a, int bx, int by,
     pdl_wait();
     pdl_trigger();
     if (tid < 5) {
-        const int slot[5] = {SC_K1, SC_K2, SC_MA, SC_MB, SC_FSCALE};
         // the SSD force scale from the settings, as the finalisation sets it
         // (with a deferred finalisation it is not set yet)
-        if (a.cost != 0) fsc[tid] = float(a.scalars[slot[tid]]);
+        if (a.cost != 0) fsc[tid] = float(a.scalars[SC_K1 + tid]);
         else if (tid == 4) fsc[4] = a.ssd_norm ? float(1.0 / double(size_t(nx) * ny)) : 1.0f;
     }
     // (a lane's x neighbours are the lanes beside it: TX is a multiple of 32)

@@ -1,7 +1,7 @@
 // split3.cu — the 3D split evaluation path.
 //
-// A tile is 32 (x) x 8 (y) x TZ (z) voxels and a block of 256 threads: lane
-// = x, warp = y, and every thread walks its z column.  All threads of a
+// A tile is 32 (x) x 8 (y) x TZ (z) voxels; lane = x, warp = y (the adjoint
+// kernel: two rows), and every thread walks its z column.  All threads of a
 // block stand on the same z plane at the same step, so the z tables are
 // uniform and the per-thread sliding windows below advance in lock step.
 //
@@ -20,9 +20,9 @@
 //       thread samples two planes per step (two independent tap chains in
 //       flight); the warped image is written and the SSD / NCC sums are
 //       accumulated; the last block finalises the cost.
-//   k_adjoint3<TZ>    central differences of the warped image (x neighbours
-//       by warp shuffle, y neighbours from the rows of the adjacent warps, z
-//       neighbours carried in registers; mia/3d/image.cc:347-466), the SSD /
+//   k_adjoint3<TZ>    central differences of the warped image (x and y
+//       neighbours from a ring of planes in shared memory, z neighbours
+//       carried in registers; mia/3d/image.cc:347-466), the SSD /
 //       NCC force (mia/template/ssd.hh:126-181, mia/3d/cost/ncc.cc:88-128),
 //       and the transposed spline contraction (translate,
 //       spline.cc:731-791): z while walking (four running sums per
@@ -47,16 +47,15 @@
 
 #include <type_traits>
 
-// the one-pair adjoint kernel: minimum resident blocks per SM (a cap of 40
-// registers, no spills) and the unroll factor of its plane walk (measured
-// at 192x192x128 SSD and 256^3 NCC against no unroll and no cap; the
-// batched kernels keep both off)
+// the adjoint kernel: resident blocks per SM and planes of its ring (five
+// blocks with four planes; six with three, at 72 registers, took 387 instead
+// of 382 us per 256^3 NCC evaluation, five planes as long as four)
 #ifndef MGR_ADJ_MINB
-#define MGR_ADJ_MINB 6
+#define MGR_ADJ_MINB 5
 #endif
-#define MGR_ADJ_BOUNDS __launch_bounds__(NT3, MGR_ADJ_MINB)
-#ifndef MGR_ADJ_UNROLL
-#define MGR_ADJ_UNROLL 2
+#define MGR_ADJ_BOUNDS __launch_bounds__(AT3, MGR_ADJ_MINB)
+#ifndef MGR_ADJ_PLANES
+#define MGR_ADJ_PLANES 4
 #endif
 
 namespace mgr {
@@ -65,7 +64,13 @@ void set_last_error(const std::string &msg);
 
 namespace {
 
-constexpr int NT3 = 256;   // threads per tile block: 8 warps
+constexpr int NT3 = 256;   // threads per tile block of the warp kernel: 8 warps
+constexpr int AT3 = 128;   // of the adjoint kernel: 4 warps, two rows each
+// the adjoint kernel's ring: per warp AD planes of 4 rows of the warped image
+// (AD_W floats: x0 - 1 .. x0 + 32, padded) and 2 of the reference
+constexpr int AD = MGR_ADJ_PLANES;
+constexpr int AD_W = 36;
+constexpr int AD_PLANE = 4 * AD_W + 2 * 32;
 constexpr int TX3 = 32;    // tile x (lanes)
 constexpr int TY3 = 8;     // tile y (warps)
 constexpr unsigned FULL = 0xffffffffu;
@@ -570,118 +575,183 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
 // ---------------------------------------------------------------------
 // gradient + force + adjoint
 // ---------------------------------------------------------------------
-template <int TZ, int UNROLL>
+// A thread walks two columns, rows 2w and 2w + 1 of the tile for warp w: the
+// two rows' arithmetic runs on register pairs, they share the loop, the
+// tables and each other's values.  Each warp copies the planes it needs (its
+// rows, the ones above and below, the rows' ends, the reference) into a ring
+// of its own, ahead of the walk and without a block barrier.  What bounds the
+// walk is the latency of those reads, one plane after another: with loads a
+// plane ahead in registers a plane took 0.7 us.  Where the image ends, a
+// neighbour's offset names the voxel that makes the difference 0 (y), or a
+// second scale is 0 (x), so the walk has no branch on it.  Against one row per
+// thread with loads at their use, alone on the GPU: 256^3 NCC 93 -> 74 us,
+// 383x351x317 SSD 180 -> 137 us; 192x192x128 SSD 30 -> 29 us (1008 tiles are
+// 1.3 waves, a block's chain of stages is its time).
+template <int TZ>
 __device__ __forceinline__ void adjoint3_body(const EvalArgs &a, int bx, int by, int bz, int tile_index)
 {
-    const int cost = a.cost;   // (a per-cost NCC kernel spills under the register cap)
-    extern __shared__ __align__(16) float sm3[];
+    const int cost = a.cost;
+    extern __shared__ __align__(16) float sm3a[];
     __shared__ int asx[TX3], asy[TY3], azs[TZ];
     __shared__ float fsc[5];   // force constants (converted once per block)
-    __shared__ float4 awx[TX3], awy[TY3], azw[TZ];
+    __shared__ float4 awx[TX3][2], awy[TY3][2], azw[TZ][2];   // each weight twice, {x, x, y, y}, {z, z, w, w}
     const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
     const int nx = a.n[0], ny = a.n[1], nz = a.n[2];
     const int x0 = bx * TX3, y0 = by * TY3, z0 = bz * TZ;
-    const int ex = min(TX3, nx - x0), ey = min(TY3, ny - y0), ez = min(TZ, nz - z0);
+    const int ey = min(TY3, ny - y0), ez = min(TZ, nz - z0);
     const int AXc = X.ac, AYc = Y.ac, AZc = Z.ac;
     const int ax0 = X.atile0[bx], ay0 = Y.atile0[by], az0 = Z.atile0[bz];
     const int tid = threadIdx.x, lane = tid & 31, wy = tid >> 5;
     float *part = a.partial + size_t(tile_index) * a.slot;
     constexpr int AZP = TX3 + 1;              // Az row pitch (odd: the x stage reads along the rows)
-    float *Az = sm3;                          // [3][AZc][8][AZP]
-    float *Ax = Az + 3 * AZc * TY3 * AZP;     // [3][AZc][8][AXc]
+    float2x *Az = reinterpret_cast<float2x *>(sm3a);                   // [3][AZc][4][AZP], the rows in pairs
+    float *Ax = sm3a + 3 * AZc * TY3 * AZP;                            // [3][AZc][8][AXc], in the ring's place
+    float *ring = sm3a + 3 * AZc * TY3 * AZP + wy * (AD * AD_PLANE);   // [AD][AD_PLANE] of this warp
 
-    // tables, scalars and the first planes of the column, loaded up front
-    const int x = x0 + lane, y = y0 + wy;
-    const bool inxy = x < nx && y < ny;
-    const size_t nxy = size_t(nx) * ny;
-    const size_t col = size_t(min(y, ny - 1)) * nx + min(x, nx - 1);
-    const float *__restrict__ W = a.warped;
-    const float *__restrict__ R = a.ref;
-    const bool bx_in = x > 0 && x < nx - 1, by_in = y > 0 && y < ny - 1;
-    // column pointers at the current plane
-    const float *__restrict__ wc = W + size_t(z0) * nxy + col;
-    const float *__restrict__ rc = R + size_t(z0) * nxy + col;
-    const int ynm = (y > 0) ? -nx : 0, ynp = (y + 1 < ny) ? nx : 0;
+    // tables and scalars, loaded up front
+    auto twice = [](float4 (&d)[2], const float4 &w) {
+        d[0] = make_float4(w.x, w.x, w.y, w.y);
+        d[1] = make_float4(w.z, w.z, w.w, w.w);
+    };
     if (tid < TX3) {
         const int xx = min(x0 + tid, nx - 1);
         asx[tid] = X.as[xx] - ax0;
-        awx[tid] = X.aw[xx];
+        twice(awx[tid], X.aw[xx]);
+    } else if (tid < TX3 + TY3) {
+        const int k = tid - TX3, yy = min(y0 + k, ny - 1);
+        asy[k] = Y.as[yy] - ay0;
+        twice(awy[k], Y.aw[yy]);
+    } else if (tid >= 64 && tid < 64 + TZ) {
+        const int k = tid - 64, zz = min(z0 + k, nz - 1);
+        azs[k] = Z.as[zz] - az0;
+        twice(azw[k], Z.aw[zz]);
     }
-    if (tid < TY3) {
-        const int yy = min(y0 + tid, ny - 1);
-        asy[tid] = Y.as[yy] - ay0;
-        awy[tid] = Y.aw[yy];
-    }
-    if (tid < TZ) {
-        const int zz = min(z0 + tid, nz - 1);
-        azs[tid] = Z.as[zz] - az0;
-        azw[tid] = Z.aw[zz];
-    }
+    // the two columns (clamped to the image; their scale is 0 beyond it) and
+    // the offsets of their neighbours in a plane
+    const int x = x0 + lane, ya = y0 + 2 * wy, yb = ya + 1;
+    const size_t nxy = size_t(nx) * ny;
+    const int xc = min(x, nx - 1);
+    const unsigned oa = unsigned(min(ya, ny - 1) * nx + xc), ob = unsigned(min(yb, ny - 1) * nx + xc);
+    const unsigned ou = ya > 0 && ya < ny - 1 ? oa - unsigned(nx) : ob;   // above row a (row b is below it)
+    const unsigned od = yb < ny - 1 ? ob + unsigned(nx) : oa;             // below row b (row a is above it)
+    // lanes 0..3 also copy the rows' ends: (row a, row b) x (left, right)
+    const int xe = lane & 1 ? min(x0 + TX3, nx - 1) : max(x0 - 1, 0);
+    const unsigned oe = (lane & 2 ? ob : oa) - unsigned(xc) + unsigned(xe);
+    const float *wsrc = a.warped + size_t(z0) * nxy;   // the next plane to copy
+    const float *rsrc = a.ref + size_t(z0) * nxy;
+    const unsigned sring = smem_u32(ring) + 4u * unsigned(lane);
+    const unsigned sedge = smem_u32(ring) + 4u * unsigned((lane & 2 ? 2 : 1) * AD_W + (lane & 1 ? TX3 + 1 : 0));
+    auto copy4 = [](unsigned dst, const float *src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+    };
+    // plane p of the tile into its slot: those the walk reads, up to the one
+    // behind the last if the image has it; a group is committed for every p
+    const int np = min(ez + 1, nz - z0);
+    auto issue = [&](int p, unsigned slot) {
+        if (p < np) {
+            const unsigned d = sring + slot;
+            copy4(d + 4u, wsrc + ou);
+            copy4(d + 4u * (AD_W + 1), wsrc + oa);
+            copy4(d + 4u * (2 * AD_W + 1), wsrc + ob);
+            copy4(d + 4u * (3 * AD_W + 1), wsrc + od);
+            if (lane < 4) copy4(sedge + slot, wsrc + oe);
+            copy4(d + 4u * (4 * AD_W), rsrc + oa);
+            copy4(d + 4u * (4 * AD_W + 32), rsrc + ob);
+            wsrc += nxy;
+            rsrc += nxy;
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
     // the warped image and the cost's scalars come from the warp kernel
     pdl_wait();
     pdl_trigger();
+    float2x wm = 0;
+    if (z0 > 0) wm = pack2(__ldcg(wsrc - nxy + oa), __ldcg(wsrc - nxy + ob));
+#pragma unroll
+    for (int p = 0; p < AD - 1; ++p) issue(p, unsigned(p) * (AD_PLANE * 4u));
     if (tid < 5) {
-        const int slot[5] = {SC_K1, SC_K2, SC_MA, SC_MB, SC_FSCALE};
-        fsc[tid] = float(a.scalars[slot[tid]]);
         // the SSD force scale from the settings, as the finalisation sets it
         // (with a deferred finalisation it is not set yet)
-        if (tid == 4 && cost == 0) fsc[4] = a.ssd_norm ? float(1.0 / double(size_t(nx) * ny * nz)) : 1.0f;
+        if (cost != 0) fsc[tid] = float(a.scalars[SC_K1 + tid]);
+        else if (tid == 4) fsc[4] = a.ssd_norm ? float(1.0 / double(size_t(nx) * ny * nz)) : 1.0f;
     }
-    float wm = (z0 > 0) ? __ldg(wc - nxy) : 0.0f;
-    float w0 = __ldg(wc);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(AD - 2) : "memory");   // plane 0
     __syncthreads();
-    const float k1 = fsc[0], k2 = fsc[1], ma = fsc[2], mb = fsc[3], hscale = 0.5f * fsc[4];
+    // central differences are taken without their factor 1/2, which joins
+    // the force's scale
+    const bool ina = x < nx && ya < ny, inb = x < nx && yb < ny;
+    float2x hs, k1 = 0, k2 = 0, ma = 0, mb = 0;
+    if (cost == 0) {
+        const float h = 0.5f * fsc[4];
+        hs = pack2(ina ? h : 0.0f, inb ? h : 0.0f);
+    } else {
+        hs = pack2(ina ? 0.5f : 0.0f, inb ? 0.5f : 0.0f);
+        k1 = pack2(fsc[0], fsc[0]);
+        k2 = pack2(fsc[1], fsc[1]);
+        ma = pack2(fsc[2], fsc[2]);
+        mb = pack2(fsc[3], fsc[3]);
+    }
 
-    float acc[3][4];
+    const float2x hx = x > 0 && x < nx - 1 ? hs : 0;   // no x difference at the image's border
+
+    float2x acc[3][4];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[c][k] = 0.0f;
+        for (int k = 0; k < 4; ++k) acc[c][k] = 0;
     int cur = 0;   // azs[0] == 0
-    auto emit = [&](int kz, int c, float v) { Az[((c * AZc + kz) * TY3 + wy) * AZP + lane] = v; };
-#pragma unroll UNROLL
+    float2x *const az = Az + wy * AZP + lane;
+    auto emit = [&](int kz, int c, float2x v) { az[(c * AZc + kz) * (TY3 / 2 * AZP)] = v; };
+    const float *rp = ring + lane;   // plane t's slot
+    float2x w0 = pack2(rp[AD_W + 1], rp[2 * AD_W + 1]);
+    unsigned fill = (AD - 1) * (AD_PLANE * 4u);   // the slot that plane t - 1 has left
+    int at = 0;                                   // t modulo AD
+#pragma unroll 1
     for (int t = 0; t < ez; ++t) {
         const int z = z0 + t;
-        const float wp = (z + 1 < nz) ? __ldg(wc + nxy) : 0.0f;
-        float left = __shfl_up_sync(FULL, w0, 1), right = __shfl_down_sync(FULL, w0, 1);
-        if (lane == 0 && x > 0) left = __ldg(wc - 1);
-        if (lane == TX3 - 1 && x + 1 < nx) right = __ldg(wc + 1);
-        float f[3] = {0.0f, 0.0f, 0.0f};
-        if (inxy) {
-            const float ym = __ldg(wc + ynm), yp = __ldg(wc + ynp);
-            float g[3];
-            // central differences without their factor 1/2, which joins
-            // the force's scale
-            g[0] = bx_in ? right - left : 0.0f;
-            g[1] = by_in ? yp - ym : 0.0f;
-            g[2] = (z > 0 && z < nz - 1) ? wp - wm : 0.0f;
-            const float b = __ldg(rc);
-            const float s = cost == 0 ? (w0 - b) * hscale : 0.5f * (k1 * (k2 * (w0 - ma) - (b - mb)));
-#pragma unroll
-            for (int k = 0; k < 3; ++k) f[k] = g[k] * s;
-        }
-        wc += nxy;
-        rc += nxy;
-        const int s = azs[t];
-        while (cur < s) {   // uniform over the block
+        issue(t + AD - 1, fill);
+        fill = fill == (AD - 1) * (AD_PLANE * 4u) ? 0u : fill + AD_PLANE * 4u;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(AD - 2) : "memory");   // plane t + 1
+        __syncwarp();
+        at = at == AD - 1 ? 0 : at + 1;
+        const float *rn = ring + at * AD_PLANE + lane;
+        const float2x wp = pack2(rn[AD_W + 1], rn[2 * AD_W + 1]);
+        const float2x left = pack2(rp[AD_W], rp[2 * AD_W]), right = pack2(rp[AD_W + 2], rp[2 * AD_W + 2]);
+        const float up = rp[1], down = rp[3 * AD_W + 1];
+        const float2x b = pack2(rp[4 * AD_W], rp[4 * AD_W + 32]);
+        rp = rn;
+        __syncwarp();   // every lane has plane t: its slot is free
+        float wa, wb;
+        unpack2(w0, wa, wb);
+        // the force's factor at the voxel, times the scale
+        float2x d;
+        if (cost == 0)
+            d = sub2(w0, b);
+        else
+            d = mul2(k1, fma2(k2, sub2(w0, ma), sub2(mb, b)));
+        const float2x s = mul2(d, hs);
+        float2x f[3];
+        f[0] = mul2(sub2(right, left), mul2(d, hx));
+        f[1] = mul2(sub2(pack2(wb, down), pack2(up, wa)), s);
+        f[2] = z > 0 && z < nz - 1 ? mul2(sub2(wp, wm), s) : 0;
+        const int sz = azs[t];
+        while (cur < sz) {   // uniform over the block
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 emit(cur, c, acc[c][0]);
                 acc[c][0] = acc[c][1];
                 acc[c][1] = acc[c][2];
                 acc[c][2] = acc[c][3];
-                acc[c][3] = 0.0f;
+                acc[c][3] = 0;
             }
             ++cur;
         }
-        const float4 w = azw[t];
+        const float4 u = azw[t][0], v = azw[t][1];
+        const float2x w4[4] = {pack2(u.x, u.y), pack2(u.z, u.w), pack2(v.x, v.y), pack2(v.z, v.w)};
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            acc[c][0] += w.x * f[c];
-            acc[c][1] += w.y * f[c];
-            acc[c][2] += w.z * f[c];
-            acc[c][3] += w.w * f[c];
-        }
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[c][k] = fma2(w4[k], f[c], acc[c][k]);
         wm = w0;
         w0 = wp;
     }
@@ -692,80 +762,78 @@ __device__ __forceinline__ void adjoint3_body(const EvalArgs &a, int bx, int by,
             for (int c = 0; c < 3; ++c) emit(cur + k, c, acc[c][k]);
     for (int kz = cur + 4; kz < AZc; ++kz)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) emit(kz, c, 0.0f);
+        for (int c = 0; c < 3; ++c) emit(kz, c, 0);
     __syncthreads();
-    // x stage, one thread per (c, kz, row) row of Az: the transposed
-    // contraction over the tile's columns as a sliding window of four sums
-    // (the column starts are the same for every thread, so the window moves
-    // in lock step).  Contracting x before y keeps the intermediate small
-    // (AXc instead of 32 values per row): the block needs less shared
-    // memory and the two stages fewer instructions.
-    for (int e = tid; e < 3 * AZc * TY3; e += NT3) {
-        if ((e & (TY3 - 1)) >= ey) continue;   // rows below the image: never read
-        const float *src = Az + e * AZP;
-        float *dst = Ax + e * AXc;
-        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+    // the transposed contraction of a line of `len` pairs onto nout
+    // coefficients as a sliding window of four sums (the starts are the same
+    // for every thread, so the window moves in lock step); entry l of the
+    // line from in(l), coefficient o to out(o, sum)
+    auto contract = [](int len, const int *start, const float4 (*w)[2], int nout, auto in, auto out) {
+        float2x s0 = 0, s1 = 0, s2 = 0, s3 = 0;
         int oc = 0;
-        // all TX3 columns: the walk leaves 0 in the columns beyond the image,
-        // whose coefficient start is the last column's
-#pragma unroll 8
-        for (int l = 0; l < TX3; ++l) {
-            const int o = asx[l];
+        auto step = [&](int l) {
+            const int o = start[l];
             while (oc < o) {
-                dst[oc] = s0;
+                out(oc, s0);
                 s0 = s1;
                 s1 = s2;
                 s2 = s3;
-                s3 = 0.0f;
+                s3 = 0;
                 ++oc;
             }
-            const float4 w = awx[l];
-            const float f = src[l];
-            s0 += w.x * f;
-            s1 += w.y * f;
-            s2 += w.z * f;
-            s3 += w.w * f;
-        }
-        if (oc < AXc) dst[oc] = s0;
-        if (oc + 1 < AXc) dst[oc + 1] = s1;
-        if (oc + 2 < AXc) dst[oc + 2] = s2;
-        if (oc + 3 < AXc) dst[oc + 3] = s3;
-        for (int ix = oc + 4; ix < AXc; ++ix) dst[ix] = 0.0f;
+            const float4 u = w[l][0], v = w[l][1];
+            const float2x f = in(l);
+            s0 = fma2(pack2(u.x, u.y), f, s0);
+            s1 = fma2(pack2(u.z, u.w), f, s1);
+            s2 = fma2(pack2(v.x, v.y), f, s2);
+            s3 = fma2(pack2(v.z, v.w), f, s3);
+        };
+        int l = 0;
+        for (; l + 8 <= len; l += 8)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) step(l + j);
+        for (; l < len; ++l) step(l);
+        if (oc < nout) out(oc, s0);
+        if (oc + 1 < nout) out(oc + 1, s1);
+        if (oc + 2 < nout) out(oc + 2, s2);
+        if (oc + 3 < nout) out(oc + 3, s3);
+        for (int o = oc + 4; o < nout; ++o) out(o, 0);
+    };
+    // x stage, one thread per (c, kz, row pair) line of Az, all TX3 columns
+    // (the walk leaves 0 in the columns beyond the image, whose coefficient
+    // start is the last column's).  Contracting x before y keeps the
+    // intermediate small (AXc instead of 32 values per row): the block needs
+    // less shared memory and the two stages fewer instructions.
+    for (int e = tid; e < 3 * AZc * (TY3 / 2); e += AT3) {
+        if (2 * (e & (TY3 / 2 - 1)) >= ey) continue;   // rows below the image: never read
+        const float2x *src = Az + e * AZP;
+        float *dst = Ax + 2 * e * AXc;
+        contract(TX3, asx, awx, AXc, [&](int l) { return src[l]; },
+                 [&](int o, float2x v) { unpack2(v, dst[o], dst[AXc + o]); });
     }
     __syncthreads();
-    // y stage, one thread per (c, kz, ix) column of Ax, the same sliding
-    // window over the rows, straight into the partial slot
-    // ((kz AYc + jy) AXc + ix) 3 + c
-    for (int e = tid; e < 3 * AZc * AXc; e += NT3) {
-        const int c = e / (AZc * AXc), r = e - c * (AZc * AXc);
-        const int kz = r / AXc, ix = r - kz * AXc;
-        const float *src = Ax + (c * AZc + kz) * TY3 * AXc + ix;
-        float *dst = part + (size_t(kz) * AYc * AXc + ix) * 3 + c;
-        const int pitch = AXc * 3;
-        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-        int oc = 0;
-        for (int yy = 0; yy < ey; ++yy) {
-            const int o = asy[yy];
-            while (oc < o) {
-                dst[oc * pitch] = s0;
-                s0 = s1;
-                s1 = s2;
-                s2 = s3;
-                s3 = 0.0f;
-                ++oc;
-            }
-            const float4 w = awy[yy];
-            const float f = src[yy * AXc];
-            s0 += w.x * f;
-            s1 += w.y * f;
-            s2 += w.z * f;
-            s3 += w.w * f;
-        }
-        if (oc < AYc) dst[oc * pitch] = s0;
-        if (oc + 1 < AYc) dst[(oc + 1) * pitch] = s1;
-        if (oc + 2 < AYc) dst[(oc + 2) * pitch] = s2;
-        if (oc + 3 < AYc) dst[(oc + 3) * pitch] = s3;
-        for (int jy = oc + 4; jy < AYc; ++jy) dst[jy * pitch] = 0.0f;
+    // y stage, one thread per two (c, kz, ix) columns of Ax, straight into the
+    // partial slot ((kz AYc + jy) AXc + ix) 3 + c
+    const int ncol = 3 * AZc * AXc, half = (ncol + 1) / 2;
+    auto column = [&](int q, const float *&src, float *&dst) {
+        const int r = q / AXc, ix = q - r * AXc;   // r = c AZc + kz
+        const int c = r / AZc, kz = r - c * AZc;
+        src = Ax + r * TY3 * AXc + ix;
+        dst = part + (size_t(kz) * AYc * AXc + ix) * 3 + c;
+    };
+    for (int e = tid; e < half; e += AT3) {
+        const bool two = e + half < ncol;
+        const float *src0, *src1;
+        float *dst0, *dst1;
+        column(e, src0, dst0);
+        column(two ? e + half : e, src1, dst1);
+        contract(ey, asy, awy, AYc, [&](int l) { return pack2(src0[l * AXc], src1[l * AXc]); },
+                 [&](int o, float2x v) {
+                     float p, q;
+                     unpack2(v, p, q);
+                     dst0[o * AXc * 3] = p;
+                     if (two) dst1[o * AXc * 3] = q;
+                 });
     }
 }
 
@@ -1152,7 +1220,7 @@ template <int TZ>
 __global__ void MGR_ADJ_BOUNDS k_adjoint3(EvalArgs a)
 {
     const int tile = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    adjoint3_body<TZ, MGR_ADJ_UNROLL>(a, blockIdx.x, blockIdx.y, blockIdx.z, tile);
+    adjoint3_body<TZ>(a, blockIdx.x, blockIdx.y, blockIdx.z, tile);
 }
 
 __global__ void MGR_GATHER_BOUNDS k_gather3(EvalArgs a, int with_gradient, int image_from_dense)
@@ -1196,7 +1264,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_batch(const EvalAr
 }
 
 template <int TZ>
-__global__ void __launch_bounds__(NT3) k_adjoint3_batch(const EvalArgs *__restrict__ args,
+__global__ void MGR_ADJ_BOUNDS k_adjoint3_batch(const EvalArgs *__restrict__ args,
                                                         const int2 *__restrict__ items, const int *__restrict__ active)
 {
     const int2 it = items[blockIdx.x];
@@ -1204,7 +1272,7 @@ __global__ void __launch_bounds__(NT3) k_adjoint3_batch(const EvalArgs *__restri
     const EvalArgs &a = args[it.x];
     int bx, by, bz, nt;
     decode_tile3(a, it.y, bx, by, bz, nt);
-    adjoint3_body<TZ, 1>(a, bx, by, bz, it.y);
+    adjoint3_body<TZ>(a, bx, by, bz, it.y);
 }
 
 // Persistent forms of the batched warp and adjoint kernels: a grid of
@@ -1253,7 +1321,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_queue(const EvalAr
 }
 
 template <int TZ>
-__global__ void __launch_bounds__(NT3) k_adjoint3_queue(const EvalArgs *__restrict__ args,
+__global__ void MGR_ADJ_BOUNDS k_adjoint3_queue(const EvalArgs *__restrict__ args,
                                                         const int2 *__restrict__ items, int nitems,
                                                         const int *__restrict__ active, int *queue)
 {
@@ -1264,7 +1332,7 @@ __global__ void __launch_bounds__(NT3) k_adjoint3_queue(const EvalArgs *__restri
         const EvalArgs &a = args[it.x];
         int bx, by, bz, nt;
         decode_tile3(a, it.y, bx, by, bz, nt);
-        adjoint3_body<TZ, 1>(a, bx, by, bz, it.y);
+        adjoint3_body<TZ>(a, bx, by, bz, it.y);
     }
     queue_done(queue);
 }
@@ -1328,7 +1396,9 @@ size_t split3_smem(const EvalArgs &a, int which)
     const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
     if (which == 0)
         return size_t(3) * Z.fc * Y.fc * (X.fc + TX3) * sizeof(float) + size_t(RING_N) * RING_PLANE * sizeof(float);
-    return size_t(3) * Z.ac * TY3 * (TX3 + 1 + X.ac) * sizeof(float);
+    return (size_t(3) * Z.ac * TY3 * (TX3 + 1) +
+            std::max(size_t(3) * Z.ac * TY3 * X.ac, size_t(AT3 / 32) * AD * AD_PLANE)) *
+           sizeof(float);
 }
 
 namespace {
@@ -1391,7 +1461,7 @@ template <int TZ>
 void launch_adjoint3_z(const EvalArgs &a, size_t sm, cudaStream_t st)
 {
     raise_smem_limit(reinterpret_cast<const void *>(k_adjoint3<TZ>), sm);
-    launch_pdl(a.pdl != 0, k_adjoint3<TZ>, dim3(a.ax[0].nt, a.ax[1].nt, a.ax[2].nt), dim3(NT3), sm, st, a);
+    launch_pdl(a.pdl != 0, k_adjoint3<TZ>, dim3(a.ax[0].nt, a.ax[1].nt, a.ax[2].nt), dim3(AT3), sm, st, a);
 }
 
 }  // namespace
@@ -1454,7 +1524,7 @@ void launch_split3_batch(int cost, const EvalArgs *args, const int2 *items, int 
     if (which == 0)
         warp3_batch_kernel(cost)<<<nitems, NT3, sm, st>>>(args, items, active);
     else
-        k_adjoint3_batch<BATCH_TZ><<<nitems, NT3, sm, st>>>(args, items, active);
+        k_adjoint3_batch<BATCH_TZ><<<nitems, AT3, sm, st>>>(args, items, active);
     count_launch();
 }
 
@@ -1465,7 +1535,7 @@ int split3_queue_grid(int cost, int which, size_t sm)
     if (which == 0)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, warp3_queue_kernel(cost), NT3, sm);
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint3_queue<BATCH_TZ>, NT3, sm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint3_queue<BATCH_TZ>, AT3, sm);
     return std::max(1, per_sm) * device_sm_count();
 }
 
@@ -1475,7 +1545,7 @@ void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int 
     if (which == 0)
         warp3_queue_kernel(cost)<<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
     else
-        k_adjoint3_queue<BATCH_TZ><<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
+        k_adjoint3_queue<BATCH_TZ><<<grid, AT3, sm, st>>>(args, items, nitems, active, queue);
     count_launch();
 }
 
