@@ -183,28 +183,6 @@ static void check_launch(const char *what)
 
 using namespace mgr;
 
-// the divcurl penalty table of the level's grid (3D: translation-invariant
-// cells; 2D: boundary-clipped CSR rows, cached across levels of equal grid)
-static void build_penalty(mgr_level *L)
-{
-    const mgr_level_desc &d = L->d;
-    if (!d.has_penalty) return;
-    const float range[3] = {float(d.size[0]), float(d.size[1]), float(d.dim == 3 ? d.size[2] : 1)};
-    if (d.dim == 3) {
-        std::vector<float> P = build_penalty3(L->nc, range, d.pen_div, d.pen_curl);
-        L->ptable.release();   // kernels queued earlier may still read the old table
-        L->ptable.upload(P, L->stream);
-    } else {
-        const auto t = penalty2_cached(L->nc, range, d.pen_div, d.pen_curl);
-        L->pen_rowptr.release();
-        L->pen_col.release();
-        L->pen_val.release();
-        L->pen_rowptr.upload(t->rowptr, L->stream);
-        L->pen_col.upload(t->col, L->stream);
-        L->pen_val.upload(t->val, L->stream);
-    }
-}
-
 namespace mgr {
 // A new coefficient grid on a level whose images stay (the second pass of a
 // registration level after refine): parameter buffers, tables and penalty
@@ -222,19 +200,10 @@ void level_set_grid(mgr_level *L, const int csize[3], const int tile[3])
     L->ncoef = size_t(L->nc[0]) * L->nc[1] * L->nc[2];
     L->nparams = L->ncoef * D;
     for (int k = 0; k < 3; ++k) L->tile[k] = tile[k];
-    L->params.release();
-    L->params_f.release();
-    L->grad_total.release();
     L->grad_image.release();
     L->grad_penalty.release();
-    L->params.alloc(L->nparams, L->stream);
-    L->params_f.alloc(L->nparams, L->stream);
-    L->grad_total.alloc(L->nparams, L->stream);
-    L->partial.release();
-    L->tile_sums.release();
-    L->pen_part.release();
+    L->build_penalty();
     L->build_tables();
-    build_penalty(L);
     check_launch("level set grid");
 }
 mgr_level *level_create_on_images(const mgr_level *S, const int csize[3], cudaStream_t st)
@@ -262,16 +231,9 @@ mgr_level *level_create_on_images(const mgr_level *S, const int csize[3], cudaSt
     L->stream = st;
     L->images_from = S;
     L->images_set = true;
-    L->params.alloc(L->nparams, st);
-    L->params_f.alloc(L->nparams, st);
-    L->grad_total.alloc(L->nparams, st);
-    L->scalars.alloc(SC_NSLOTS, st);
-    L->costs.alloc(2, st);
-    L->counters.alloc(8, st);
-    ck(cudaMemsetAsync(L->counters.p, 0, 8 * sizeof(unsigned), st), "memset");
-    ck(cudaMemsetAsync(L->scalars.p, 0, SC_NSLOTS * sizeof(double), st), "memset");
+    L->alloc_state();
+    L->build_penalty();
     L->build_tables();
-    build_penalty(L.get());
     check_launch("level create on images");
     return L.release();
 }
@@ -294,6 +256,13 @@ mgr_status mgr_debug_fail_allocation(long long k)
 unsigned long long mgr_allocation_count(void) { return g_allocs.load(); }
 
 mgr_status mgr_level_create(const mgr_level_desc *desc, int device, void *stream, mgr_level **out)
+{
+    return level_create(desc, device, stream, nullptr, out);
+}
+
+}  // extern "C"
+
+mgr_status mgr::level_create(const mgr_level_desc *desc, int device, void *stream, const int *tile, mgr_level **out)
 {
     if (!desc || !out) return fail(MGR_ERR_ARG, "null argument");
     *out = nullptr;
@@ -325,7 +294,10 @@ mgr_status mgr_level_create(const mgr_level_desc *desc, int device, void *stream
         L->N = size_t(L->n[0]) * L->n[1] * L->n[2];
         L->ncoef = size_t(L->nc[0]) * L->nc[1] * L->nc[2];
         L->nparams = L->ncoef * d.dim;
-        L->choose_tile();
+        if (tile && L->tile_fits(tile, false))
+            for (int k = 0; k < 3; ++k) L->tile[k] = tile[k];
+        else
+            L->choose_tile();
         L->device = device;
         ck(cudaSetDevice(device), "cudaSetDevice");
         configure_pool(device);
@@ -340,32 +312,27 @@ mgr_status mgr_level_create(const mgr_level_desc *desc, int device, void *stream
             ck(cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking), "cudaStreamCreate");
             L->own_stream = true;
         }
-        L->coef.alloc(L->N, L->stream);
-        L->coef_pad.alloc(pad_floats(d.dim, L->n[0], L->n[1], L->n[2]), L->stream);
+        alloc_together(L->slab_images, L->stream, [&](auto buf) {
+            buf(L->coef, L->N);
+            buf(L->coef_pad, pad_floats(d.dim, L->n[0], L->n[1], L->n[2]));
+            buf(L->ref, L->N);
+            buf(L->warped, L->N);
+            buf(L->minmax, 2);
+            buf(L->mmpart, size_t(prefilter_x_blocks(d.dim, L->n[0], L->n[1], L->n[2])));
+            buf(L->mpart, d.cost == MGR_COST_NCC ? 2 * 1024 : 0);
+        });
         if (d.dim == 3) L->has_tmap = encode_pad_tmap(&L->tmap, L->coef_pad.p, L->n[0], L->n[1], L->n[2]);
-        L->ref.alloc(L->N, L->stream);
-        L->warped.alloc(L->N, L->stream);
-        L->minmax.alloc(2, L->stream);
-        L->mmpart.alloc(prefilter_x_blocks(d.dim, L->n[0], L->n[1], L->n[2]), L->stream);
-        L->params.alloc(L->nparams, L->stream);
-        L->params_f.alloc(L->nparams, L->stream);
-        L->grad_total.alloc(L->nparams, L->stream);
-        L->scalars.alloc(SC_NSLOTS, L->stream);
-        L->costs.alloc(2, L->stream);
-        L->means.alloc(2, L->stream);
-        ck(cudaMemsetAsync(L->means.p, 0, 2 * sizeof(double), L->stream), "memset");
-        if (d.cost == MGR_COST_NCC) L->mpart.alloc(2 * 1024, L->stream);
-        L->counters.alloc(8, L->stream);
-        ck(cudaMemsetAsync(L->counters.p, 0, 8 * sizeof(unsigned), L->stream), "memset");
-        ck(cudaMemsetAsync(L->scalars.p, 0, SC_NSLOTS * sizeof(double), L->stream), "memset");
+        L->alloc_state();
+        L->build_penalty();
         L->build_tables();
-        build_penalty(L.get());
         check_launch("level create");
     });
     if (st == MGR_OK) *out = L.release();
     else mgr_level_destroy(L.release());   // buffers made so far, and a stream the level created
     return st;
 }
+
+extern "C" {
 
 mgr_status mgr_level_destroy(mgr_level *lvl)
 {
@@ -557,7 +524,6 @@ mgr_status mgr_level_set_images(mgr_level *lvl, const float *src, const float *r
             if (!std::isfinite(src[i]) || !std::isfinite(ref[i]))
                 throw std::invalid_argument("images must be finite");
         ck(cudaSetDevice(lvl->device), "cudaSetDevice");
-        lvl->warped.alloc(lvl->N, lvl->stream);
         ck(cudaMemcpyAsync(lvl->warped.p, src, lvl->N * sizeof(float), cudaMemcpyHostToDevice, lvl->stream), "src");
         ck(cudaMemcpyAsync(lvl->ref.p, ref, lvl->N * sizeof(float), cudaMemcpyHostToDevice, lvl->stream), "ref");
         set_images_impl(lvl, lvl->warped.p, lvl->ref.p);

@@ -337,6 +337,11 @@ __global__ void k_count_active(const MinState *st, int npairs, int *count)
     if (threadIdx.x == 0) *count = c;
 }
 
+__global__ void k_collect_flags(const EvalArgs *args, int npairs, unsigned *flags)
+{
+    for (int p = threadIdx.x; p < npairs; p += blockDim.x) flags[p] = args[p].counters[6];
+}
+
 struct PairRun {
     mgr_level_desc full{};
     int size[3] = {1, 1, 1}, prev[3] = {0, 0, 0}, csize[3] = {1, 1, 1};
@@ -346,8 +351,8 @@ struct PairRun {
     mgr_level *lvl0 = nullptr;       // the pass-0 level while lvl (refine pass) uses its images
     std::vector<mgr_level *> made;   // per level (index shift): made ahead, not yet in use
     std::vector<mgr_level *> made1;  // per level: the refine pass's level on made[shift]'s images
-    bool x_on_device = false;        // x holds the parameters of the next pass (params only sized)
-    DevBuf<double> x, g, xt, gt, costs;
+    double *x = nullptr;                       // the parameters, in xbuf
+    std::shared_ptr<DevBuf<double>> xbuf;      // shared by the pairs of a pass
     bool identity = false;   // both images of one value
     bool in_pass = false;
     double cost = 0.0;
@@ -393,9 +398,11 @@ void ckm(mgr_status s)
 }
 
 // Run the minimizer of every pair with in_pass set, in lock step, until all
-// have finished.  Steps are captured into a CUDA graph when use_graphs.
+// have finished.  x_on_device: x of these pairs, one after the other in one
+// buffer, holds their parameters (params is only sized).  Steps are captured
+// into a CUDA graph when use_graphs.
 void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_desc &mz, int dim, int tile[3],
-              bool use_graphs, bool persistent, cudaStream_t st, const char *label)
+              bool x_on_device, bool use_graphs, bool persistent, cudaStream_t st, const char *label)
 {
     std::vector<int> members;
     for (size_t i = 0; i < pairs.size(); ++i)
@@ -411,34 +418,50 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     size_t sm_warp = 0, sm_adj = 0, max_params = 0;
     int has_pen = 0;
     const int cost = pairs[members[0]]->full.cost;   // (the same for all pairs of a batch)
+    // the pairs' parameters: in the refine pass in place, else one upload
+    std::vector<size_t> off(np + 1, 0);
+    for (int k = 0; k < np; ++k) off[k + 1] = off[k] + pairs[members[k]]->params.size();
+    if (!x_on_device) {
+        std::vector<double> h(off[np]);
+        auto xbuf = std::make_shared<DevBuf<double>>();
+        for (int k = 0; k < np; ++k) {
+            PairRun &r = *pairs[members[k]];
+            std::copy(r.params.begin(), r.params.end(), h.begin() + off[k]);
+        }
+        xbuf->upload(h, st);
+        for (int k = 0; k < np; ++k) {
+            PairRun &r = *pairs[members[k]];
+            r.xbuf = xbuf;
+            r.x = xbuf->p + off[k];
+        }
+    }
+    // per pair and in this order: gradient, trial point and its gradient,
+    // costs (the vectors as long as the parameters)
+    DevBuf<double> d_vec;
+    d_vec.alloc(3 * off[np] + 2 * size_t(np), st);
     for (int k = 0; k < np; ++k) {
         PairRun &r = *pairs[members[k]];
         const size_t n = r.params.size();
-        if (r.x_on_device) r.x.alloc(n, st);   // (already there: the refine wrote it)
-        else r.x.upload(r.params, st);
-        r.x_on_device = false;
-        r.g.alloc(n, st);
-        r.xt.alloc(n, st);
-        r.gt.alloc(n, st);
-        r.costs.alloc(2, st);
+        double *const g = d_vec.p + 3 * off[k] + 2 * size_t(k), *const xt = g + n, *const gt = xt + n;
+        double *const costs = gt + n;
         EvalArgs a = r.lvl->args();
-        a.params = r.xt.p;
-        a.grad_total = r.gt.p;
+        a.params = xt;
+        a.grad_total = gt;
         a.grad_image = nullptr;
         a.grad_penalty = nullptr;
-        a.costs = r.costs.p;
+        a.costs = costs;
         a.convert = 0;   // k_min_propose writes the float copy
         // 2D SSD: the gather's last block finalises the cost
         a.defer_cost = dim == 2 && a.cost == MGR_COST_SSD;
         args[k] = a;
-        vecs[k] = PairVec{r.x.p, r.g.p, r.xt.p, r.gt.p, r.costs.p, int(n), a.params_f};
+        vecs[k] = PairVec{r.x, g, xt, gt, costs, int(n), a.params_f};
         MinState s{};
         s.step = mz.step;
         states[k] = s;
         const int nt = a.ax[0].nt * a.ax[1].nt * (dim == 3 ? a.ax[2].nt : 1);
         for (int t = 0; t < nt; ++t) titems.push_back(make_int2(k, t));
         nblocks[k] = gather_blocks(a);
-        for (int b = 0; b < nblocks[k]; ++b) gitems.push_back(make_int2(k, b));
+        for (int q = 0; q < nblocks[k]; ++q) gitems.push_back(make_int2(k, q));
         sm_warp = std::max(sm_warp, split_smem(a, 0));
         sm_adj = std::max(sm_adj, split_smem(a, 1));
         has_pen |= a.has_penalty;
@@ -457,7 +480,8 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         return o;
     };
     const size_t o_args = place(sizeof(EvalArgs) * np), o_vecs = place(sizeof(PairVec) * np);
-    const size_t o_states = place(sizeof(MinState) * np), o_titems = place(sizeof(int2) * titems.size());
+    const size_t o_states = place(sizeof(MinState) * np), o_flags = place(sizeof(unsigned) * np);
+    const size_t o_titems = place(sizeof(int2) * titems.size());
     const size_t o_gitems = place(sizeof(int2) * gitems.size()), o_nblocks = place(sizeof(int) * np);
     const size_t o_active = place(sizeof(int) * np), o_count = place(sizeof(int));
     const size_t o_moved = place(sizeof(int) * np), o_mcount = place(sizeof(unsigned) * np);
@@ -476,6 +500,7 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     EvalArgs *d_args = reinterpret_cast<EvalArgs *>(d_pass.p + o_args);
     PairVec *d_vecs = reinterpret_cast<PairVec *>(d_pass.p + o_vecs);
     MinState *d_states = reinterpret_cast<MinState *>(d_pass.p + o_states);
+    unsigned *d_flags = reinterpret_cast<unsigned *>(d_pass.p + o_flags);
     int2 *d_titems = reinterpret_cast<int2 *>(d_pass.p + o_titems);
     int2 *d_gitems = reinterpret_cast<int2 *>(d_pass.p + o_gitems);
     int *d_nblocks = reinterpret_cast<int *>(d_pass.p + o_nblocks);
@@ -565,31 +590,21 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_steps0).count();
     TraceScope tr_back("batch: readback", st);
     if (exec) cudaGraphExecDestroy(exec);
-    ck(cudaMemcpyAsync(states.data(), d_states, np * sizeof(MinState), cudaMemcpyDeviceToHost, st), "D2H");
-    // every pair's parameters and status flag (counters[6] of its level)
-    // gathered on the device, so that one copy brings them back
-    std::vector<size_t> off(np + 1, 0);
-    for (int k = 0; k < np; ++k) off[k + 1] = off[k] + pairs[members[k]]->params.size();
-    const size_t flags_at = off[np] * sizeof(double);
-    DevBuf<unsigned char> d_back;
-    d_back.alloc(flags_at + size_t(np) * sizeof(unsigned), st);
-    for (int k = 0; k < np; ++k) {
-        PairRun &r = *pairs[members[k]];
-        ck(cudaMemcpyAsync(d_back.p + off[k] * sizeof(double), r.x.p, r.params.size() * sizeof(double),
-                           cudaMemcpyDeviceToDevice, st),
-           "gather");
-        ck(cudaMemcpyAsync(d_back.p + flags_at + size_t(k) * sizeof(unsigned), r.lvl->counters.p + 6,
-                           sizeof(unsigned), cudaMemcpyDeviceToDevice, st),
-           "gather");
-    }
-    std::vector<unsigned char> back(d_back.n);
-    ck(cudaMemcpyAsync(back.data(), d_back.p, back.size(), cudaMemcpyDeviceToHost, st), "D2H");
+    // the states and status flags (counters[6] of the levels) in one copy,
+    // every pair's parameters in another
+    k_collect_flags<<<1, 32, 0, st>>>(d_args, np, d_flags);
+    count_launch();
+    std::vector<unsigned char> back(o_flags + sizeof(unsigned) * np - o_states);
+    ck(cudaMemcpyAsync(back.data(), d_states, back.size(), cudaMemcpyDeviceToHost, st), "D2H");
+    std::vector<double> xs(off[np]);
+    ck(cudaMemcpyAsync(xs.data(), pairs[members[0]]->x, xs.size() * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
     ck(cudaStreamSynchronize(st), "batch sync");
     std::vector<unsigned> flags(np, 0u);
+    std::memcpy(states.data(), back.data(), np * sizeof(MinState));
+    std::memcpy(flags.data(), back.data() + (o_flags - o_states), np * sizeof(unsigned));
     for (int k = 0; k < np; ++k) {
         PairRun &r = *pairs[members[k]];
-        std::memcpy(r.params.data(), back.data() + off[k] * sizeof(double), r.params.size() * sizeof(double));
-        std::memcpy(&flags[k], back.data() + flags_at + size_t(k) * sizeof(unsigned), sizeof(unsigned));
+        std::copy(xs.begin() + off[k], xs.begin() + off[k + 1], r.params.begin());
     }
     for (int k = 0; k < np; ++k) throw_if_flagged(pairs[members[k]]->lvl, flags[k]);
     double vox_evals = 0.0;
@@ -838,23 +853,27 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                             }
                             ncn[k] = refine_csize(size[k], r.full.rate[k]);
                         }
-                        const size_t n = size_t(size[0]) * size[1] * (dim == 3 ? size[2] : 1);
-                        DevBuf<float> src_l, ref_l;   // freed in stream order after the level's copies
-                        src_l.alloc(n, sp);
-                        ref_l.alloc(n, sp);
-                        scale_image(r.src_n.p, r.full.size, src_l.p, size, dim, sp);
-                        scale_image(r.ref_n.p, r.full.size, ref_l.p, size, dim, sp);
                         mgr_level_desc d = r.full;
                         for (int k = 0; k < 3; ++k) {
                             d.size[k] = k < dim ? size[k] : 1;
                             d.csize[k] = k < dim ? csize[k] : 0;
                         }
                         mgr_level *L = nullptr;
-                        ckm(mgr_level_create(&d, device, sp, &L));
-                        r.made[shift] = L;
                         const int *tile = level_tile[shift].data();
+                        ckm(level_create(&d, device, sp, tile, &L));
+                        r.made[shift] = L;
+                        // (a tile that level_create has not taken is refused here)
                         ckm(mgr_level_set_path(L, MGR_PATH_SPLIT, tile[0], tile[1], tile[2]));
-                        level_set_images_async(L, src_l.p, ref_l.p);
+                        if (shift == 0) {
+                            level_set_images_async(L, r.src_n.p, r.ref_n.p);
+                        } else {
+                            // scaled into the level's own buffers (the moving
+                            // image's coefficients are made from the copy)
+                            const float *const from[2] = {r.src_n.p, r.ref_n.p};
+                            float *const to[2] = {L->warped.p, L->ref.p};
+                            scale_images(2, from, r.full.size, to, size, dim, sp);
+                            level_set_images_async(L, to[0], to[1]);
+                        }
                         if (refine_grows(dim, csize, ncn)) {
                             // the refine pass's grid, on the same images
                             r.made1[shift] = level_create_on_images(L, ncn, sp);
@@ -909,51 +928,58 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                     // resized: the pass's readback refreshes it).  Grids
                     // with an axis of fewer than 4 coefficients are refined
                     // on the host.
+                    // The refined parameters go to one buffer, pair after pair.
                     std::vector<RefineJobSpec> jobs;
-                    std::vector<PairRun *> on_dev;
-                    std::vector<size_t> at;
+                    std::vector<std::array<int, 3>> grown(pairs.size());
                     size_t total = 0;
-                    for (auto &rp : pairs) {
-                        PairRun &r = *rp;
+                    for (size_t i = 0; i < pairs.size(); ++i) {
+                        PairRun &r = *pairs[i];
+                        r.in_pass = false;
                         if (r.identity) continue;
-                        int ncn[3] = {1, 1, 1};
-                        for (int k = 0; k < dim; ++k) ncn[k] = refine_csize(r.size[k], r.full.rate[k]);
-                        r.in_pass = refine_grows(dim, r.csize, ncn);
+                        for (int k = 0; k < 3; ++k)
+                            grown[i][k] = k < dim ? refine_csize(r.size[k], r.full.rate[k]) : 1;
+                        r.in_pass = refine_grows(dim, r.csize, grown[i].data());
+                        if (r.in_pass) total += size_t(grown[i][0]) * grown[i][1] * grown[i][2] * dim;
+                    }
+                    auto xnew = std::make_shared<DevBuf<double>>();
+                    xnew->alloc(total, st);
+                    std::vector<std::vector<double>> on_host;   // kept until the stream has been waited for
+                    size_t at = 0;
+                    for (size_t i = 0; i < pairs.size(); ++i) {
+                        PairRun &r = *pairs[i];
                         if (!r.in_pass) continue;
+                        const int *ncn = grown[i].data();
+                        double *const to = xnew->p + at;
+                        const size_t n = size_t(ncn[0]) * ncn[1] * ncn[2] * dim;
                         bool small = false;
                         for (int k = 0; k < dim; ++k) small |= r.csize[k] < 4 || ncn[k] < 4;
                         if (small) {
                             refine_params(dim, r.csize, ncn, r.params);
+                            on_host.push_back(r.params);
+                            ck(cudaMemcpyAsync(to, on_host.back().data(), n * sizeof(double), cudaMemcpyHostToDevice, st),
+                               "refined parameters");
                         } else {
                             RefineJobSpec j;
                             for (int k = 0; k < 3; ++k) {
                                 j.nc_old[k] = r.csize[k];
                                 j.nc_new[k] = ncn[k];
                             }
-                            j.in = r.x.p;
-                            j.out = nullptr;
+                            j.in = r.x;
+                            j.out = to;
                             jobs.push_back(j);
-                            on_dev.push_back(&r);
-                            at.push_back(total);
-                            total += size_t(ncn[0]) * ncn[1] * ncn[2] * dim;
-                        }
-                        for (int k = 0; k < 3; ++k) r.csize[k] = ncn[k];
-                    }
-                    if (!jobs.empty()) {
-                        DevBuf<double> d_new;
-                        d_new.alloc(total, st);
-                        for (size_t j = 0; j < jobs.size(); ++j) jobs[j].out = d_new.p + at[j];
-                        refine_params_device(dim, jobs, st);
-                        for (size_t j = 0; j < jobs.size(); ++j) {
-                            PairRun &r = *on_dev[j];
-                            const size_t n = size_t(r.csize[0]) * r.csize[1] * r.csize[2] * dim;
-                            r.x.alloc(n, st);   // (the old buffer is freed after the refine read it)
-                            ck(cudaMemcpyAsync(r.x.p, d_new.p + at[j], n * sizeof(double), cudaMemcpyDeviceToDevice,
-                                               st),
-                               "refined parameters");
                             r.params.resize(n);
-                            r.x_on_device = true;
                         }
+                        at += n;
+                    }
+                    if (!jobs.empty()) refine_params_device(dim, jobs, st);
+                    at = 0;
+                    for (size_t i = 0; i < pairs.size(); ++i) {
+                        PairRun &r = *pairs[i];
+                        if (!r.in_pass) continue;
+                        r.x = xnew->p + at;
+                        r.xbuf = xnew;   // (the old buffer is freed after the refine read it)
+                        at += r.params.size();
+                        for (int k = 0; k < 3; ++k) r.csize[k] = grown[i][k];
                     }
                 }
                 TraceScope tr_grid(pass == 1 ? "batch: set grid (refine pass)" : "batch: destroy+take level", st);
@@ -1000,7 +1026,7 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                 tr_grid.stop();
                 tr_lvl.stop();
                 const std::string label = "level " + std::to_string(shift) + " pass " + std::to_string(pass);
-                run_pass(pairs, *mz, dim, tile, (use_graphs & 1) != 0, (use_graphs & 2) != 0, st, label.c_str());
+                run_pass(pairs, *mz, dim, tile, pass == 1, (use_graphs & 1) != 0, (use_graphs & 2) != 0, st, label.c_str());
             }
             for (auto &rp : pairs)
                 for (int k = 0; k < 3; ++k) rp->prev[k] = rp->size[k];

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -51,15 +52,25 @@ struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     cudaStream_t st = nullptr;
+    bool own = true;   // false: part of another buffer (borrow)
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }
     void release()
     {
-        if (p) cudaFreeAsync(p, st);
+        if (p && own) cudaFreeAsync(p, st);
         p = nullptr;
         n = 0;
+        own = true;
+    }
+    // count elements at q, inside a buffer that outlives this one
+    void borrow(void *q, size_t count)
+    {
+        release();
+        p = static_cast<T *>(q);
+        n = count;
+        own = false;
     }
     void alloc(size_t count, cudaStream_t s)
     {
@@ -76,6 +87,26 @@ struct DevBuf {
         if (!h.empty()) ck(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s), "upload");
     }
 };
+
+// The buffers that `each` lists (each(f) calls f(buffer, count) for all of
+// them) in one allocation: a level has about twenty, and the cost of a
+// stream-ordered allocation grows with the blocks that the pool holds and the
+// streams they were freed on.
+template <class Each>
+void alloc_together(DevBuf<unsigned char> &slab, cudaStream_t s, Each each)
+{
+    auto bytes = [](auto &b, size_t count) { return (count * sizeof(*b.p) + 255) & ~size_t(255); };
+    size_t total = 0;
+    each([&](auto &b, size_t count) { total += bytes(b, count); });
+    slab.release();
+    slab.alloc(total, s);
+    size_t at = 0;
+    each([&](auto &b, size_t count) {
+        if (count == 0) b.release();
+        else b.borrow(slab.p + at, count);
+        at += bytes(b, count);
+    });
+}
 
 // the per-axis tables of a level, packed with the other tables into one
 // host blob and uploaded with one copy; `off` are byte offsets into it
@@ -142,7 +173,12 @@ struct mgr_level {
     int path = MGR_PATH_SPLIT;
     int tile[3] = {32, 8, 16};
     AxisDev ax[3];
-    DevBuf<unsigned char> axis_tables;   // the packed AxisDev tables
+    // the allocations that hold the buffers below: images, state (counters,
+    // scalars), and what depends on the coefficient grid and the tile
+    DevBuf<unsigned char> slab_images, slab_state, slab_grid;
+    DevBuf<unsigned char> axis_tables;   // the packed AxisDev tables, then the penalty's
+    std::vector<float> ptable_host;                        // 3D: the penalty's cells
+    std::shared_ptr<const Penalty2Table> penalty2_host;    // 2D
     // MGR_PATH_FUSED: the tables of the fused kernel's tiles (30 x 8 x TZ),
     // for its launch and the gather after it; the other kernels keep ax
     AxisDev axf[3];
@@ -185,6 +221,7 @@ struct mgr_level {
         auto re = [s](auto &b) {
             if (b.p) b.st = s;
         };
+        re(slab_images), re(slab_state), re(slab_grid);
         re(axis_tables);
         re(axis_tables_f);
         re(coef), re(coef_pad), re(ref), re(warped), re(minmax), re(partial), re(ptable), re(pen_val), re(params_f);
@@ -313,13 +350,12 @@ struct mgr_level {
         }
     }
 
-    // the per-axis tables of tiles t into A (packed, uploaded to tables);
+    // the per-axis tables of tiles t into A, packed at the end of blob;
     // returns the number of tiles and sets the partial slot size
-    int build_axis_set(const int t[3], AxisDev (&A)[3], DevBuf<unsigned char> &tables, int &slot_size)
+    int build_axis_set(const int t[3], AxisDev (&A)[3], std::vector<unsigned char> &blob, int &slot_size) const
     {
         const int D = d.dim;
         AxisDev *ax = A;
-        std::vector<unsigned char> blob;
         for (int k = 0; k < D; ++k) build_axis(ax[k].h, n[k], nc[k], t[k]);
         if (D == 3) {
             // per axis and coefficient: the partial-slot offset parts of the
@@ -345,10 +381,6 @@ struct mgr_level {
             }
         }
         for (int k = 0; k < D; ++k) ax[k].pack_all(blob);
-        // a fresh buffer: kernels queued earlier may still read the old one
-        tables.release();
-        tables.upload(blob, stream);
-        for (int k = 0; k < D; ++k) ax[k].base = tables.p;
         slot_size = D * ax[0].h.ac * ax[1].h.ac * (D == 3 ? ax[2].h.ac : 1);
         return ax[0].h.nt * ax[1].h.nt * (D == 3 ? ax[2].h.nt : 1);
     }
@@ -362,22 +394,79 @@ struct mgr_level {
         t[2] = tile[2];
     }
 
+    // the penalty's cells of the grid on the host (3D: translation-invariant;
+    // 2D: boundary-clipped CSR rows, cached across levels of equal grid)
+    void build_penalty()
+    {
+        if (!d.has_penalty) return;
+        const float range[3] = {float(d.size[0]), float(d.size[1]), float(d.dim == 3 ? d.size[2] : 1)};
+        if (d.dim == 3) ptable_host = build_penalty3(nc, range, d.pen_div, d.pen_curl);
+        else penalty2_host = penalty2_cached(nc, range, d.pen_div, d.pen_curl);
+    }
+
+    // Everything that depends on the coefficient grid and the tile: the
+    // tables (with the penalty's, one upload), the parameter and gradient
+    // buffers, the partials.  In a fresh allocation: kernels queued earlier
+    // may still read the old one, which is freed in stream order.
     void build_tables()
     {
-        const int ntiles = build_axis_set(tile, ax, axis_tables, slot);
+        std::vector<unsigned char> blob;
+        const int ntiles = build_axis_set(tile, ax, blob, slot);
         size_t part = size_t(ntiles) * slot, sums = size_t(ntiles);
         if (path == MGR_PATH_FUSED) {
+            std::vector<unsigned char> blob_f;
             int t[3];
             fused_tile(t);
-            const int ntf = build_axis_set(t, axf, axis_tables_f, slot_f);
+            const int ntf = build_axis_set(t, axf, blob_f, slot_f);
             part = std::max(part, size_t(ntf) * slot_f);
             sums = std::max(sums, size_t(ntf));
+            axis_tables_f.release();
+            axis_tables_f.upload(blob_f, stream);
+            for (int k = 0; k < d.dim; ++k) axf[k].base = axis_tables_f.p;
         }
-        partial.alloc(part, stream);
+        size_t at_pen[3] = {0, 0, 0};
+        if (d.has_penalty && d.dim == 3) {
+            at_pen[0] = AxisDev::pack(blob, ptable_host);
+        } else if (d.has_penalty) {
+            at_pen[0] = AxisDev::pack(blob, penalty2_host->rowptr);
+            at_pen[1] = AxisDev::pack(blob, penalty2_host->col);
+            at_pen[2] = AxisDev::pack(blob, penalty2_host->val);
+        }
+        EvalArgs sizes{};   // what the counts below depend on
+        sizes.dim = d.dim;
+        for (int k = 0; k < 3; ++k) sizes.nc[k] = nc[k];
         const size_t plain_blocks = (N + 255) / 256;
-        tile_sums.alloc(std::max<size_t>(sums, plain_blocks) * 5, stream);
-        pen_part.alloc(size_t(gather_blocks(args())) + 1, stream);
+        alloc_together(slab_grid, stream, [&](auto buf) {
+            buf(params, nparams);
+            buf(params_f, nparams);
+            buf(grad_total, nparams);
+            buf(axis_tables, blob.size());
+            buf(partial, part);
+            buf(tile_sums, std::max<size_t>(sums, plain_blocks) * 5);
+            buf(pen_part, size_t(gather_blocks(sizes)) + 1);
+        });
+        axis_tables.upload(blob, stream);
+        for (int k = 0; k < d.dim; ++k) ax[k].base = axis_tables.p;
+        if (d.has_penalty && d.dim == 3) {
+            ptable.borrow(axis_tables.p + at_pen[0], ptable_host.size());
+        } else if (d.has_penalty) {
+            pen_rowptr.borrow(axis_tables.p + at_pen[0], penalty2_host->rowptr.size());
+            pen_col.borrow(axis_tables.p + at_pen[1], penalty2_host->col.size());
+            pen_val.borrow(axis_tables.p + at_pen[2], penalty2_host->val.size());
+        }
         tables_valid = true;
+    }
+
+    // counters and scalars, zero; means of the images
+    void alloc_state()
+    {
+        alloc_together(slab_state, stream, [&](auto buf) {
+            buf(counters, 8);
+            buf(scalars, SC_NSLOTS);
+            buf(costs, 2);
+            buf(means, 2);
+        });
+        ck(cudaMemsetAsync(slab_state.p, 0, slab_state.n, stream), "memset");
     }
 };
 
@@ -395,6 +484,9 @@ inline void registration_tile(int dim, int t[3])
     t[1] = dim == 3 ? 8 : 16;
     t[2] = dim == 3 ? 16 : 1;
 }
+// mgr_level_create, with the split path's tile when tile is given (and
+// fits: else the level keeps the one it would choose)
+mgr_status level_create(const mgr_level_desc *desc, int device, void *stream, const int *tile, mgr_level **out);
 // mgr_level_set_images_device without the final stream synchronisation
 void level_set_images_async(mgr_level *L, const float *d_src, const float *d_ref);
 // a new coefficient grid (and tile) on a level, images kept

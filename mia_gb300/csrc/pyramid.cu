@@ -129,8 +129,13 @@ __global__ void k_apply_linear(const float *__restrict__ in, float *__restrict__
 // line.
 constexpr int SCALE_NT = 256;
 
-__global__ void __launch_bounds__(SCALE_NT) k_scale_lines(const float *__restrict__ in, float *__restrict__ out,
-                                                          int lb, int n_in, int n_out, int nlines,
+struct ScaleImages {
+    const float *in[2];
+    float *out[2];
+};
+
+// blockIdx.y: the image
+__global__ void __launch_bounds__(SCALE_NT) k_scale_lines(ScaleImages im, int lb, int n_in, int n_out, int nlines,
                                                           size_t in_line_stride, size_t in_elem_stride,
                                                           size_t out_line_stride, size_t out_elem_stride,
                                                           int lines_per_plane, size_t in_plane_stride,
@@ -138,6 +143,8 @@ __global__ void __launch_bounds__(SCALE_NT) k_scale_lines(const float *__restric
                                                           const int4 *idx, const float4 *wts)
 {
     extern __shared__ float sl[];
+    const float *__restrict__ in = im.in[blockIdx.y];
+    float *__restrict__ out = im.out[blockIdx.y];
     const int pitch = n_in | 1;
     const int tid = threadIdx.x;
     const int l0 = blockIdx.x * lb;
@@ -290,41 +297,48 @@ AxisPlan plan_axis(int n_in, int n_out)
     return p;
 }
 
-void scale_axis(const float *in, float *out, const AxisPlan &p, int n_in, int n_out, int nlines, size_t ils,
-                size_t ies, size_t ols, size_t oes, int lpp, size_t ips, size_t ops, cudaStream_t st)
+// an axis' plan (mask, taps, weights) as float at the end of blob
+struct PlanAt {
+    size_t mask, idx, wts;
+};
+
+PlanAt pack_plan(std::vector<unsigned char> &blob, const AxisPlan &p)
 {
-    // the plan (mask, taps, weights) as float in one stream-ordered upload;
-    // the host blob may go away once the pageable copy has been issued
-    std::vector<float> mask(p.mask.begin(), p.mask.end());
+    auto put = [&](const void *src, size_t n) {
+        const size_t o = (blob.size() + 15) & ~size_t(15);
+        blob.resize(o + n);
+        std::memcpy(blob.data() + o, src, n);
+        return o;
+    };
+    const std::vector<float> mask(p.mask.begin(), p.mask.end());
     std::vector<float4> wts;
     for (const Wt4 &w : p.wts) wts.push_back(make_float4(float(w.x), float(w.y), float(w.z), float(w.w)));
-    const size_t o_idx = ((mask.size() * sizeof(float) + 15) / 16) * 16;
-    const size_t o_wts = o_idx + p.idx.size() * sizeof(int4);
-    const size_t bytes = o_wts + wts.size() * sizeof(float4);
-    std::vector<unsigned char> blob(bytes, 0);
-    std::memcpy(blob.data(), mask.data(), mask.size() * sizeof(float));
-    std::memcpy(blob.data() + o_idx, p.idx.data(), p.idx.size() * sizeof(int4));
-    std::memcpy(blob.data() + o_wts, wts.data(), wts.size() * sizeof(float4));
-    unsigned char *d = nullptr;
-    ck(dev_malloc_async(reinterpret_cast<void **>(&d), bytes, st), "cudaMallocAsync");
-    ck(cudaMemcpyAsync(d, blob.data(), bytes, cudaMemcpyHostToDevice, st), "H2D");
+    PlanAt a;
+    a.mask = put(mask.data(), mask.size() * sizeof(float));
+    a.idx = put(p.idx.data(), p.idx.size() * sizeof(int4));
+    a.wts = put(wts.data(), wts.size() * sizeof(float4));
+    return a;
+}
+
+void scale_axis(const ScaleImages &im, int nimg, const unsigned char *d, const PlanAt &at, int gw, int n_in, int n_out,
+                int nlines, size_t ils, size_t ies, size_t ols, size_t oes, int lpp, size_t ips, size_t ops,
+                cudaStream_t st)
+{
     // lines per block: at most 64 and 96 KB of staged lines, fewer while
     // the launch would have less than two blocks per SM (the block's line
     // recursion is its critical path)
     const int pitch = n_in | 1;
     int lb = 64;
     while (lb > 1 && size_t(lb) * 2 * pitch * sizeof(float) > 96 * 1024) lb >>= 1;
-    while (lb > 8 && (nlines + lb - 1) / lb < 2 * num_sms()) lb >>= 1;
+    while (lb > 8 && (nlines + lb - 1) / lb * nimg < 2 * num_sms()) lb >>= 1;
     const size_t sm = size_t(lb) * 2 * pitch * sizeof(float);
     if (sm > 200 * 1024) throw std::invalid_argument("scale: image line too long");
-    cudaFuncSetAttribute(k_scale_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    k_scale_lines<<<(nlines + lb - 1) / lb, SCALE_NT, sm, st>>>(in, out, lb, n_in, n_out, nlines, ils, ies, ols, oes, lpp,
-                                                         ips, ops, p.gw, reinterpret_cast<const float *>(d),
-                                                         reinterpret_cast<const int4 *>(d + o_idx),
-                                                         reinterpret_cast<const float4 *>(d + o_wts));
+    raise_smem_limit(reinterpret_cast<const void *>(k_scale_lines), sm);
+    k_scale_lines<<<dim3((nlines + lb - 1) / lb, nimg), SCALE_NT, sm, st>>>(
+        im, lb, n_in, n_out, nlines, ils, ies, ols, oes, lpp, ips, ops, gw, reinterpret_cast<const float *>(d + at.mask),
+        reinterpret_cast<const int4 *>(d + at.idx), reinterpret_cast<const float4 *>(d + at.wts));
     count_launch();
     ck(cudaGetLastError(), "scale kernel");
-    cudaFreeAsync(d, st);
 }
 
 }  // namespace
@@ -455,39 +469,65 @@ std::vector<char> normalize_pairs(const std::vector<const float *> &src, const s
     return varied;
 }
 
-void scale_image(const float *d_in, const int in_size[3], float *d_out, const int out_size[3], int dim,
-                 cudaStream_t st)
+void scale_images(int nimg, const float *const *d_in, const int in_size[3], float *const *d_out,
+                  const int out_size[3], int dim, cudaStream_t st)
 {
     const int nx = in_size[0], ny = in_size[1], nz = dim == 3 ? in_size[2] : 1;
     const int mx = out_size[0], my = out_size[1], mz = dim == 3 ? out_size[2] : 1;
     if (nx == mx && ny == my && nz == mz) {
-        ck(cudaMemcpyAsync(d_out, d_in, size_t(nx) * ny * nz * sizeof(float), cudaMemcpyDeviceToDevice, st), "copy");
+        for (int i = 0; i < nimg; ++i)
+            ck(cudaMemcpyAsync(d_out[i], d_in[i], size_t(nx) * ny * nz * sizeof(float), cudaMemcpyDeviceToDevice, st),
+               "copy");
         return;
     }
     for (int k = 0; k < dim; ++k)
         if (out_size[k] > in_size[k] || out_size[k] < 2)
             throw std::invalid_argument("scale: only downscaling to sizes >= 2 is supported");
-    // x: lines = rows (y, z)
-    float *t1 = nullptr, *t2 = nullptr;
-    ck(dev_malloc_async(reinterpret_cast<void **>(&t1), size_t(mx) * ny * nz * sizeof(float), st), "cudaMallocAsync");
-    const AxisPlan px = plan_axis(nx, mx);
-    const AxisPlan py = plan_axis(ny, my);
-    // (C1DScalar copies when the size does not change on an axis)
-    scale_axis(d_in, t1, px, nx, mx, ny * nz, size_t(nx), 1, size_t(mx), 1, ny * nz, 0, 0, st);
-    if (dim == 2) {
-        // y: lines = columns x, stride mx
-        scale_axis(t1, d_out, py, ny, my, mx, 1, size_t(mx), 1, size_t(mx), mx, 0, 0, st);
-        cudaFreeAsync(t1, st);
-        return;
+    // the plans of all axes and the images between the passes in one
+    // stream-ordered allocation, one upload; the host blob may go away once
+    // the pageable copy has been issued
+    const AxisPlan px = plan_axis(nx, mx), py = plan_axis(ny, my);
+    const AxisPlan pz = dim == 3 ? plan_axis(nz, mz) : AxisPlan();
+    std::vector<unsigned char> blob;
+    const PlanAt ax = pack_plan(blob, px), ay = pack_plan(blob, py), az = pack_plan(blob, pz);
+    const size_t n1 = size_t(mx) * ny * nz, n2 = dim == 3 ? size_t(mx) * my * nz : 0;
+    const size_t plans = (blob.size() + 255) & ~size_t(255);
+    unsigned char *d = nullptr;
+    ck(dev_malloc_async(reinterpret_cast<void **>(&d), plans + (n1 + n2) * nimg * sizeof(float), st), "cudaMallocAsync");
+    float *const t = reinterpret_cast<float *>(d + plans);
+    ScaleImages im[3] = {};   // the images of each pass
+    for (int i = 0; i < nimg; ++i) {
+        float *t1 = t + n1 * i, *t2 = t + n1 * nimg + n2 * i;
+        im[0].in[i] = d_in[i];
+        im[0].out[i] = t1;
+        im[1].in[i] = t1;
+        im[1].out[i] = dim == 3 ? t2 : d_out[i];
+        im[2].in[i] = t2;
+        im[2].out[i] = d_out[i];
     }
-    ck(dev_malloc_async(reinterpret_cast<void **>(&t2), size_t(mx) * my * nz * sizeof(float), st), "cudaMallocAsync");
-    // y: lines = (x, z): per plane z, mx lines of stride 1, element stride mx
-    scale_axis(t1, t2, py, ny, my, mx * nz, 1, size_t(mx), 1, size_t(mx), mx, size_t(mx) * ny, size_t(mx) * my, st);
-    // z: lines = (x, y): mx*my lines, element stride mx*my
-    const AxisPlan pz = plan_axis(nz, mz);
-    scale_axis(t2, d_out, pz, nz, mz, mx * my, 1, size_t(mx) * my, 1, size_t(mx) * my, mx * my, 0, 0, st);
-    cudaFreeAsync(t1, st);
-    cudaFreeAsync(t2, st);
+    try {
+        ck(cudaMemcpyAsync(d, blob.data(), blob.size(), cudaMemcpyHostToDevice, st), "H2D");
+        // (C1DScalar copies when the size does not change on an axis)
+        // x: lines = rows (y, z)
+        scale_axis(im[0], nimg, d, ax, px.gw, nx, mx, ny * nz, size_t(nx), 1, size_t(mx), 1, ny * nz, 0, 0, st);
+        // y: lines = (x, z): per plane z, mx lines of stride 1, element stride mx
+        scale_axis(im[1], nimg, d, ay, py.gw, ny, my, mx * nz, 1, size_t(mx), 1, size_t(mx), mx, size_t(mx) * ny,
+                   size_t(mx) * my, st);
+        // z: lines = (x, y): mx*my lines, element stride mx*my
+        if (dim == 3)
+            scale_axis(im[2], nimg, d, az, pz.gw, nz, mz, mx * my, 1, size_t(mx) * my, 1, size_t(mx) * my, mx * my, 0, 0,
+                       st);
+    } catch (...) {
+        cudaFreeAsync(d, st);
+        throw;
+    }
+    cudaFreeAsync(d, st);
+}
+
+void scale_image(const float *d_in, const int in_size[3], float *d_out, const int out_size[3], int dim,
+                 cudaStream_t st)
+{
+    scale_images(1, &d_in, in_size, &d_out, out_size, dim, st);
 }
 
 }  // namespace mgr

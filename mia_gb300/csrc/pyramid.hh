@@ -29,7 +29,10 @@ std::vector<char> normalize_pairs(const std::vector<const float *> &src, const s
                                   const std::vector<float *> &ref_out, cudaStream_t st,
                                   bool copy_first = false);
 
-// The `scale` filter (downscaling only); a copy when the sizes agree.
+// The `scale` filter (downscaling only) on nimg (1 or 2) images of one size;
+// a copy when the sizes agree.
+void scale_images(int nimg, const float *const *d_in, const int in_size[3], float *const *d_out,
+                  const int out_size[3], int dim, cudaStream_t st);
 void scale_image(const float *d_in, const int in_size[3], float *d_out, const int out_size[3], int dim,
                  cudaStream_t st);
 

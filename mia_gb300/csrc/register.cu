@@ -48,7 +48,7 @@ double register_pair_device(const mgr_level_desc &full, int levels, const mgr_mi
     const int dim = full.dim;
     const int nz = dim == 3 ? full.size[2] : 1;
     const size_t n_full = size_t(full.size[0]) * full.size[1] * nz;
-    DevBuf<float> src_n, ref_n, src_l, ref_l;
+    DevBuf<float> src_n, ref_n, img_l;   // img_l: the level's two images
     src_n.alloc(n_full, st);
     ref_n.alloc(n_full, st);
     int evals = 0;
@@ -80,10 +80,10 @@ double register_pair_device(const mgr_level_desc &full, int levels, const mgr_mi
         }
         const size_t n = size_t(size[0]) * size[1] * (dim == 3 ? size[2] : 1);
         TraceScope tr_scale("pair: scale filter", st);
-        src_l.alloc(n, st);
-        ref_l.alloc(n, st);
-        scale_image(src_n.p, full.size, src_l.p, size, dim, st);
-        scale_image(ref_n.p, full.size, ref_l.p, size, dim, st);
+        img_l.alloc(2 * n, st);
+        const float *const from[2] = {src_n.p, ref_n.p};
+        float *const to[2] = {img_l.p, img_l.p + n};
+        scale_images(2, from, full.size, to, size, dim, st);
         tr_scale.stop();
         for (int pass = 0; pass < 2; ++pass) {
             mgr_level_desc d = full;
@@ -93,12 +93,12 @@ double register_pair_device(const mgr_level_desc &full, int levels, const mgr_mi
             }
             TraceScope tr_lvl("pair: level setup", st);
             LevelHandle lv;
-            ckm(mgr_level_create(&d, device, st, &lv.h));
             int t[3];
             registration_tile(dim, t);
+            ckm(level_create(&d, device, st, nullptr, &lv.h));
             if (lv.h->tile_fits(t)) ckm(mgr_level_set_path(lv.h, path, t[0], t[1], t[2]));
             else ckm(mgr_level_set_path(lv.h, path, 0, 0, 0));
-            level_set_images_async(lv.h, src_l.p, ref_l.p);
+            level_set_images_async(lv.h, to[0], to[1]);
             tr_lvl.stop();
             TraceScope tr_min("pair: minimizer", st);
             FDF fdf = [&](const std::vector<double> &x, std::vector<double> &g) {
