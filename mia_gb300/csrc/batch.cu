@@ -32,6 +32,7 @@
 #include "../../include/mgr.h"
 #include "driver.hh"
 #include "level.hh"
+#include "mgr_launch.hh"
 #include "pyramid.hh"
 #include "trace.hh"
 
@@ -79,70 +80,108 @@ struct MinScratch {
     int nblk;
 };
 
-// sums of a and b and the maximum of c over the block, returned to every
-// thread (fixed order)
-__device__ void block_reduce3(double &a, double &b, double &c, double *red)
+// The sums and the maximum that an update needs: q, and for gdsq q2 and mx.
+// FP64 instructions (1/64 of the FP32 rate) and the steps between them are
+// what these kernels' time goes to, so only what the minimizer uses is
+// reduced, the maximum of magnitudes as integers (their order; NaN counts as
+// 0), and a pair whose vectors are one block's needs no partial sums at all.
+__device__ __forceinline__ double max_magnitude(double m, double g)
+{
+    const long long b = __double_as_longlong(g) & 0x7fffffffffffffffll, k = __double_as_longlong(m);
+    return b > 0x7ff0000000000000ll || b < k ? m : __longlong_as_double(b);
+}
+
+// a, b and the maximum c over the block, in thread 0 (fixed order: a tree per
+// warp, then the warps in order)
+__device__ void block_reduce3(double &a, double &b, double &c, bool all, double *red)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    a = warp_sum(a);
-    b = warp_sum(b);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c = fmax(c, __shfl_xor_sync(0xffffffffu, c, o));
     __syncthreads();   // red may still be read by a previous call
-    if (lane == 0) {
-        red[w] = a;
-        red[MT / 32 + w] = b;
-        red[2 * MT / 32 + w] = c;
+    if (all) {
+        const double s = warp_sum2(a, b, lane);
+        if ((lane & 15) == 0) red[(lane >> 4) * (MT / 32) + w] = s;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) c = max_magnitude(c, __shfl_xor_sync(0xffffffffu, c, o));
+        if (lane == 0) red[2 * MT / 32 + w] = c;
+    } else {
+        a = warp_sum(a);
+        if (lane == 0) red[w] = a;
     }
     __syncthreads();
+    if (threadIdx.x != 0) return;
     a = 0.0;
     b = 0.0;
     c = 0.0;
-    for (int k = 0; k < MT / 32; ++k) {
-        a += red[k];
-        b += red[MT / 32 + k];
-        c = fmax(c, red[2 * MT / 32 + k]);
-    }
+    for (int k = 0; k < MT / 32; ++k) a += red[k];
+    if (all)
+        for (int k = 0; k < MT / 32; ++k) {
+            b += red[MT / 32 + k];
+            c = max_magnitude(c, red[2 * MT / 32 + k]);
+        }
 }
 
-// store this block's partials; true in the pair's last block, which then
-// holds the totals (partials added in block order) in a, b, c
-__device__ bool pair_totals(const MinScratch &m, int p, int nb, double &a, double &b, double &c, double *red)
+// the block is the last of the pair's nb to arrive (its threads' writes before
+// this are visible to the last one's after it)
+__device__ bool last_of_pair(const MinScratch &m, int p, int nb)
 {
     __shared__ bool last;
-    block_reduce3(a, b, c, red);
+    __syncthreads();   // every thread has read the pair's state
+    if (nb == 1) return true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&m.count[p], 1u) == unsigned(nb - 1);
+        if (last) m.count[p] = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// the pair's totals of a, b (sums, partials added in block order) and c
+// (maximum) in thread 0 of its last block, for which true is returned; all:
+// b and c are wanted, too
+__device__ bool pair_totals(const MinScratch &m, int p, int nb, double &a, double &b, double &c, bool all, double *red)
+{
+    block_reduce3(a, b, c, all, red);
+    if (nb == 1) {
+        // (the sum that a second reduction of one partial would give)
+        a = 0.0 + a;
+        b = 0.0 + b;
+        return true;
+    }
     if (threadIdx.x == 0) {
         double *pp = m.part + (size_t(p) * m.nblk + blockIdx.x) * 3;
         pp[0] = a;
         pp[1] = b;
         pp[2] = c;
-        __threadfence();
-        last = atomicAdd(&m.count[p], 1u) == unsigned(nb - 1);
     }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
+    if (!last_of_pair(m, p, nb)) return false;
     a = 0.0;
     b = 0.0;
     c = 0.0;
     for (int k = threadIdx.x; k < nb; k += MT) {
         const double *pp = m.part + (size_t(p) * m.nblk + k) * 3;
         a += __ldcg(pp);
-        b += __ldcg(pp + 1);
-        c = fmax(c, __ldcg(pp + 2));
+        if (all) {
+            b += __ldcg(pp + 1);
+            c = max_magnitude(c, __ldcg(pp + 2));
+        }
     }
-    block_reduce3(a, b, c, red);
-    if (threadIdx.x == 0) m.count[p] = 0;
+    block_reduce3(a, b, c, all, red);
     return true;
 }
 
+// The kernels of a step are launched to overlap (pdl_wait): each waits before
+// it reads anything that the step before has written.
 __global__ void __launch_bounds__(MT) k_min_propose(MinState *st, const PairVec *vec, mgr_minimizer_desc mz,
                                                     int *active, MinScratch m)
 {
-    __shared__ double red[3 * MT / 32];
+    __shared__ double factor;
     const int p = blockIdx.y, tid = threadIdx.x;
     const PairVec v = vec[p];
     const int nb = (v.n + MCH - 1) / MCH;
+    pdl_wait();
+    pdl_trigger();
     if (int(blockIdx.x) >= nb) return;
     const int i0 = blockIdx.x * MCH, i1 = min(v.n, i0 + MCH);
     const bool lead = blockIdx.x == 0 && tid == 0;
@@ -169,20 +208,25 @@ __global__ void __launch_bounds__(MT) k_min_propose(MinState *st, const PairVec 
             }
             return;
         }
-        const double a = -s.step / s.gnorm;
+        if (tid == 0) factor = -s.step / s.gnorm;   // one thread's division: they share the FP64 pipe
+        __syncthreads();
+        const double a = factor;
         int mv = 0;
         for (int i = i0 + tid; i < i1; i += MT) {
-            const double x1 = __dadd_rn(v.x[i], __dmul_rn(a, v.g[i]));
+            const double xi = v.x[i];
+            const double x1 = __dadd_rn(xi, __dmul_rn(a, v.g[i]));
             v.xt[i] = x1;
             v.xf[i] = float(x1);
-            if (x1 != v.x[i]) mv = 1;
+            if (x1 != xi) mv = 1;
         }
         mv = __syncthreads_or(mv);
-        if (tid == 0 && mv) atomicOr(&m.moved[p], 1);
-        double d0 = 0.0, d1 = 0.0, d2 = 0.0;
-        if (!pair_totals(m, p, nb, d0, d1, d2, red)) return;
+        if (nb > 1) {
+            if (tid == 0 && mv) atomicOr(&m.moved[p], 1);
+            if (!last_of_pair(m, p, nb)) return;
+            if (tid == 0) mv = atomicExch(&m.moved[p], 0);
+        }
         if (tid == 0) {
-            if (atomicExch(&m.moved[p], 0) == 0) {   // the step no longer changes x
+            if (mv == 0) {   // the step no longer changes x
                 st[p].done = 1;
                 st[p].status = 1;
                 active[p] = 0;
@@ -208,8 +252,8 @@ __global__ void __launch_bounds__(MT) k_min_propose(MinState *st, const PairVec 
             v.xt[i] = xi;
             v.xf[i] = float(xi);
         }
-        double d0 = 0.0, d1 = 0.0, d2 = 0.0;
-        if (!pair_totals(m, p, nb, d0, d1, d2, red)) return;
+        // (every block has read the state before its last one changes it)
+        if (!last_of_pair(m, p, nb)) return;
         if (tid == 0) {
             st[p].iter = s.iter + 1;
             active[p] = 1;
@@ -222,22 +266,25 @@ __global__ void __launch_bounds__(MT) k_min_update(MinState *st, const PairVec *
 {
     __shared__ double red[3 * MT / 32];
     const int p = blockIdx.y, tid = threadIdx.x;
-    if (!active[p]) return;
     const PairVec v = vec[p];
     const int nb = (v.n + MCH - 1) / MCH;
+    pdl_wait();
+    pdl_trigger();
+    if (!active[p]) return;
     if (int(blockIdx.x) >= nb) return;
     const int i0 = blockIdx.x * MCH, i1 = min(v.n, i0 + MCH);
     const MinState s = st[p];
     const double fe = v.costs[0] + v.costs[1];
+    const bool gdsq = mz.kind != MGR_MIN_GSL_SD;
     double q = 0.0, q2 = 0.0, mx = 0.0;
     if (s.phase == 0) {
         for (int i = i0 + tid; i < i1; i += MT) {
             const double gi = v.gt[i];
             v.g[i] = gi;
             q += gi * gi;
-            mx = fmax(mx, fabs(gi));
+            if (gdsq) mx = max_magnitude(mx, gi);
         }
-        if (!pair_totals(m, p, nb, q, q2, mx, red)) return;
+        if (!pair_totals(m, p, nb, q, q2, mx, gdsq, red)) return;
         if (tid == 0) {
             MinState &o = st[p];
             o.f = fe;
@@ -246,11 +293,11 @@ __global__ void __launch_bounds__(MT) k_min_update(MinState *st, const PairVec *
             o.phase = 1;
             o.evals = s.evals + 1;
             // all |g| < xtol
-            if (mz.kind == MGR_MIN_GDSQ && !(mx >= mz.xtol)) o.success = s.success | 1;
+            if (gdsq && !(mx >= mz.xtol)) o.success = s.success | 1;
         }
         return;
     }
-    if (mz.kind == MGR_MIN_GSL_SD) {
+    if (!gdsq) {
         if (fe > s.f) {
             if (blockIdx.x == 0 && tid == 0) {
                 st[p].evals = s.evals + 1;
@@ -265,7 +312,7 @@ __global__ void __launch_bounds__(MT) k_min_update(MinState *st, const PairVec *
             v.g[i] = gi;
             q += gi * gi;
         }
-        if (!pair_totals(m, p, nb, q, q2, mx, red)) return;
+        if (!pair_totals(m, p, nb, q, q2, mx, false, red)) return;
         if (tid == 0) {
             MinState &o = st[p];
             const double gn = sqrt(q);
@@ -293,9 +340,9 @@ __global__ void __launch_bounds__(MT) k_min_update(MinState *st, const PairVec *
             q2 += gs * gs;
             v.x[i] = v.xt[i];
             v.g[i] = gi;
-            mx = fmax(mx, fabs(gi));
+            mx = max_magnitude(mx, gi);
         }
-        if (!pair_totals(m, p, nb, q, q2, mx, red)) return;
+        if (!pair_totals(m, p, nb, q, q2, mx, true, red)) return;
         if (tid == 0) {
             MinState &o = st[p];
             const double nrm = sqrt(q2);
@@ -316,9 +363,9 @@ __global__ void __launch_bounds__(MT) k_min_update(MinState *st, const PairVec *
     } else {
         for (int i = i0 + tid; i < i1; i += MT) {
             v.xt[i] = v.x[i];
-            mx = fmax(mx, fabs(v.g[i]));
+            mx = max_magnitude(mx, v.g[i]);
         }
-        if (!pair_totals(m, p, nb, q, q2, mx, red)) return;
+        if (!pair_totals(m, p, nb, q, q2, mx, true, red)) return;
         if (tid == 0) {
             MinState &o = st[p];
             const double step = s.step / mz.scale;
@@ -516,6 +563,7 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     // (pair, tile) items from the device queue; the grid sizes are fixed
     // before any capture
     const bool queue = persistent && dim == 3;
+    const bool pdl = pairs[members[0]]->lvl->pdl;   // (the environment's setting: the same for all)
     int qgrid[2] = {0, 0};
     if (queue) {
         prepare_split_batch(dim, cost, tile[0], tile[1], tile[2], sm_warp, sm_adj);
@@ -523,21 +571,21 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         qgrid[1] = std::min(int(titems.size()), split3_queue_grid(cost, 1, sm_adj));
     }
     auto step = [&]() {
-        k_min_propose<<<mgrid, MT, 0, st>>>(d_states, d_vecs, mz, d_active, msc);
+        launch_pdl(pdl, k_min_propose, mgrid, dim3(MT), 0, st, d_states, d_vecs, mz, d_active, msc);
         if (queue) {
             launch_split3_queue(cost, d_args, d_titems, int(titems.size()), d_active, d_queue, qgrid[0], sm_warp,
-                                0, st);
+                                0, pdl, st);
             launch_split3_queue(cost, d_args, d_titems, int(titems.size()), d_active, d_queue + 2, qgrid[1], sm_adj,
-                                1, st);
+                                1, pdl, st);
         } else {
             if (!launch_split_batch(dim, cost, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
-                                    d_active, sm_warp, 0, st))
+                                    d_active, sm_warp, 0, pdl, st))
                 throw std::invalid_argument("tile shape not compiled in");
             launch_split_batch(dim, cost, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
-                               d_active, sm_adj, 1, st);
+                               d_active, sm_adj, 1, pdl, st);
         }
-        launch_gather_batch(dim, d_args, d_gitems, int(gitems.size()), d_active, d_nblocks, has_pen, st);
-        k_min_update<<<mgrid, MT, 0, st>>>(d_states, d_vecs, mz, d_active, msc);
+        launch_gather_batch(dim, d_args, d_gitems, int(gitems.size()), d_active, d_nblocks, pdl, st);
+        launch_pdl(pdl, k_min_update, mgrid, dim3(MT), 0, st, d_states, d_vecs, mz, d_active, msc);
         count_launch(2);
     };
     const int chunk = 8;

@@ -481,7 +481,7 @@ __device__ __forceinline__ void fused3_body(const EvalArgs &a, int bx, int by, i
     __syncthreads();
     if (is_last) {
         __threadfence();
-        reduce_tile_sums(a, ntiles, N, red);
+        reduce_tile_sums<NTF>(a, ntiles, N, red);
         if (tid == 0) a.counters[0] = 0;
     }
 }

@@ -180,15 +180,17 @@ __device__ __forceinline__ void gather2_body(const EvalArgs &a, int with_gradien
         double v2[2] = {0.0, 0.0};
         if (fin) {
             const int nt = X.nt * Y.nt;
-            for (int t = tid; t < nt; t += GT) v2[0] += __ldcg(a.tile_sums + size_t(t) * 5);
+            v2[0] = strided_sum(a.tile_sums, nt, tid, GT, 5);
         }
-        for (unsigned b = tid; b < unsigned(nblk); b += GT) v2[1] += ((volatile double *)a.pen_part)[b];
+        v2[1] = strided_sum(a.pen_part, nblk, tid, GT, 1);
         block_sum<2>(v2, red);
-        if (tid == 0) {
+        if (tid < 32) {
             if (fin) {
                 const double s5[5] = {v2[0], 0.0, 0.0, 0.0, 0.0};
                 finalise_cost(a, s5, size_t(a.n[0]) * a.n[1]);
             }
+        }
+        if (tid == 0) {
             double *sc = a.scalars;
             const double pen = a.has_penalty ? v2[1] : 0.0;
             sc[SC_PEN] = pen;
@@ -226,19 +228,19 @@ __global__ void __launch_bounds__(GT) k_gather2_batch(const EvalArgs *__restrict
                                                       const int *__restrict__ active, const int *__restrict__ nblocks)
 {
     const int2 it = items[blockIdx.x];
+    pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     gather2_body(args[it.x], 1, 0, it.y, nblocks[it.x]);
 }
 
 void launch_gather_batch(int dim, const EvalArgs *args, const int2 *items, int nitems, const int *active,
-                         const int *nblocks, int has_penalty, cudaStream_t st)
+                         const int *nblocks, bool pdl, cudaStream_t st)
 {
-    (void)has_penalty;
     if (dim == 3) {
-        launch_gather3_batch(args, items, nitems, active, nblocks, st);
+        launch_gather3_batch(args, items, nitems, active, nblocks, pdl, st);
         return;
     }
-    k_gather2_batch<<<nitems, GT, 0, st>>>(args, items, active, nblocks);
+    launch_pdl(pdl, k_gather2_batch, dim3(nitems), dim3(GT), 0, st, args, items, active, nblocks);
     count_launch();
 }
 

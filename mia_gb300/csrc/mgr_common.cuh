@@ -209,49 +209,94 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// The sums over the warp of five floats per lane in double, each with
-// warp_sum's tree (the same bits): lanes exchange halves of four of the
-// values, so that a step adds each pair once instead of in both lanes (11
-// FP64 additions per lane instead of 25).  v[k] of lane warp_sum5_lane(k)
-// holds sum k.
-__device__ __forceinline__ double warp_sum5(const float (&x)[5], int lane)
+// Sums over the warp, each with warp_sum's tree (the same bits).  FP64
+// additions issue at 1/64 of the FP32 rate here and several sums by every
+// lane are what a reduction's time goes to, so lanes exchange halves of the
+// values: a step adds each pair once instead of in both lanes.
+//
+// Two sums, 5 additions per lane instead of 10: sum 0 in lanes 0-15, sum 1 in
+// lanes 16-31.
+__device__ __forceinline__ double warp_sum2(double x0, double x1, int lane)
+{
+    const bool h16 = lane & 16;
+    double a = (h16 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, h16 ? x0 : x1, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+// Five sums, 11 additions instead of 25: even lanes hold sum (lane >> 3) & 3
+// of the first four, odd lanes sum 4.
+__device__ __forceinline__ double warp_sum5(const double (&x)[5], int lane)
 {
     const bool h16 = lane & 16, h8 = lane & 8;
-    const double x0 = widen(x[0]), x1 = widen(x[1]), x2 = widen(x[2]), x3 = widen(x[3]);
-    double a = (h16 ? x2 : x0) + __shfl_xor_sync(0xffffffffu, h16 ? x0 : x2, 16);
-    const double b = (h16 ? x3 : x1) + __shfl_xor_sync(0xffffffffu, h16 ? x1 : x3, 16);
+    double a = (h16 ? x[2] : x[0]) + __shfl_xor_sync(0xffffffffu, h16 ? x[0] : x[2], 16);
+    const double b = (h16 ? x[3] : x[1]) + __shfl_xor_sync(0xffffffffu, h16 ? x[1] : x[3], 16);
     a = (h8 ? b : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
     a += __shfl_xor_sync(0xffffffffu, a, 4);
     a += __shfl_xor_sync(0xffffffffu, a, 2);
     a += __shfl_xor_sync(0xffffffffu, a, 1);
-    const double e = warp_sum(widen(x[4]));
-    return lane & 1 ? e : a;   // even lanes: sum 2 * h16 + h8, odd lanes: sum 4
+    const double e = warp_sum(x[4]);
+    return lane & 1 ? e : a;
 }
 
-// Block-wide sum of K doubles per thread into red[0..K-1] (thread 0 holds
-// the result after the final __syncthreads).  `scratch` holds
-// K * (blockDim.x/32) doubles.  Order is fixed, so the result is
-// reproducible from run to run.
-template <int K>
+// Block-wide sums of K (1, 2 or 5) doubles per thread in a block of NW warps:
+// a warp_sum tree per warp, then the same tree over the warps' sums.  Every
+// lane of warp 0 holds the results after it; `scratch` holds K * NW doubles.
+// Order is fixed, so the result is reproducible from run to run.
+template <int K, int NW = 8>
 __device__ __forceinline__ void block_sum(double (&v)[K], double *scratch)
 {
+    static_assert(K == 1 || K == 2 || K == 5, "the sums that are taken together");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = warp_sum(v[k]);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < K; ++k) scratch[k * nw + wid] = v[k];
+    if constexpr (K == 1) {
+        const double s = warp_sum(v[0]);
+        if (lane == 0) scratch[wid] = s;
+    } else if constexpr (K == 2) {
+        const double s = warp_sum2(v[0], v[1], lane);
+        if ((lane & 15) == 0) scratch[(lane >> 4) * NW + wid] = s;
+    } else {
+        const double s = warp_sum5(v, lane);
+        if ((lane & 7) == 0) scratch[(lane >> 3) * NW + wid] = s;
+        if (lane == 1) scratch[4 * NW + wid] = s;
+    }
     __syncthreads();
-    if (wid == 0) {
+    if (NW != 8 && wid == 0) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            double s = lane < nw ? scratch[k * nw + lane] : 0.0;
-            s = warp_sum(s);
-            v[k] = s;
+        for (int k = 0; k < K; ++k) v[k] = warp_sum(lane < NW ? scratch[k * NW + lane] : 0.0);
+    } else if (wid == 0) {
+        // lane 8 k + w: sum k of warp w (k < 4), the last of five apart; the
+        // tree's first steps would add zeros
+#pragma unroll
+        for (int h = 0; h < (K == 5 ? 2 : 1); ++h) {
+            const int at = h * 4 * NW + lane;
+            double s = at < K * NW ? scratch[at] : 0.0;
+#pragma unroll
+            for (int o = NW / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+            for (int k = h * 4; k < (K < h * 4 + 4 ? K : h * 4 + 4); ++k)
+                v[k] = __shfl_sync(0xffffffffu, s, (k - h * 4) * NW);
         }
     }
     __syncthreads();
+}
+
+// p[t], p[t + step], ... below n added in this order, in batches of loads
+// (values that other blocks wrote: read through the L2); element i of p is
+// `stride` doubles after element i - 1
+template <int B = 8>
+__device__ __forceinline__ double strided_sum(const double *p, int n, int t, int step, int stride)
+{
+    double v = 0.0;
+    for (; t < n; t += B * step) {
+        double x[B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) x[j] = t + j * step < n ? __ldcg(p + size_t(t + j * step) * stride) : 0.0;
+#pragma unroll
+        for (int j = 0; j < B; ++j)
+            if (t + j * step < n) v += x[j];
+    }
+    return v;
 }
 
 // ---------------------------------------------------------------------

@@ -6,16 +6,21 @@
 
 namespace mgr {
 
-// Final SSD / NCC cost and force constants from the reduced sums (thread 0
-// of the last block only).  SSD: s[0] = sum (a-b)^2; value 0.5*s (x 1/N with
-// norm) as FEvalSSD (mia/template/ssd.hh:54-99).  NCC: s = sums of
-// da = a - c_a, db = b - c_b, da^2, db^2, da*db about provisional centres;
-// value and gradient helper as NCCSums::value / get_grad_helper of the SSE2
-// build (mia/core/nccsum.cc:31-120: 1e-10 and 1e-5 thresholds).
+// Final SSD / NCC cost and force constants from the reduced sums, by the lanes
+// of one warp (all call it with the same sums; lane 0 writes).  SSD: s[0] =
+// sum (a-b)^2; value 0.5*s (x 1/N with norm) as FEvalSSD
+// (mia/template/ssd.hh:54-99).  NCC: s = sums of da = a - c_a, db = b - c_b,
+// da^2, db^2, da*db about provisional centres; value and gradient helper as
+// NCCSums::value / get_grad_helper of the SSE2 build
+// (mia/core/nccsum.cc:31-120: 1e-10 and 1e-5 thresholds).  The quotients that
+// do not depend on one another are taken by different lanes: a division is a
+// chain of FP64 instructions, the longest part of a finalisation.
 __device__ __forceinline__ void finalise_cost(const EvalArgs &a, const double s[5], size_t N)
 {
+    const int lane = threadIdx.x & 31;
     double *sc = a.scalars;
     if (a.cost == 0) {
+        if (lane != 0) return;
         const double scale = a.ssd_norm ? 0.5 / double(N) : 0.5;
         sc[SC_VALUE] = scale * s[0];
         sc[SC_FORCE_COST] = scale * s[0];
@@ -25,20 +30,27 @@ __device__ __forceinline__ void finalise_cost(const EvalArgs &a, const double s[
     }
     const double n = double(N);
     const double sa = s[0], sb = s[1], saa = s[2], sbb = s[3], sab = s[4];
-    const double ma = a.centers[0] + sa / n, mb = a.centers[1] + sb / n;
-    const double s2a = saa - sa * sa / n;
-    const double s2b = sbb - sb * sb / n;
-    const double cab = sab - sa * sb / n;
+    const double ca = a.centers[0], cb = a.centers[1];
+    const double num = lane == 0 ? sa : lane == 1 ? sb : lane == 2 ? sa * sa : lane == 3 ? sb * sb : sa * sb;
+    const double q = num / n;
+    auto quotient = [](double x, int from) { return __shfl_sync(0xffffffffu, x, from); };
+    const double ma = ca + quotient(q, 0), mb = cb + quotient(q, 1);
+    const double s2a = saa - quotient(q, 2);
+    const double s2b = sbb - quotient(q, 3);
+    const double cab = sab - quotient(q, 4);
     const double p1 = s2a * s2b;
+    const double r = (lane == 0 ? cab * cab : cab) / (lane == 2 ? s2a : p1);
+    const double r0 = quotient(r, 0), r1 = quotient(r, 1), r2 = quotient(r, 2);   // cab^2 / p1, cab / p1, cab / s2a
+    if (lane != 0) return;
     double v = 1.0;
-    if (p1 > 1e-10) v = 1.0 - cab * cab / p1;
+    if (p1 > 1e-10) v = 1.0 - r0;
     else if (s2a < 1e-5 && s2b < 1e-5) v = 0.0;
     sc[SC_VALUE] = v;
     double fv = 1.0, k1 = 0.0, k2 = 0.0, hma = 0.0, hmb = 0.0;
     if (p1 > 1e-5) {
-        fv = 1.0 - cab * cab / p1;
-        k1 = 2.0 * (cab / p1);
-        k2 = cab / s2a;
+        fv = 1.0 - r0;
+        k1 = 2.0 * r1;
+        k2 = r2;
         hma = ma;
         hmb = mb;
     } else if (s2a < 1e-5 && s2b < 1e-5) {
@@ -53,17 +65,16 @@ __device__ __forceinline__ void finalise_cost(const EvalArgs &a, const double s[
 }
 
 // Reduce the per-tile sums in a fixed order (every thread of the last block
-// calls this), then finalise the cost.
+// calls this, NT threads), then finalise the cost.
+template <int NT = 256>
 __device__ __forceinline__ void reduce_tile_sums(const EvalArgs &a, int ntiles, size_t N, double *red)
 {
     double v[5] = {0, 0, 0, 0, 0};
-    for (int t = threadIdx.x; t < ntiles; t += blockDim.x) {
-        const volatile double *p = a.tile_sums + size_t(t) * 5;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) v[k] += p[k];
-    }
-    block_sum<5>(v, red);
-    if (threadIdx.x == 0) finalise_cost(a, v, N);
+    for (int k = 0; k < 5; ++k)
+        if (k == 0 || a.cost != 0) v[k] = strided_sum<4>(a.tile_sums + k, ntiles, threadIdx.x, NT, 5);
+    block_sum<5, NT / 32>(v, red);
+    if (threadIdx.x < 32) finalise_cost(a, v, N);
 }
 
 __device__ __forceinline__ float aw_at(const float4 *aw, int i, int k)

@@ -128,12 +128,13 @@ bool tile_supported(int dim, int tx, int ty, int tz);
 // (pair, tile) items (which = 0 warp, 1 adjoint) or (pair, block) items
 // (gather); pairs with active[pair] == 0 are skipped
 size_t split_smem(const EvalArgs &a, int which);
-// (all pairs of a batch have the same cost)
+// (all pairs of a batch have the same cost; pdl: launched to overlap with the
+// kernel before, EvalArgs::pdl)
 void prepare_split_batch(int dim, int cost, int tx, int ty, int tz, size_t sm_warp, size_t sm_adj);
 bool launch_split_batch(int dim, int cost, int tx, int ty, int tz, const EvalArgs *args, const int2 *items, int nitems,
-                        const int *active, size_t smem, int which, cudaStream_t st);
+                        const int *active, size_t smem, int which, bool pdl, cudaStream_t st);
 void launch_gather_batch(int dim, const EvalArgs *args, const int2 *items, int nitems, const int *active,
-                         const int *nblocks, int has_penalty, cudaStream_t st);
+                         const int *nblocks, bool pdl, cudaStream_t st);
 
 // 3D split path (split3.cu): tiles of 32 x 8 x tz voxels, z-walking threads;
 // launch_warp3 converts the parameters to float first (launch_params_f32)
@@ -149,7 +150,7 @@ void launch_adjoint3(const EvalArgs &a, cudaStream_t st);
 // before the first launch; the last block resets it)
 int split3_queue_grid(int cost, int which, size_t sm);
 void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue,
-                         int grid, size_t sm, int which, cudaStream_t st);
+                         int grid, size_t sm, int which, bool pdl, cudaStream_t st);
 // the fused SSD kernel (fused3.cu): warp, force and adjoint in one pass per
 // 30 x 8 x TZ tile; with_gradient = 0 sums the cost only
 bool tile_supported_fused3(int tx, int ty, int tz);
@@ -159,9 +160,9 @@ int gather3_blocks(const EvalArgs &a);
 void launch_gather3(const EvalArgs &a, int with_gradient, int dense, cudaStream_t st);
 void prepare_split3_batch(int cost, size_t sm_warp, size_t sm_adj);
 void launch_split3_batch(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
-                         int which, cudaStream_t st);
+                         int which, bool pdl, cudaStream_t st);
 void launch_gather3_batch(const EvalArgs *args, const int2 *items, int nitems, const int *active, const int *nblocks,
-                          cudaStream_t st);
+                          bool pdl, cudaStream_t st);
 
 // standalone pieces for tests and the plain path
 void launch_force(const EvalArgs &a, float *force, cudaStream_t st);       // force field from `warped`

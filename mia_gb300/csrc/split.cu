@@ -175,8 +175,9 @@ __device__ __forceinline__ void warp2_body(const EvalArgs &a, int bx, int by, in
         const double v = warp_sum(widen(acc[0]));
         if (lane == 0) red[wid] = v;
     } else {
-        const double v = warp_sum5(acc, lane);
-        if ((lane & 7) == 0) red[((lane >> 3) & 3) * NW + wid] = v;
+        const double x[5] = {widen(acc[0]), widen(acc[1]), widen(acc[2]), widen(acc[3]), widen(acc[4])};
+        const double v = warp_sum5(x, lane);
+        if ((lane & 7) == 0) red[(lane >> 3) * NW + wid] = v;
         if (lane == 1) red[4 * NW + wid] = v;
     }
     __syncthreads();
@@ -353,6 +354,7 @@ __global__ void __launch_bounds__(NT) k_warp2_batch(const EvalArgs *__restrict__
                                                     const int *__restrict__ active)
 {
     const int2 it = items[blockIdx.x];
+    pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     const EvalArgs &a = args[it.x];
     const int ntx = a.ax[0].nt;
@@ -364,6 +366,7 @@ __global__ void __launch_bounds__(NT) k_adjoint2_batch(const EvalArgs *__restric
                                                        const int2 *__restrict__ items, const int *__restrict__ active)
 {
     const int2 it = items[blockIdx.x];
+    pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     const EvalArgs &a = args[it.x];
     const int ntx = a.ax[0].nt;
@@ -456,12 +459,10 @@ size_t split_smem(const EvalArgs &a, int which)
 
 template <int TX, int TY>
 static void launch_batch_tile(const EvalArgs *args, const int2 *items, int nitems, const int *active,
-                              size_t sm, int which, cudaStream_t st)
+                              size_t sm, int which, bool pdl, cudaStream_t st)
 {
-    if (which == 0)
-        k_warp2_batch<TX, TY><<<nitems, NT, sm, st>>>(args, items, active);
-    else
-        k_adjoint2_batch<TX, TY><<<nitems, NT, sm, st>>>(args, items, active);
+    launch_pdl(pdl, which == 0 ? k_warp2_batch<TX, TY> : k_adjoint2_batch<TX, TY>, dim3(nitems), dim3(NT), sm, st, args,
+               items, active);
     count_launch();
 }
 
@@ -489,16 +490,16 @@ void prepare_split_batch(int dim, int cost, int tx, int ty, int tz, size_t sm_wa
 }
 
 bool launch_split_batch(int dim, int cost, int tx, int ty, int tz, const EvalArgs *args, const int2 *items, int nitems,
-                        const int *active, size_t sm, int which, cudaStream_t st)
+                        const int *active, size_t sm, int which, bool pdl, cudaStream_t st)
 {
     if (dim == 3) {
         if (!tile_supported3_batch(tx, ty, tz)) return false;
-        launch_split3_batch(cost, args, items, nitems, active, sm, which, st);
+        launch_split3_batch(cost, args, items, nitems, active, sm, which, pdl, st);
         return true;
     }
 #define MGR_BTILE2(X_, Y_)                                                      \
     if (tx == X_ && ty == Y_) {                                                 \
-        launch_batch_tile<X_, Y_>(args, items, nitems, active, sm, which, st); \
+        launch_batch_tile<X_, Y_>(args, items, nitems, active, sm, which, pdl, st); \
         return true;                                                            \
     }
     MGR_BTILE2(32, 8)

@@ -1167,15 +1167,17 @@ __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradien
         double v2[2] = {0.0, 0.0};
         if (fin) {
             const int ntw = a.ax[0].nt * a.ax[1].nt * a.ax[2].nt;
-            for (int t = tid; t < ntw; t += GT3) v2[0] += ((volatile double *)a.tile_sums)[size_t(t) * 5];
+            v2[0] = strided_sum(a.tile_sums, ntw, tid, GT3, 5);
         }
-        for (unsigned b = tid; b < unsigned(nblk); b += GT3) v2[1] += ((volatile double *)a.pen_part)[b];
+        v2[1] = strided_sum(a.pen_part, nblk, tid, GT3, 1);
         block_sum<2>(v2, red);
-        if (tid == 0) {
+        if (tid < 32) {
             if (fin) {
                 const double s5[5] = {v2[0], 0.0, 0.0, 0.0, 0.0};
                 finalise_cost(a, s5, size_t(a.n[0]) * a.n[1] * a.n[2]);
             }
+        }
+        if (tid == 0) {
             double *sc = a.scalars;
             const double pen = a.has_penalty ? v2[1] : 0.0;
             sc[SC_PEN] = pen;
@@ -1256,6 +1258,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_batch(const EvalAr
                                                                     const int *__restrict__ active)
 {
     const int2 it = items[blockIdx.x];
+    pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     const EvalArgs &a = args[it.x];
     int bx, by, bz, nt;
@@ -1268,6 +1271,7 @@ __global__ void MGR_ADJ_BOUNDS k_adjoint3_batch(const EvalArgs *__restrict__ arg
                                                         const int2 *__restrict__ items, const int *__restrict__ active)
 {
     const int2 it = items[blockIdx.x];
+    pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     const EvalArgs &a = args[it.x];
     int bx, by, bz, nt;
@@ -1310,6 +1314,8 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_queue(const EvalAr
 {
     __shared__ int slot;
     int2 it;
+    pdl_wait();
+    pdl_trigger();
     while (next_item(queue, nitems, items, it, slot)) {
         if (!active[it.x]) continue;
         const EvalArgs &a = args[it.x];
@@ -1327,6 +1333,8 @@ __global__ void MGR_ADJ_BOUNDS k_adjoint3_queue(const EvalArgs *__restrict__ arg
 {
     __shared__ int slot;
     int2 it;
+    pdl_wait();
+    pdl_trigger();
     while (next_item(queue, nitems, items, it, slot)) {
         if (!active[it.x]) continue;
         const EvalArgs &a = args[it.x];
@@ -1342,6 +1350,7 @@ __global__ void MGR_GATHER_BOUNDS k_gather3_batch(const EvalArgs *__restrict__ a
                                                        const int *__restrict__ nblocks)
 {
     const int2 it = items[blockIdx.x];
+    pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     gather3_body(args[it.x], 1, 0, it.y, nblocks[it.x]);
 }
@@ -1519,12 +1528,12 @@ void prepare_split3_batch(int cost, size_t sm_warp, size_t sm_adj)
 }
 
 void launch_split3_batch(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
-                         int which, cudaStream_t st)
+                         int which, bool pdl, cudaStream_t st)
 {
     if (which == 0)
-        warp3_batch_kernel(cost)<<<nitems, NT3, sm, st>>>(args, items, active);
+        launch_pdl(pdl, warp3_batch_kernel(cost), dim3(nitems), dim3(NT3), sm, st, args, items, active);
     else
-        k_adjoint3_batch<BATCH_TZ><<<nitems, AT3, sm, st>>>(args, items, active);
+        launch_pdl(pdl, k_adjoint3_batch<BATCH_TZ>, dim3(nitems), dim3(AT3), sm, st, args, items, active);
     count_launch();
 }
 
@@ -1540,19 +1549,19 @@ int split3_queue_grid(int cost, int which, size_t sm)
 }
 
 void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, int *queue,
-                         int grid, size_t sm, int which, cudaStream_t st)
+                         int grid, size_t sm, int which, bool pdl, cudaStream_t st)
 {
     if (which == 0)
-        warp3_queue_kernel(cost)<<<grid, NT3, sm, st>>>(args, items, nitems, active, queue);
+        launch_pdl(pdl, warp3_queue_kernel(cost), dim3(grid), dim3(NT3), sm, st, args, items, nitems, active, queue);
     else
-        k_adjoint3_queue<BATCH_TZ><<<grid, AT3, sm, st>>>(args, items, nitems, active, queue);
+        launch_pdl(pdl, k_adjoint3_queue<BATCH_TZ>, dim3(grid), dim3(AT3), sm, st, args, items, nitems, active, queue);
     count_launch();
 }
 
 void launch_gather3_batch(const EvalArgs *args, const int2 *items, int nitems, const int *active, const int *nblocks,
-                          cudaStream_t st)
+                          bool pdl, cudaStream_t st)
 {
-    k_gather3_batch<<<nitems, GT3, 0, st>>>(args, items, active, nblocks);
+    launch_pdl(pdl, k_gather3_batch, dim3(nitems), dim3(GT3), 0, st, args, items, active, nblocks);
     count_launch();
 }
 
