@@ -94,8 +94,11 @@ constexpr unsigned FULL = 0xffffffffu;
 // one after another 99.3 -> 92.2 us, 256^3 NCC 431 -> 396 us.
 //
 // COST: the image cost (MGR_COST_SSD / NCC); compiled per cost, the SSD
-// kernel keeps one sum and no branch on it
-template <int TZ, int COST>
+// kernel keeps one sum and no branch on it.  BATCH: a tile whose box is too
+// large for the ring (without the margin below) adds its squares rounded to
+// the SSD sum, every other one unrounded: the sums differ in the last bits,
+// and a batch's line searches would take other steps
+template <int TZ, int COST, bool BATCH>
 __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, int bz, int ntiles, int tile)
 {
     constexpr int NW = NT3 / 32;
@@ -284,7 +287,7 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
     // aligned in the padded rows), rows from ylo, planes zbase .. zbase +
     // nplanes - 1 of which step t needs t .. t + span - 1
     constexpr int H = PAD_H;
-    bool staged;
+    bool staged, rounded;   // rounded: the squares of planes not walked (BATCH)
     int xs, ylo, zbase, nplanes, span;
     {
         float ulo[3], uhi[3];
@@ -311,23 +314,24 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             m = fmaxf(m, fmaxf(fabsf(ulo[c]), fabsf(uhi[c])));
         }
         m = 1.0e-4f + 1.0e-6f * (m + float(max(nx, max(ny, nz))));
-        xs = ylo = zbase = nplanes = span = 0;
-        if (ok) {
-            const int xlo = int(floorf(float(x0) - uhi[0] - m)) - 1;
+        auto fits = [&](float margin) {
+            const int xlo = int(floorf(float(x0) - uhi[0] - margin)) - 1;
             const int xe = int(floorf(float(x0 + TX3 - 1) - ulo[0])) + 3;
             xs = ((xlo + H) & ~3) - H;
-            ylo = int(floorf(float(y0) - uhi[1] - m)) - 1;
+            ylo = int(floorf(float(y0) - uhi[1] - margin)) - 1;
             const int yhi = int(floorf(float(y0 + ey - 1) - ulo[1])) + 3;
-            const int dzl = int(floorf(-uhi[2] - m)) - 1;
+            const int dzl = int(floorf(-uhi[2] - margin)) - 1;
             const int dzh = int(floorf(-ulo[2])) + 3;
-            ok = xs >= -H && xe <= nx + H - 1 && xe - xs + 1 <= RING_X && ylo >= -H && yhi <= ny + H - 1 &&
-                 yhi - ylo + 1 <= RING_Y && z0 + dzl >= -H && z0 + ez - 1 + dzh <= nz + H - 1 &&
-                 dzh - dzl + 1 <= RING_N - 2;
             zbase = z0 + dzl;
             span = dzh - dzl + 1;
             nplanes = ez + span - 1;
-        }
-        staged = ok;
+            return xs >= -H && xe <= nx + H - 1 && xe - xs + 1 <= RING_X && ylo >= -H && yhi <= ny + H - 1 &&
+                   yhi - ylo + 1 <= RING_Y && z0 + dzl >= -H && z0 + ez - 1 + dzh <= nz + H - 1 &&
+                   span <= RING_N - 2;
+        };
+        xs = ylo = zbase = nplanes = span = 0;
+        staged = ok && fits(m);
+        rounded = BATCH && COST == MGR_COST_SSD && !staged && !(ok && fits(0.0f));
     }
     if (lane == 0) {   // for the refills this lane may issue
         boxs[wy][0] = xs + H;
@@ -366,10 +370,10 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
     const size_t nxy = size_t(nx) * ny;
     const size_t col = size_t(y) * nx + x + size_t(z0) * nxy;
     float acc[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    auto add_cost = [&](float wv, float b) {
+    auto add_cost = [&](float wv, float b, bool round) {
         if (cost == 0) {
             const float d = wv - b;
-            acc[0] += d * d;
+            acc[0] = round ? __fadd_rn(acc[0], __fmul_rn(d, d)) : __fmaf_rn(d, d, acc[0]);
         } else {
             const float da = wv - ca, db = b - cb;
             acc[0] += da;
@@ -471,10 +475,10 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
                 wa = fminf(fmaxf(wa, mn), mxv);
                 wb = fminf(fmaxf(wb, mn), mxv);
                 wout[0] = wa;
-                add_cost(wa, r0);
+                add_cost(wa, r0, false);
                 if (two) {
                     wout[nxy] = wb;
-                    add_cost(wb, r1);
+                    add_cost(wb, r1, false);
                 }
             }
             r0 = r2;
@@ -524,7 +528,7 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
                 u[c] = wa.x * qat(c, s) + wa.z * qat(c, s + 1) + wb.x * qat(c, s + 2) + wb.z * qat(c, s + 3);
             const float wv = taps3_global(a, px0 - u[0], py0 - u[1], float(z0 + t) - u[2], mn, mxv);
             a.warped[col + size_t(t) * nxy] = wv;
-            add_cost(wv, __ldg(a.ref + col + size_t(t) * nxy));
+            add_cost(wv, __ldg(a.ref + col + size_t(t) * nxy), rounded);
         }
     // tile sums: a float tree within each warp (5 levels), the warps' sums
     // added in double in a fixed order, one thread per sum (FP64 is slow
@@ -1215,7 +1219,7 @@ template <int TZ, int COST>
 __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3(const __grid_constant__ EvalArgs a)
 {
     const int tile = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    warp3_body<TZ, COST>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x * gridDim.y * gridDim.z, tile);
+    warp3_body<TZ, COST, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x * gridDim.y * gridDim.z, tile);
 }
 
 template <int TZ>
@@ -1263,7 +1267,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_batch(const EvalAr
     const EvalArgs &a = args[it.x];
     int bx, by, bz, nt;
     decode_tile3(a, it.y, bx, by, bz, nt);
-    warp3_body<TZ, COST>(a, bx, by, bz, nt, it.y);
+    warp3_body<TZ, COST, true>(a, bx, by, bz, nt, it.y);
 }
 
 template <int TZ>
@@ -1321,7 +1325,7 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_queue(const EvalAr
         const EvalArgs &a = args[it.x];
         int bx, by, bz, nt;
         decode_tile3(a, it.y, bx, by, bz, nt);
-        warp3_body<TZ, COST>(a, bx, by, bz, nt, it.y);
+        warp3_body<TZ, COST, true>(a, bx, by, bz, nt, it.y);
     }
     queue_done(queue);
 }
