@@ -47,21 +47,47 @@ __device__ __forceinline__ void gather2_body(const EvalArgs &a, int with_gradien
     const int cx = valid ? int(i % ncx) : 0;
     const int cy = valid ? int(i / ncx) : 0;
 
-    // the slots that hold the coefficient: entries k = w, w + GW, ... of the
-    // tiles [gx, gy]
+    // the first loads of both chains: the cells of the coefficient's row and
+    // the slots that hold it (entries k = w, w + GW, ... of the tiles)
     const bool img = valid && with_gradient && !image_from_dense;
-    int2 gx = make_int2(0, -1), gy = gx;
+    const bool pen = valid && a.has_penalty;
+    int nX = 0, nY = 0, e0 = 0, e1 = 0;
     if (img) {
-        gx = X.gtile[cx];
-        gy = Y.gtile[cy];
+        nX = X.glen[cx];
+        nY = Y.glen[cy];
     }
-    const int nX = gx.y - gx.x + 1, nY = gy.y - gy.x + 1;
+    if (pen) {
+        e0 = a.pen_rowptr[i] + w;
+        e1 = a.pen_rowptr[i + 1];
+    }
+    const bool lists = nX >= 0 && nY >= 0;
+    const int2 none = make_int2(0, -1);
+    const int2 gx = img && !lists ? X.gtile[cx] : none, gy = img && !lists ? Y.gtile[cy] : none;
+    if (!lists) {
+        nX = gx.y - gx.x + 1;
+        nY = gy.y - gy.x + 1;
+    }
     const int total = (nX > 0 && nY > 0) ? nX * nY : 0;
     auto slot = [&](int k) -> const float * {
-        const int jy = k / nX, tx = gx.x + (k - jy * nX), ty = gy.x + jy;
+        const int jy = k / nX, jx = k - jy * nX;
+        if (lists)
+            return a.partial + (X.glist[size_t(cx) * GATHER_LMAX + jx] + Y.glist[size_t(cy) * GATHER_LMAX + jy]);
+        const int tx = gx.x + jx, ty = gy.x + jy;
         const int lx = cx - X.atile0[tx], ly = cy - Y.atile0[ty];
         return a.partial + (size_t(ty) * X.nt + tx) * a.slot + (size_t(ly) * X.ac + lx) * 2;
     };
+    // the second loads: cells, slot offsets
+    float4 cell[GCELLS];
+    int col[GCELLS];
+    auto cells = [&]() {
+#pragma unroll
+        for (int u = 0; u < GCELLS; ++u) {
+            const bool in = e0 + u * GW < e1;
+            col[u] = in ? a.pen_col[e0 + u * GW] : -1;
+            cell[u] = in ? a.pen_val[e0 + u * GW] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    cells();
     const float *sp[GSLOTS];
 #pragma unroll
     for (int u = 0; u < GSLOTS; ++u) sp[u] = w + u * GW < total ? slot(w + u * GW) : nullptr;
@@ -72,34 +98,26 @@ __device__ __forceinline__ void gather2_body(const EvalArgs &a, int with_gradien
     // L2, never from a line an earlier kernel left in L1.
     if (!with_gradient) pdl_wait();
     float g[2] = {0.0f, 0.0f}, r[3] = {0, 0, 0}, s[2] = {0.0f, 0.0f};
-    if (valid && a.has_penalty) {
-        const int e1 = a.pen_rowptr[i + 1];
-        for (int e0 = a.pen_rowptr[i] + w; e0 < e1; e0 += GW * GCELLS) {
-            float4 v[GCELLS];
-            int j[GCELLS];
-            float2 c[GCELLS];
+    while (e0 < e1) {   // (at most once: a row has at most 49 cells)
+        float2 c[GCELLS];
 #pragma unroll
-            for (int u = 0; u < GCELLS; ++u) {
-                const bool in = e0 + u * GW < e1;
-                j[u] = in ? a.pen_col[e0 + u * GW] : -1;
-                v[u] = in ? a.pen_val[e0 + u * GW] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int u = 0; u < GCELLS; ++u)
+            c[u] = col[u] >= 0 ? __ldcg(reinterpret_cast<const float2 *>(a.params_f) + col[u])
+                               : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < GCELLS; ++u)
+            if (col[u] >= 0) {
+                const float cjx = c[u].x, cjy = c[u].y;
+                const float4 v = cell[u];
+                const float aa = cjx * v.x, bb = cjy * v.y, cxx = cjx * v.z, cyy = cjy * v.z;
+                g[0] += aa + aa + cyy;
+                g[1] += bb + bb + cxx;
+                r[0] += aa;
+                r[1] += cyy;
+                r[2] += bb;
             }
-#pragma unroll
-            for (int u = 0; u < GCELLS; ++u)
-                c[u] = j[u] >= 0 ? __ldcg(reinterpret_cast<const float2 *>(a.params_f) + j[u])
-                                 : make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int u = 0; u < GCELLS; ++u)
-                if (j[u] >= 0) {
-                    const float cjx = c[u].x, cjy = c[u].y;
-                    const float aa = cjx * v[u].x, bb = cjy * v[u].y, cxx = cjx * v[u].z, cyy = cjy * v[u].z;
-                    g[0] += aa + aa + cyy;
-                    g[1] += bb + bb + cxx;
-                    r[0] += aa;
-                    r[1] += cyy;
-                    r[2] += bb;
-                }
-        }
+        e0 += GW * GCELLS;
+        if (e0 < e1) cells();
     }
     float2 ci = make_float2(0.0f, 0.0f);
     if (w == 0 && valid && a.has_penalty) ci = __ldcg(reinterpret_cast<const float2 *>(a.params_f) + i);

@@ -357,15 +357,16 @@ struct mgr_level {
         const int D = d.dim;
         AxisDev *ax = A;
         for (int k = 0; k < D; ++k) build_axis(ax[k].h, n[k], nc[k], t[k]);
-        if (D == 3) {
+        {
             // per axis and coefficient: the partial-slot offset parts of the
-            // tiles that hold it, slot entry (tx, ty, tz) of coefficient
-            // (cx, cy, cz) being at glist_x + glist_y + glist_z
-            const int sl = D * ax[0].h.ac * ax[1].h.ac * ax[2].h.ac;
-            const long long total = (long long)ax[0].h.nt * ax[1].h.nt * ax[2].h.nt * sl;
+            // tiles that hold it, slot entry (tx, ty[, tz]) of coefficient
+            // (cx, cy[, cz]) being at glist_x + glist_y [+ glist_z]
+            const int acz = D == 3 ? ax[2].h.ac : 1, ntz = D == 3 ? ax[2].h.nt : 1;
+            const int sl = D * ax[0].h.ac * ax[1].h.ac * acz;
+            const long long total = (long long)ax[0].h.nt * ax[1].h.nt * ntz * sl;
             const long long ts[3] = {sl, (long long)ax[0].h.nt * sl, (long long)ax[0].h.nt * ax[1].h.nt * sl};
             const long long ls[3] = {D, (long long)ax[0].h.ac * D, (long long)ax[0].h.ac * ax[1].h.ac * D};
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < D; ++k) {
                 AxisHost &h = ax[k].h;
                 h.glist.assign(size_t(h.nc) * GATHER_LMAX, 0);
                 h.glen.assign(h.nc, -1);

@@ -171,6 +171,53 @@ __device__ __forceinline__ float sample2_at(const float *base, int sy, float px,
 }
 
 // ---------------------------------------------------------------------
+// Pairs of floats in a 64-bit register pair: one instruction does the
+// arithmetic of both, each rounded as its scalar form rounds.
+// ---------------------------------------------------------------------
+typedef unsigned long long float2x;
+
+__device__ __forceinline__ float2x pack2(float a, float b)
+{
+    float2x r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(float2x v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ float2x add2(float2x a, float2x b)
+{
+    float2x r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x add2_down(float2x a, float2x b)
+{
+    float2x r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x sub2(float2x a, float2x b)
+{
+    float2x r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x mul2(float2x a, float2x b)
+{
+    float2x r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c)
+{
+    float2x r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// ---------------------------------------------------------------------
 // programmatic dependent launch
 // ---------------------------------------------------------------------
 // A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization
@@ -311,8 +358,8 @@ struct Axis {
     const int *ftile0;  // per tile: first coefficient of the forward footprint
     const int *atile0;  // per tile: first coefficient of the adjoint footprint
     const int2 *gtile;  // per coefficient: tiles [lo, hi] whose adjoint footprint holds it
-    const int *glist;   // 3D, per coefficient: GATHER_LMAX offsets into the partial slots, this axis' part
-    const int *glen;    // 3D, per coefficient: entries of glist (-1: longer than GATHER_LMAX)
+    const int *glist;   // per coefficient: GATHER_LMAX offsets into the partial slots, this axis' part
+    const int *glen;    // per coefficient: entries of glist (-1: longer than GATHER_LMAX)
     int n;              // voxels
     int nc;             // coefficients
     int t;              // tile length (voxels)
@@ -322,7 +369,7 @@ struct Axis {
 };
 
 // longest per-axis list of tiles whose adjoint footprint holds a coefficient
-// that the 3D gather reads from the tables (longer lists take a slower path)
+// that the gather reads from the tables (longer lists take a slower path)
 constexpr int GATHER_LMAX = 24;
 // planes of the 3D warp kernel's shared-memory tap ring (split3.cu); the
 // tile-fit rule (mgr_level::tile_fits) counts them.  12 keeps three warp

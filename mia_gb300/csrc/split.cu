@@ -22,8 +22,11 @@
 // kernels are launched to overlap (pdl_wait), load everything that does not
 // depend on the kernel before them ahead of that wait, take the taps from
 // global memory (one round of 16 independent loads; staging them in shared
-// memory costs two more barriers and a copy) and spread each contraction
-// over one thread per output.
+// memory costs two more barriers and a copy).  1024x1024 NCC (1024 tiles) is
+// the other end: there the warp kernel's FP64 sums and the adjoint kernel's
+// shared-memory reads were the time; with four threads per sum, component
+// pairs and whole lines per thread 26 -> 22 and 15.7 -> 11.6 us, evaluations
+// one after another 26.6 -> 21.9 us (96x96 SSD 30.7 -> 30.4).
 #include "mgr_cost.cuh"
 #include "mgr_launch.hh"
 
@@ -32,6 +35,11 @@ namespace mgr {
 namespace {
 
 constexpr int NT = 256;
+constexpr int ACC_P = 36;   // pitch of a warp's 32 values (banks four apart from warp to warp)
+// resident blocks per SM of the warp kernel, whose threads wait for their
+// taps most of the time: 1024x1024 NCC 24.7 us an evaluation with the
+// compiler's choice, 21.9 with 4, 23.1 with 6, 24.1 with 8 (spills)
+constexpr int WARP2_MINB = 4;
 
 // bicubic sample at (px, py): from the mirror-padded copy while the taps lie
 // inside it, else with the indices folded on the unpadded image (sample2);
@@ -63,6 +71,7 @@ __device__ __forceinline__ void warp2_body(const EvalArgs &a, int bx, int by, in
     constexpr int NR = NT / TX, PT = TY / NR;
     extern __shared__ __align__(16) float sm[];
     __shared__ double red[5 * (NT / 32)];
+    __shared__ float accs[5][(NT / 32) * ACC_P];
     __shared__ float csc[2];   // NCC centres (converted once per block)
     __shared__ int fsy[TY];
     __shared__ float4 fwy[TY];
@@ -166,19 +175,29 @@ __device__ __forceinline__ void warp2_body(const EvalArgs &a, int bx, int by, in
             acc[4] += da * db;
         }
     }
-    // tile sums: warp trees in double (SSD has one sum), then a tree over
-    // the eight warps; FP64 additions are the kernel's slowest instructions
-    // (the five sums by every lane took half of it at 1024x1024)
+    // tile sums: per warp warp_sum's tree over its 32 lanes in double, then a
+    // tree over the eight warps.  FP64 additions are the kernel's slowest
+    // instructions (five trees by every lane took half of it at 1024x1024),
+    // so the values go through shared memory and four threads sum a tree: the
+    // lanes j, j + 4, ... of a warp each (levels 16, 8, 4), then among
+    // themselves (levels 2, 1).
     constexpr int NW = NT / 32;
     static_assert(NW == 8, "the tree over the warps");
-    if (a.cost == 0) {
-        const double v = warp_sum(widen(acc[0]));
-        if (lane == 0) red[wid] = v;
-    } else {
-        const double x[5] = {widen(acc[0]), widen(acc[1]), widen(acc[2]), widen(acc[3]), widen(acc[4])};
-        const double v = warp_sum5(x, lane);
-        if ((lane & 7) == 0) red[(lane >> 3) * NW + wid] = v;
-        if (lane == 1) red[4 * NW + wid] = v;
+    const int ncomp = a.cost == 0 ? 1 : 5;
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        if (k < ncomp) accs[k][wid * ACC_P + lane] = acc[k];
+    __syncthreads();
+    if (tid < ncomp * 32) {
+        const int k = tid >> 5, w8 = (tid >> 2) & 7, j = tid & 3;
+        const float *f = &accs[k][w8 * ACC_P + j];
+        double t[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) t[m] = widen(f[4 * m]) + widen(f[4 * m + 16]);
+        double v = (t[0] + t[2]) + (t[1] + t[3]);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        if (j == 0) red[k * NW + w8] = v;
     }
     __syncthreads();
     if (tid < 5) {
@@ -212,9 +231,12 @@ template <int TX, int TY>
 __device__ __forceinline__ void adjoint2_body(const EvalArgs &a, int bx, int by, int tile_index)
 {
     constexpr int NR = NT / TX, PT = TY / NR, TXP = TX + 1;
+    // the x stage by whole lines or by outputs (below)
+    constexpr bool LINES = TY >= 16;
     extern __shared__ __align__(16) float sm[];
     __shared__ int asx[TX], asy[TY];
     __shared__ float awx[TX * 4], awy[TY * 4];
+    __shared__ float4 awx2[LINES ? TX : 1][2];   // LINES: awx, each weight twice
     __shared__ float fsc[5];   // force constants (converted once per block)
     const Axis &X = a.ax[0], &Y = a.ax[1];
     const int nx = a.n[0], ny = a.n[1];
@@ -224,15 +246,17 @@ __device__ __forceinline__ void adjoint2_body(const EvalArgs &a, int bx, int by,
     const int ax0 = X.atile0[bx], ay0 = Y.atile0[by];
     const int tid = threadIdx.x, lane = tid & 31;
     float *part = a.partial + size_t(tile_index) * a.slot;
-    float *F = sm;                                        // [2][TY][TXP]
-    float *AX = F + 2 * TY * TXP;                         // [2][TY][AXc]
-    int2 *rx = reinterpret_cast<int2 *>(sm + ((2 * TY * (TXP + AXc) + 1) & ~1));   // [AXc] columns of a coefficient
+    // both components side by side: their arithmetic runs on register pairs
+    float2x *F = reinterpret_cast<float2x *>(sm);         // [TY][TXP]
+    float2x *AX = F + TY * TXP;                           // [TY][AXc]
+    int2 *rx = reinterpret_cast<int2 *>(AX + TY * AXc);   // [AXc] columns of a coefficient
     int2 *ry = rx + AXc;                                  // [AYc] rows
 
     // the level's tables and the reference, ahead of the wait
     for (int e = tid; e < TX * 4; e += NT) {
         const int xc = min(x0 + e / 4, nx - 1);
         awx[e] = reinterpret_cast<const float *>(X.aw)[size_t(xc) * 4 + (e & 3)];
+        if (LINES) reinterpret_cast<float2 *>(awx2[e / 4])[e & 3] = make_float2(awx[e], awx[e]);
         if ((e & 3) == 0) asx[e / 4] = X.as[xc] - ax0;
     }
     for (int e = tid; e < TY * 4; e += NT) {
@@ -303,33 +327,72 @@ __device__ __forceinline__ void adjoint2_body(const EvalArgs &a, int bx, int by,
                     f[1] = s * g[1];
                 }
             }
-            F[yy * TXP + xx] = f[0];
-            F[(TY + yy) * TXP + xx] = f[1];
+            F[yy * TXP + xx] = pack2(f[0], f[1]);
         }
     }
     __syncthreads();
-    // x stage: coefficient ox of row (component, yy), its columns ascending
-    for (int e = tid; e < 2 * TY * AXc; e += NT) {
-        const int r = e / AXc, ox = e - r * AXc;
-        if (r % TY >= ey) continue;
-        const float *f = F + r * TXP;
-        const int2 v = rx[ox];
-        float acc = 0.0f;
+    // x stage.  Tall tiles: a thread per row, a sliding window of four sums
+    // over its columns (a third of the loads, and shared-memory reads bound
+    // the kernel where there are many tiles); flat ones, of small images: a
+    // thread per output, the output's columns ascending (a short chain, all
+    // threads busy).  The same sums.
+    if (LINES) {
+        if (tid < ey) {
+            const float2x *f = F + tid * TXP;
+            float2x *dst = AX + tid * AXc;
+            float2x s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+            int oc = 0;
 #pragma unroll 4
-        for (int i = v.x; i < v.y; ++i) acc += awx[i * 4 + (ox - asx[i])] * f[i];
-        AX[e] = acc;
+            for (int i = 0; i < ex; ++i) {
+                const int o = asx[i];
+                while (oc < o) {
+                    dst[oc] = s0;
+                    s0 = s1;
+                    s1 = s2;
+                    s2 = s3;
+                    s3 = 0;
+                    ++oc;
+                }
+                const float4 u = awx2[i][0], v = awx2[i][1];
+                const float2x g = f[i];
+                s0 = fma2(pack2(u.x, u.y), g, s0);
+                s1 = fma2(pack2(u.z, u.w), g, s1);
+                s2 = fma2(pack2(v.x, v.y), g, s2);
+                s3 = fma2(pack2(v.z, v.w), g, s3);
+            }
+            if (oc < AXc) dst[oc] = s0;
+            if (oc + 1 < AXc) dst[oc + 1] = s1;
+            if (oc + 2 < AXc) dst[oc + 2] = s2;
+            if (oc + 3 < AXc) dst[oc + 3] = s3;
+            for (int o = oc + 4; o < AXc; ++o) dst[o] = 0;
+        }
+    } else {
+        for (int e = tid; e < ey * AXc; e += NT) {
+            const int r = e / AXc, ox = e - r * AXc;
+            const float2x *f = F + r * TXP;
+            const int2 v = rx[ox];
+            float2x acc = 0;
+#pragma unroll 4
+            for (int i = v.x; i < v.y; ++i) {
+                const float w = awx[i * 4 + (ox - asx[i])];
+                acc = fma2(pack2(w, w), f[i], acc);
+            }
+            AX[e] = acc;
+        }
     }
     __syncthreads();
     // y stage: coefficient (oy, ox), its rows ascending, into the slot
-    for (int e = tid; e < 2 * AYc * AXc; e += NT) {
-        const int comp = e & 1, q = e >> 1;
-        const int oy = q / AXc, ox = q - oy * AXc;
-        const float *f = AX + comp * TY * AXc + ox;
+    for (int e = tid; e < AYc * AXc; e += NT) {
+        const int oy = e / AXc, ox = e - oy * AXc;
+        const float2x *f = AX + ox;
         const int2 v = ry[oy];
-        float acc = 0.0f;
+        float2x acc = 0;
 #pragma unroll 4
-        for (int i = v.x; i < v.y; ++i) acc += awy[i * 4 + (oy - asy[i])] * f[i * AXc];
-        part[e] = acc;
+        for (int i = v.x; i < v.y; ++i) {
+            const float w = awy[i * 4 + (oy - asy[i])];
+            acc = fma2(pack2(w, w), f[i * AXc], acc);
+        }
+        reinterpret_cast<float2x *>(part)[e] = acc;
     }
 }
 
@@ -338,7 +401,7 @@ __device__ __forceinline__ void adjoint2_body(const EvalArgs &a, int bx, int by,
 // of (pair, tile) items; pairs whose minimizer has finished are skipped)
 // ---------------------------------------------------------------------
 template <int TX, int TY>
-__global__ void __launch_bounds__(NT) k_warp2(const __grid_constant__ EvalArgs a)
+__global__ void __launch_bounds__(NT, WARP2_MINB) k_warp2(const __grid_constant__ EvalArgs a)
 {
     warp2_body<TX, TY>(a, blockIdx.x, blockIdx.y, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x);
 }
@@ -350,7 +413,7 @@ __global__ void __launch_bounds__(NT) k_adjoint2(const __grid_constant__ EvalArg
 }
 
 template <int TX, int TY>
-__global__ void __launch_bounds__(NT) k_warp2_batch(const EvalArgs *__restrict__ args, const int2 *__restrict__ items,
+__global__ void __launch_bounds__(NT, WARP2_MINB) k_warp2_batch(const EvalArgs *__restrict__ args, const int2 *__restrict__ items,
                                                     const int *__restrict__ active)
 {
     const int2 it = items[blockIdx.x];
@@ -385,8 +448,7 @@ static size_t warp_smem(const EvalArgs &a)
 static size_t adjoint_smem(const EvalArgs &a)
 {
     const Axis &X = a.ax[0], &Y = a.ax[1];
-    const size_t f = (size_t(2) * Y.t * (X.t + 1 + X.ac) + 1) & ~size_t(1);
-    return (f + 2 * (X.ac + Y.ac)) * sizeof(float);
+    return (size_t(2) * Y.t * (X.t + 1 + X.ac) + 2 * (X.ac + Y.ac)) * sizeof(float);
 }
 
 template <int TX, int TY>

@@ -46,53 +46,6 @@ __device__ __noinline__ float taps3_global(const EvalArgs &a, float px, float py
     return sample3(a.coef_img, nx, ny, nz, px, py, pz, mn, mx);
 }
 
-// ---------------------------------------------------------------------
-// Pairs of floats in a 64-bit register pair: one instruction does the
-// arithmetic of both, each rounded as its scalar form rounds.
-// ---------------------------------------------------------------------
-typedef unsigned long long float2x;
-
-__device__ __forceinline__ float2x pack2(float a, float b)
-{
-    float2x r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(float2x v, float &a, float &b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ float2x add2(float2x a, float2x b)
-{
-    float2x r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float2x add2_down(float2x a, float2x b)
-{
-    float2x r;
-    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float2x sub2(float2x a, float2x b)
-{
-    float2x r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float2x mul2(float2x a, float2x b)
-{
-    float2x r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c)
-{
-    float2x r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // ffloor16 of two coordinates below 2^22 in magnitude: rounding to the
 // nearest multiple of 2^-16 before the floor is adding half of one before it,
 // and a sum rounded down at 1.5 * 2^23 has the floor in its low bits: returns
