@@ -104,3 +104,30 @@ def test_host_access_and_launch_forms_agree(size, cost):
         c = call()
         w = lv.evaluate(params)
         assert c == w[0] + w[1] and np.array_equal(grad, w[4])
+
+
+@pytest.mark.parametrize("at", [(16, 12), (31, 31), (32, 8), (8, 24), (33, 15)])
+def test_an_infinite_force_reaches_the_four_coefficients_of_each_axis(at):
+    """A force that overflows: the gradient is not finite at the four
+    by four coefficients that the spline contracts its pixel with, those of
+    weight 0 included (pixels on a coefficient), and finite at every other
+    one, for every tile shape."""
+    import mia_gb300 as M
+    from mia_gb300 import synth
+    size = (41, 33)   # rate 8: every eighth pixel lies on a coefficient
+    rng = np.random.default_rng(5)
+    mov, ref = (1e6 * rng.random((2, size[1], size[0]))).astype(np.float32)
+    ref[at[1], at[0]] = 3e38   # times a difference of about 1e5
+    lv = M.Level(size, rate=8.0, cost="ssd")
+    p = synth.smooth_params(lv.csize, 0.7, seed=2)
+    ncx, ncy = lv.csize[:2]
+
+    def first(i):   # first coefficient o >= 0 with |i / 8 + 1 - o| < 2
+        return i // 8
+    want = np.zeros((ncy, ncx), bool)
+    want[first(at[1]):first(at[1]) + 4, first(at[0]):first(at[0]) + 4] = True
+    lv.set_images(mov, ref)
+    for tile in TILES:
+        lv.set_path("split", tile)
+        g = np.asarray(lv.evaluate(p)[2]).reshape(ncy, ncx, 2)
+        np.testing.assert_array_equal(~np.isfinite(g).all(axis=2), want, err_msg=str(tile))
