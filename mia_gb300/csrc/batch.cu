@@ -128,12 +128,10 @@ __device__ bool last_of_pair(const MinScratch &m, int p, int nb)
     __syncthreads();   // every thread has read the pair's state
     if (nb == 1) return true;
     if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(&m.count[p], 1u) == unsigned(nb - 1);
+        last = arrive_last(&m.count[p], nb);
         if (last) m.count[p] = 0;
     }
     __syncthreads();
-    if (last) __threadfence();
     return last;
 }
 
@@ -498,8 +496,8 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         a.grad_penalty = nullptr;
         a.costs = costs;
         a.convert = 0;   // k_min_propose writes the float copy
-        // 2D SSD: the gather's last block finalises the cost
-        a.defer_cost = dim == 2 && a.cost == MGR_COST_SSD;
+        // SSD: the gather's last block finalises the cost
+        a.defer_cost = a.cost == MGR_COST_SSD;
         args[k] = a;
         vecs[k] = PairVec{r.x, g, xt, gt, costs, int(n), a.params_f};
         MinState s{};

@@ -16,7 +16,11 @@
 // A few blocks with a chain of dependent loads (row range, cell, parameter;
 // tile range, tile start, slot): latency bounds it, so the loads of a step
 // are issued together and everything but the slots is done before the wait
-// for the adjoint kernel.
+// for the adjoint kernel.  Of 18.7 k cycles at 96x96 the last block's sums
+// were 7 k and the blocks' ends 5 k: a warp per gradient component and one
+// for the value, whose thread arrives with no other store in flight, and
+// loads in flight together make it 10.3 -> 8.0 us (an evaluation from host
+// memory 30.1 -> 28.7 us).
 #include "mgr_cost.cuh"
 #include "mgr_launch.hh"
 
@@ -120,9 +124,12 @@ __device__ __forceinline__ void gather2_body(const EvalArgs &a, int with_gradien
         if (e0 < e1) cells();
     }
     float2 ci = make_float2(0.0f, 0.0f);
-    if (w == 0 && valid && a.has_penalty) ci = __ldcg(reinterpret_cast<const float2 *>(a.params_f) + i);
+    if (w == 2 && pen) ci = __ldcg(reinterpret_cast<const float2 *>(a.params_f) + i);
     if (with_gradient) pdl_wait();
     pdl_trigger();
+    // parameters the warp kernel found non-finite: nothing is written to the
+    // caller's buffers (read by every block before its arrival)
+    const bool bad = a.params_host && *(volatile unsigned *)&a.counters[7] != 0u;
     {
         float2 v[GSLOTS];
 #pragma unroll
@@ -156,83 +163,28 @@ __device__ __forceinline__ void gather2_body(const EvalArgs &a, int with_gradien
         part[0][w][lane] = t;
     }
     __syncthreads();
-    if (w == 0) {
-        double pval = 0.0;
-        // parameters the warp kernel found non-finite: nothing is written to
-        // the caller's buffers (uniform over the block)
-        const bool bad = a.params_host && *(volatile unsigned *)&a.counters[7] != 0u;
-        if (valid) {
-            const float G[2] = {part[0][0][lane], part[0][1][lane]};
-            const float R[3] = {part[0][2][lane], part[0][3][lane], part[0][4][lane]};
-            const float S[2] = {part[0][5][lane], part[0][6][lane]};
-            double gp[2] = {0.0, 0.0};
-            if (a.has_penalty) {
-                const float v = ci.x * R[0] + ci.x * R[1] + ci.y * R[2];
-                pval = v;
-#pragma unroll
-                for (int k = 0; k < 2; ++k) gp[k] = (a.pen_grad_sign * a.pen_weight) * double(G[k]);
-            }
-            if (with_gradient && !bad) {
-#pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    const double gi = image_from_dense ? a.grad_image[i * 2 + k] : a.cost_weight * (-double(S[k]));
-                    a.grad_total[i * 2 + k] = gi + gp[k];
-                    if (a.grad_image && !image_from_dense) a.grad_image[i * 2 + k] = gi;
-                    if (a.grad_penalty) a.grad_penalty[i * 2 + k] = gp[k];
-                }
-            }
+    // a warp per component of the gradient, one for the penalty's value and
+    // the block's arrival
+    if (w < 2) {
+        if (valid && with_gradient && !bad) {
+            const size_t o = i * 2 + w;
+            const double gp = a.has_penalty ? a.pen_grad_w * widen(part[0][w][lane]) : 0.0;
+            const double gi = image_from_dense ? a.grad_image[o] : a.cost_weight * widen(-part[0][5 + w][lane]);
+            a.grad_total[o] = gi + gp;
+            if (a.grad_image && !image_from_dense) a.grad_image[o] = gi;
+            if (a.grad_penalty) a.grad_penalty[o] = gp;
         }
+    } else if (w == 2) {
+        double pval = 0.0;
+        if (pen) pval = widen(ci.x * part[0][2][lane] + ci.x * part[0][3][lane] + ci.y * part[0][4][lane]);
         pval = warp_sum(pval);
         if (lane == 0) {
             a.pen_part[blk] = pval;
-            __threadfence();
-            is_last = (atomicAdd(&a.counters[1], 1u) == unsigned(nblk - 1));
+            is_last = arrive_last(&a.counters[1], nblk);
         }
     }
     __syncthreads();
-    if (is_last) {
-        __threadfence();
-        // v[0]: a deferred SSD cost from the warp kernel's tile sums (the
-        // order of reduce_tile_sums); v[1]: the blocks' penalty partials
-        const bool fin = a.defer_cost && a.cost == 0;
-        double v2[2] = {0.0, 0.0};
-        if (fin) {
-            const int nt = X.nt * Y.nt;
-            v2[0] = strided_sum(a.tile_sums, nt, tid, GT, 5);
-        }
-        v2[1] = strided_sum(a.pen_part, nblk, tid, GT, 1);
-        block_sum<2>(v2, red);
-        if (tid < 32) {
-            if (fin) {
-                const double s5[5] = {v2[0], 0.0, 0.0, 0.0, 0.0};
-                finalise_cost(a, s5, size_t(a.n[0]) * a.n[1]);
-            }
-        }
-        if (tid == 0) {
-            double *sc = a.scalars;
-            const double pen = a.has_penalty ? v2[1] : 0.0;
-            sc[SC_PEN] = pen;
-            const double im = with_gradient ? sc[SC_FORCE_COST] : sc[SC_VALUE];
-            sc[SC_COST_IMG] = a.cost_weight * im;
-            sc[SC_COST_PEN] = a.has_penalty ? a.pen_weight * pen : 0.0;
-            if (a.costs) {
-                a.costs[0] = sc[SC_COST_IMG];
-                a.costs[1] = sc[SC_COST_PEN];
-            }
-            if (a.host_out) {
-                // the costs and both status flags to the caller's host
-                // memory; the non-finite flag is cleared for the next call
-                // (every block has read it before its arrival above)
-                a.host_out[0] = sc[SC_COST_IMG];
-                a.host_out[1] = sc[SC_COST_PEN];
-                unsigned *hf = reinterpret_cast<unsigned *>(a.host_out + 2);
-                hf[0] = *(volatile unsigned *)&a.counters[6];
-                hf[1] = *(volatile unsigned *)&a.counters[7];
-                a.counters[7] = 0;
-            }
-            a.counters[1] = 0;
-        }
-    }
+    if (is_last) gather_costs<GT>(a, X.nt * Y.nt, nblk, with_gradient, size_t(a.n[0]) * a.n[1], red);
 }
 
 __global__ void __launch_bounds__(GT) k_gather2(const __grid_constant__ EvalArgs a, int with_gradient,

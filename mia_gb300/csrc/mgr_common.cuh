@@ -328,22 +328,36 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double *scratch)
     __syncthreads();
 }
 
-// p[t], p[t + step], ... below n added in this order, in batches of loads
-// (values that other blocks wrote: read through the L2); element i of p is
-// `stride` doubles after element i - 1
-template <int B = 8>
-__device__ __forceinline__ double strided_sum(const double *p, int n, int t, int step, int stride)
+// K sums at a time: components 0 .. K - 1 of the elements t, t + step, ...
+// below n of p (element i at p + i * stride) added to v in this order, in
+// batches of B elements whose loads are all in flight together (values that
+// other blocks wrote: read through the L2)
+template <int B, int K>
+__device__ __forceinline__ void strided_sums(const double *p, int n, int t, int step, int stride, double (&v)[K])
 {
-    double v = 0.0;
     for (; t < n; t += B * step) {
-        double x[B];
-#pragma unroll
-        for (int j = 0; j < B; ++j) x[j] = t + j * step < n ? __ldcg(p + size_t(t + j * step) * stride) : 0.0;
+        double x[B][K];
 #pragma unroll
         for (int j = 0; j < B; ++j)
-            if (t + j * step < n) v += x[j];
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                x[j][k] = t + j * step < n ? __ldcg(p + size_t(t + j * step) * stride + k) : 0.0;
+#pragma unroll
+        for (int j = 0; j < B; ++j)
+            if (t + j * step < n)
+#pragma unroll
+                for (int k = 0; k < K; ++k) v[k] += x[j][k];
     }
-    return v;
+}
+
+// Arrival at a counter: true for the last of n.  What the thread wrote before
+// it, and what its block wrote before the barrier before it, is visible to
+// the last one and, after its next barrier, to its block.
+__device__ __forceinline__ bool arrive_last(unsigned *counter, int n)
+{
+    unsigned before;
+    asm volatile("atom.acq_rel.gpu.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+    return before == unsigned(n - 1);
 }
 
 // ---------------------------------------------------------------------

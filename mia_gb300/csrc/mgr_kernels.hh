@@ -82,7 +82,10 @@ struct EvalArgs {
     // penalty
     int has_penalty;
     double pen_weight;     // effective weight (norm already applied)
-    double pen_grad_sign;  // -1: the reference's penalty gradient sign, +1: corrected
+    double pen_grad_w;     // pen_weight, negative for the reference's penalty gradient sign (corrected: positive)
+    // the gather's weights as float (3D; FP64 instructions are slow)
+    float pen_grad_wf;     // pen_grad_w
+    float cost_wf;         // cost_weight
     int pen_equal_w;       // div == curl (multiply skips the cross terms)
     const float *ptable;   // 3D: 9x9x9 cells x 6 floats (xx, xy, yy, yz, zz, xz)
     const int *pen_rowptr; // 2D: CSR rows of the boundary-clipped matrix
@@ -106,7 +109,8 @@ struct EvalArgs {
     // reduction): an SSD cost by the gather's last block (the adjoint takes
     // its force scale from the settings), an NCC cost by k_finalise3, which
     // launch_warp3 queues right after the warp kernel (2D: SSD only); 0: the
-    // warp kernel's last block finalises the cost
+    // warp kernel's last block finalises the cost (3D: only a batch's NCC
+    // kernel can, a single evaluation's is followed by k_finalise3)
     int defer_cost;
     // 1: the split path's adjoint and gather kernels (3D: the warp kernel,
     // too) are launched with programmatic stream serialisation (each may start while the one

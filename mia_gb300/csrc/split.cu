@@ -212,13 +212,9 @@ __device__ __forceinline__ void warp2_body(const EvalArgs &a, int bx, int by, in
     // last-block pass here
     if (a.defer_cost) return;
     __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        is_last = (atomicAdd(&a.counters[0], 1u) == unsigned(ntiles - 1));
-    }
+    if (tid == 0) is_last = arrive_last(&a.counters[0], ntiles);
     __syncthreads();
     if (is_last) {
-        __threadfence();
         reduce_tile_sums(a, ntiles, size_t(nx) * ny, red);
         if (tid == 0) a.counters[0] = 0;
     }

@@ -560,17 +560,14 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             for (int w = 0; w < NW; ++w) v += widen(wsum[tid][w]);
         a.tile_sums[size_t(tile) * 5 + tid] = v;
     }
-    // a deferred finalisation (the gather's for SSD, k_finalise3's for NCC)
-    // needs no last-block pass here
-    if (a.defer_cost) return;
+    // SSD costs are finalised by the gather, a single evaluation's NCC cost by
+    // k_finalise3: only a batch's NCC kernel has a last-block pass (its code
+    // alone costs the others 1 %: 383x351x317 SSD 662 -> 654 us)
+    if (!BATCH || COST == MGR_COST_SSD) return;
     __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        is_last = (atomicAdd(&a.counters[0], 1u) == unsigned(ntiles - 1));
-    }
+    if (tid == 0) is_last = arrive_last(&a.counters[0], ntiles);
     __syncthreads();
     if (is_last) {
-        __threadfence();
         reduce_tile_sums(a, ntiles, size_t(nx) * ny * nz, red);
         if (tid == 0) a.counters[0] = 0;
     }
@@ -847,11 +844,10 @@ __device__ __forceinline__ void adjoint3_body(const EvalArgs &a, int bx, int by,
 #ifndef MGR_GATHER_THREADS
 #define MGR_GATHER_THREADS 256
 #endif
-#ifdef MGR_GATHER_MINB
-#define MGR_GATHER_BOUNDS __launch_bounds__(MGR_GATHER_THREADS, MGR_GATHER_MINB)
-#else
-#define MGR_GATHER_BOUNDS __launch_bounds__(MGR_GATHER_THREADS)
+#ifndef MGR_GATHER_MINB
+#define MGR_GATHER_MINB 4
 #endif
+#define MGR_GATHER_BOUNDS __launch_bounds__(MGR_GATHER_THREADS, MGR_GATHER_MINB)
 namespace {
 constexpr int GT3 = MGR_GATHER_THREADS;
 constexpr int GBX = 4, GBY = 4, GBZ = 2;   // coefficients per block: 32, lane = coefficient
@@ -875,6 +871,13 @@ static_assert(!GALIAS || GSUB * GNQ * 32 <= 4 * GTAB, "partials must fit in the 
 // issued in two batches: the tables, the parameters with a 3-node halo and
 // the penalty cells; then the partial slots, in flight while the stencil
 // is summed.
+// A block's chain of steps is the kernel's time on small grids, so its end is
+// short: a warp per gradient component, one for the value, whose thread
+// arrives with no other store in flight, no FP64 but the sums, and a last
+// block whose loads are in flight together.  40x44x36 NCC, alone on the GPU:
+// 13.1 -> 11.7 us (of 29.8 k cycles 10 k were the end, 6 k the last block);
+// evaluations one after another 13.8 -> 13.0 us, the value alone of
+// 160x176x144 120 -> 117 us.
 __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradient, int image_from_dense, int blk,
                                              int nblk)
 {
@@ -898,16 +901,18 @@ __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradien
     const bool img = with_gradient && !image_from_dense;
 
     // fixed tables first: offset lists and penalty cells
-    if (img && tid < 3 * GBX) {
-        const int ax = tid / GBX, k = tid - ax * GBX;
-        const Axis &A = a.ax[ax];
-        const int c = (ax == 0 ? cx0 : ax == 1 ? cy0 : cz0) + k;
-        int cnt = 0;
-        if (c < A.nc && (ax < 2 || k < GBZ)) {
-            cnt = A.glen[c];
-            for (int j = 0; j < cnt; ++j) gl[ax][k][j] = A.glist[size_t(c) * GATHER_LMAX + j];
+    if (img) {
+        if (tid < 3 * GBX) {
+            const int ax = tid / GBX, k = tid - ax * GBX;
+            const int c = (ax == 0 ? cx0 : ax == 1 ? cy0 : cz0) + k;
+            gn[ax][k] = c < a.nc[ax] && (ax < 2 || k < GBZ) ? a.ax[ax].glen[c] : 0;
         }
-        gn[ax][k] = cnt;
+        // whole lists (0 past their length), every entry by a thread of its own
+        for (int e = tid; e < 3 * GBX * GATHER_LMAX; e += GT3) {
+            const int ax = e / (GBX * GATHER_LMAX), r = e - ax * (GBX * GATHER_LMAX), k = r / GATHER_LMAX;
+            const int base = ax == 0 ? cx0 : ax == 1 ? cy0 : cz0;
+            if (base + k < a.nc[ax]) gl[ax][k][r - k * GATHER_LMAX] = a.ax[ax].glist[size_t(base) * GATHER_LMAX + r];
+        }
     }
     if (a.has_penalty) {
         constexpr int KT = (343 + GT3 - 1) / GT3;
@@ -993,10 +998,12 @@ __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradien
     }
     pdl_wait();
     pdl_trigger();
+    // parameters the conversion found non-finite: nothing is written to the
+    // caller's buffers (read by every block before its arrival)
+    const bool bad = a.params_host && *(volatile unsigned *)&a.counters[7] != 0u;
     // the adjoint's partial slots: this warp's share (entries k = w,
-    // w + GSUB, ...) of the lane's coefficient, one batch of loads
+    // w + GSUB, ...) of the lane's coefficient, in batches of loads
     constexpr int SMAX = GSMAX;
-    float sv[SMAX][3];
     int tot = 0, nX = 0, nY = 0, nZ = 0;
     bool lists = false;
     if (valid && img) {
@@ -1006,55 +1013,47 @@ __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradien
         lists = nX >= 0 && nY >= 0 && nZ >= 0;
         if (lists) tot = nX * nY * nZ;
     }
-#pragma unroll
-    for (int u = 0; u < SMAX; ++u) {
-        const int k = w + GSUB * u;
-        sv[u][0] = sv[u][1] = sv[u][2] = 0.0f;
-        if (k < tot) {
-            const int jx = k % nX, r = k / nX;
-            const int jy = r % nY, jz = r / nY;
-            const float *p = a.partial + (size_t(gl[2][lz][jz] + gl[1][ly][jy]) + gl[0][lx][jx]);
-            sv[u][0] = p[0];
-            sv[u][1] = p[1];
-            sv[u][2] = p[2];
-        }
-    }
     float S0 = 0.0f, S1 = 0.0f, S2 = 0.0f;
+    for (int k0 = w; k0 < tot; k0 += GSUB * SMAX) {
+        float sv[SMAX][3];
 #pragma unroll
-    for (int u = 0; u < SMAX; ++u) {
-        S0 += sv[u][0];
-        S1 += sv[u][1];
-        S2 += sv[u][2];
-    }
-    if (valid && img) {
-        if (lists) {
-            for (int k = w + GSUB * SMAX; k < tot; k += GSUB) {
+        for (int u = 0; u < SMAX; ++u) {
+            const int k = k0 + GSUB * u;
+            sv[u][0] = sv[u][1] = sv[u][2] = 0.0f;
+            if (k < tot) {
                 const int jx = k % nX, r = k / nX;
                 const int jy = r % nY, jz = r / nY;
                 const float *p = a.partial + (size_t(gl[2][lz][jz] + gl[1][ly][jy]) + gl[0][lx][jx]);
-                S0 += p[0];
-                S1 += p[1];
-                S2 += p[2];
+                sv[u][0] = p[0];
+                sv[u][1] = p[1];
+                sv[u][2] = p[2];
             }
-        } else {
-            const int2 gx = X.gtile[cx], gy = Y.gtile[cy], gz = Z.gtile[cz];
-            const int mX = gx.y - gx.x + 1, mY = gy.y - gy.x + 1, mZ = gz.y - gz.x + 1;
-            const int mt = (mX > 0 && mY > 0 && mZ > 0) ? mX * mY * mZ : 0;
-            for (int k = w; k < mt; k += GSUB) {
-                const int tx = gx.x + k % mX, ty = gy.x + (k / mX) % mY, tz = gz.x + k / (mX * mY);
-                const int lxo = cx - X.atile0[tx], lyo = cy - Y.atile0[ty], lzo = cz - Z.atile0[tz];
-                const size_t t = (size_t(tz) * Y.nt + ty) * X.nt + tx;
-                const float *p = a.partial + t * a.slot + ((size_t(lzo) * Y.ac + lyo) * X.ac + lxo) * 3;
-                S0 += p[0];
-                S1 += p[1];
-                S2 += p[2];
-            }
+        }
+#pragma unroll
+        for (int u = 0; u < SMAX; ++u) {
+            S0 += sv[u][0];
+            S1 += sv[u][1];
+            S2 += sv[u][2];
+        }
+    }
+    if (valid && img && !lists) {
+        const int2 gx = X.gtile[cx], gy = Y.gtile[cy], gz = Z.gtile[cz];
+        const int mX = gx.y - gx.x + 1, mY = gy.y - gy.x + 1, mZ = gz.y - gz.x + 1;
+        const int mt = (mX > 0 && mY > 0 && mZ > 0) ? mX * mY * mZ : 0;
+        for (int k = w; k < mt; k += GSUB) {
+            const int tx = gx.x + k % mX, ty = gy.x + (k / mX) % mY, tz = gz.x + k / (mX * mY);
+            const int lxo = cx - X.atile0[tx], lyo = cy - Y.atile0[ty], lzo = cz - Z.atile0[tz];
+            const size_t t = (size_t(tz) * Y.nt + ty) * X.nt + tx;
+            const float *p = a.partial + t * a.slot + ((size_t(lzo) * Y.ac + lyo) * X.ac + lxo) * 3;
+            S0 += p[0];
+            S1 += p[1];
+            S2 += p[2];
         }
     }
     // the lane's own parameters (the penalty value), read before the
     // partials may take the tables' place
     float ci[3] = {0.0f, 0.0f, 0.0f};
-    if (w == 0 && a.has_penalty) {
+    if (w == 3 && a.has_penalty) {
         const float4 c4 = Ps[((lz + GH) * GPY + (ly + GH)) * GPP + (lx + GH)];
         ci[0] = c4.x;
         ci[1] = c4.y;
@@ -1084,126 +1083,71 @@ __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradien
         pacc[0][k][lane] = t;
     }
     __syncthreads();
-    if (w == 0) {
-        float pval = 0.0f;
-        // parameters the conversion found non-finite: nothing is written to
-        // the caller's buffers (uniform over the block)
-        const bool bad = a.params_host && *(volatile unsigned *)&a.counters[7] != 0u;
-        double gt[3] = {0.0, 0.0, 0.0};
-        if (valid) {
-            float v9[GNQ];
-#pragma unroll
-            for (int k = 0; k < GNQ; ++k) v9[k] = pacc[0][k][lane];
-            float gp[3] = {0.0f, 0.0f, 0.0f};
-            const float pw = float(a.pen_grad_sign * a.pen_weight), cw = float(a.cost_weight);
-            if (a.has_penalty) {
-                const float ci0 = ci[0], ci1 = ci[1], ci2 = ci[2];
-                if (with_gradient)
-                    pval = ci0 * v9[0] + ci0 * v9[1] + ci1 * v9[2] + ci1 * v9[3] + ci2 * v9[4] + ci2 * v9[5];
-                else
-                    pval = ci0 * v9[0] + ci1 * v9[2] + ci2 * v9[4] + ci0 * v9[1] + ci0 * v9[6] + ci1 * v9[3];
-                gp[0] = pw * (v9[6] + (2.0f * v9[0] + v9[1]));
-                gp[1] = pw * (v9[7] + (2.0f * v9[2] + v9[3]));
-                gp[2] = pw * (v9[8] + (2.0f * v9[4] + v9[5]));
-            }
-            if (with_gradient && !bad) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const double gi = image_from_dense ? a.grad_image[i * 3 + k] : double(cw * -v9[9 + k]);
-                    gt[k] = gi + double(gp[k]);
-                    if (a.grad_image && !image_from_dense) a.grad_image[i * 3 + k] = gi;
-                    if (a.grad_penalty) a.grad_penalty[i * 3 + k] = double(gp[k]);
-                }
-            }
+    // a warp per component of the gradient, one for the penalty's value and
+    // the block's arrival
+    __shared__ __align__(16) double gst[32 * 3];
+    if (w < 3) {
+        if (valid && with_gradient && !bad) {
+            const size_t o = i * 3 + w;
+            const float gp = a.has_penalty ? a.pen_grad_wf * (pacc[0][6 + w][lane] +
+                                                   (2.0f * pacc[0][2 * w][lane] + pacc[0][2 * w + 1][lane]))
+                                           : 0.0f;
+            const double gi = image_from_dense ? a.grad_image[o] : widen(a.cost_wf * -pacc[0][9 + w][lane]);
+            const double gpd = widen(gp), gt = gi + gpd;
+            if (a.params_host) gst[lane * 3 + w] = gt;
+            else a.grad_total[o] = gt;
+            if (a.grad_image && !image_from_dense) a.grad_image[o] = gi;
+            if (a.grad_penalty) a.grad_penalty[o] = gpd;
         }
-        if (with_gradient && !bad && !a.params_host) {
-            if (valid)
+    } else if (w == 3) {
+        float pval = 0.0f;
+        if (valid && a.has_penalty) {
+            float v[7];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) a.grad_total[i * 3 + k] = gt[k];
-        } else if (with_gradient && !bad) {
-            // the total gradient into the caller's host memory: the lanes of
-            // a row (ly, lz) hold four consecutive coefficients, 96
-            // contiguous bytes of the output; a row whose four coefficients
-            // are all in the grid and whose start is 16-byte aligned is
-            // stored as six 16-byte pieces (few large writes over the
-            // CPU-GPU link: an evaluation from host buffers took 153.9
-            // instead of 158.0 us at 192x192x128), any other lane stores
-            // its own three values
-            __shared__ __align__(16) double gst[32 * 3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) gst[lane * 3 + k] = gt[k];
-            __syncwarp();
-            auto row_dst = [&](int r) -> double * {
-                const int ry = cy0 + (r & 3), rz = cz0 + (r >> 2);
-                return a.grad_total + ((size_t(rz) * ncy + ry) * ncx + cx0) * 3;
-            };
-            auto row_vec = [&](int r) -> bool {
-                const int ry = cy0 + (r & 3), rz = cz0 + (r >> 2);
-                return cx0 + GBX <= ncx && ry < ncy && rz < ncz &&
-                       (reinterpret_cast<uintptr_t>(row_dst(r)) & 15u) == 0;
-            };
-            for (int c = lane; c < 48; c += 32) {
-                const int r = c / 6, piece = c - r * 6;
-                if (row_vec(r))
-                    reinterpret_cast<double2 *>(row_dst(r))[piece] =
-                        *reinterpret_cast<const double2 *>(&gst[r * 12 + piece * 2]);
-            }
-            if (valid && !row_vec(lane >> 2))
-#pragma unroll
-                for (int k = 0; k < 3; ++k) a.grad_total[i * 3 + k] = gt[k];
+            for (int k = 0; k < 7; ++k) v[k] = pacc[0][k][lane];
+            if (with_gradient)
+                pval = ci[0] * v[0] + ci[0] * v[1] + ci[1] * v[2] + ci[1] * v[3] + ci[2] * v[4] + ci[2] * v[5];
+            else
+                pval = ci[0] * v[0] + ci[1] * v[2] + ci[2] * v[4] + ci[0] * v[1] + ci[0] * v[6] + ci[1] * v[3];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) pval += __shfl_xor_sync(FULL, pval, o);
         if (lane == 0) {
-            a.pen_part[blk] = double(pval);
-            __threadfence();
-            is_last = (atomicAdd(&a.counters[1], 1u) == unsigned(nblk - 1));
+            a.pen_part[blk] = widen(pval);
+            is_last = arrive_last(&a.counters[1], nblk);
         }
     }
     __syncthreads();
+    if (w == 0 && with_gradient && !bad && a.params_host) {
+        // the total gradient into the caller's host memory: the lanes of
+        // a row (ly, lz) hold four consecutive coefficients, 96
+        // contiguous bytes of the output; a row whose four coefficients
+        // are all in the grid and whose start is 16-byte aligned is
+        // stored as six 16-byte pieces (few large writes over the
+        // CPU-GPU link: an evaluation from host buffers took 153.9
+        // instead of 158.0 us at 192x192x128), any other lane stores
+        // its own three values
+        auto row_dst = [&](int r) -> double * {
+            const int ry = cy0 + (r & 3), rz = cz0 + (r >> 2);
+            return a.grad_total + ((size_t(rz) * ncy + ry) * ncx + cx0) * 3;
+        };
+        auto row_vec = [&](int r) -> bool {
+            const int ry = cy0 + (r & 3), rz = cz0 + (r >> 2);
+            return cx0 + GBX <= ncx && ry < ncy && rz < ncz && (reinterpret_cast<uintptr_t>(row_dst(r)) & 15u) == 0;
+        };
+        for (int c = lane; c < 48; c += 32) {
+            const int r = c / 6, piece = c - r * 6;
+            if (row_vec(r))
+                reinterpret_cast<double2 *>(row_dst(r))[piece] =
+                    *reinterpret_cast<const double2 *>(&gst[r * 12 + piece * 2]);
+        }
+        if (valid && !row_vec(lane >> 2))
+#pragma unroll
+            for (int k = 0; k < 3; ++k) a.grad_total[i * 3 + k] = gst[lane * 3 + k];
+    }
     if (is_last) {
-        __threadfence();
         __shared__ double red[2 * (GT3 / 32)];
-        // v[0]: a deferred SSD cost from the warp kernel's tile sums (the
-        // fixed-order reduction of reduce_tile_sums: same striding, same
-        // tree); v[1]: the blocks' penalty partials; one pass for both
-        const bool fin = a.defer_cost && a.cost == 0;
-        double v2[2] = {0.0, 0.0};
-        if (fin) {
-            const int ntw = a.ax[0].nt * a.ax[1].nt * a.ax[2].nt;
-            v2[0] = strided_sum(a.tile_sums, ntw, tid, GT3, 5);
-        }
-        v2[1] = strided_sum(a.pen_part, nblk, tid, GT3, 1);
-        block_sum<2>(v2, red);
-        if (tid < 32) {
-            if (fin) {
-                const double s5[5] = {v2[0], 0.0, 0.0, 0.0, 0.0};
-                finalise_cost(a, s5, size_t(a.n[0]) * a.n[1] * a.n[2]);
-            }
-        }
-        if (tid == 0) {
-            double *sc = a.scalars;
-            const double pen = a.has_penalty ? v2[1] : 0.0;
-            sc[SC_PEN] = pen;
-            sc[SC_COST_IMG] = a.cost_weight * sc[SC_VALUE];
-            sc[SC_COST_PEN] = a.has_penalty ? a.pen_weight * pen : 0.0;
-            if (a.costs) {
-                a.costs[0] = sc[SC_COST_IMG];
-                a.costs[1] = sc[SC_COST_PEN];
-            }
-            if (a.host_out) {
-                // the costs and both status flags to the caller's host
-                // memory; the non-finite flag is cleared for the next call
-                // (every block has read it before its arrival above)
-                a.host_out[0] = sc[SC_COST_IMG];
-                a.host_out[1] = sc[SC_COST_PEN];
-                unsigned *hf = reinterpret_cast<unsigned *>(a.host_out + 2);
-                hf[0] = *(volatile unsigned *)&a.counters[6];
-                hf[1] = *(volatile unsigned *)&a.counters[7];
-                a.counters[7] = 0;
-            }
-            a.counters[1] = 0;
-        }
+        gather_costs<GT3>(a, X.nt * Y.nt * Z.nt, nblk, false, size_t(a.n[0]) * a.n[1] * a.n[2], red);
     }
 }
 
@@ -1485,7 +1429,7 @@ void launch_warp3(const EvalArgs &a, cudaStream_t st)
     const size_t sm = split3_smem(a, 0);
     with_tz(a.ax[2].t, [&](auto z) { launch_warp3_z<decltype(z)::value>(a, sm, st); });
     count_launch();
-    if (a.defer_cost && a.cost != MGR_COST_SSD) {
+    if (!a.defer_cost || a.cost != MGR_COST_SSD) {
         launch_pdl(a.pdl != 0, k_finalise3, dim3(1), dim3(NT3), 0, st, a);
         count_launch();
     }
