@@ -25,10 +25,13 @@ namespace mgr {
 // the first (x) reads the caller's image (no copy of it is made) and finds
 // its minimum and maximum, the last writes the mirror-padded copy beside the
 // coefficients.  What bounds a pass is the latency of load, recursion and
-// store, one after the other in a block; blocks of 32 lines keep three to
-// five of them on an SM.  New images on a kept level and the evaluation
-// after them, 192x192x128 SSD: 325 us with a kernel each for copy, bounds,
-// means, three passes and padding, 188 us so.
+// store, one after the other in a block, so all its blocks are resident at
+// once (eight of 32 lines on an SM), many loads are in flight and the
+// recursion's loads run ahead of its chain: at 192x192x128 the recursion of a
+// z line took 15.3 k cycles, 8.5 k now.  New images on a kept level and the
+// evaluation after them, 192x192x128 SSD: 325 us with a kernel each for copy,
+// bounds, means, three passes and padding, 180 us in three passes, 165 us so
+// (169 with five blocks an SM, 172 with six, 167 with blocks of 128 threads).
 //
 // The reference filters each line in a double buffer; FP64 arithmetic runs
 // at a small fraction of the FP32 rate on this GPU, so the recursion runs in
@@ -39,6 +42,7 @@ namespace mgr {
 constexpr int PF_NT = 256;
 constexpr int PF_NW = PF_NT / 32;
 constexpr int PF_BATCH = 8;   // line values a thread holds in registers at a time
+constexpr int PF_MINB = 8;    // resident blocks per SM
 
 struct PrefilterPass {
     const float *in;
@@ -71,52 +75,65 @@ __device__ __forceinline__ void prefilter_line(float *c, int n, int s)
     float z2n = powf(p, float(n - 1));
     float sum = c[0] + z2n * c[(n - 1) * s];
     z2n *= z2n * iz;
-    for (int k0 = 1; k0 < n - 1; k0 += PF_BATCH) {
+    // Each of the three walks goes in batches of PF_BATCH values, the next
+    // batch's loads under way while this one's chain of dependent operations
+    // runs: f(x) for each of the `count` values q[0], q[step], ...; store: the
+    // value it returns in their place
+    auto walk = [&](float *q, int step, int count, bool store, auto f, auto done) {
+        if (count >= PF_BATCH) {
+            float v[PF_BATCH];
+#pragma unroll
+            for (int j = 0; j < PF_BATCH; ++j) v[j] = q[j * step];
+#pragma unroll 2
+            for (; count >= 2 * PF_BATCH; count -= PF_BATCH) {
+                float w[PF_BATCH];
+                float *qn = q + PF_BATCH * step;
+#pragma unroll
+                for (int j = 0; j < PF_BATCH; ++j) w[j] = qn[j * step];
+#pragma unroll
+                for (int j = 0; j < PF_BATCH; ++j) v[j] = f(v[j]);
+                if (done()) return;
+#pragma unroll
+                for (int j = 0; j < PF_BATCH; ++j) {
+                    if (store) q[j * step] = v[j];
+                    v[j] = w[j];
+                }
+                q = qn;
+            }
+#pragma unroll
+            for (int j = 0; j < PF_BATCH; ++j) {
+                const float r = f(v[j]);
+                if (store) q[j * step] = r;
+            }
+            count -= PF_BATCH;
+            q += PF_BATCH * step;
+        }
         float v[PF_BATCH];
 #pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 + j < n - 1 ? c[(k0 + j) * s] : 0.0f;
+        for (int j = 0; j < PF_BATCH - 1; ++j) v[j] = j < count ? q[j * step] : 0.0f;
 #pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j)
-            if (k0 + j < n - 1) {
-                sum += (zn + z2n) * v[j];
-                zn *= p;
-                z2n *= iz;
+        for (int j = 0; j < PF_BATCH - 1; ++j)
+            if (j < count) {
+                const float r = f(v[j]);
+                if (store) q[j * step] = r;
             }
-        if (zn == 0.0f && z2n == 0.0f) break;
-    }
-    float prev = sum / (1.0f - zn * zn), before = prev;
+    };
+    auto never = [] { return false; };
+    walk(c + s, s, n - 2, false,
+         [&](float x) {
+             sum += (zn + z2n) * x;
+             zn *= p;
+             z2n *= iz;
+             return x;
+         },
+         [&] { return zn == 0.0f && z2n == 0.0f; });
+    float prev = sum / (1.0f - zn * zn);
     c[0] = prev;
-    for (int k0 = 1; k0 < n; k0 += PF_BATCH) {
-        float v[PF_BATCH];
-#pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 + j < n ? c[(k0 + j) * s] : 0.0f;
-#pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j)
-            if (k0 + j < n) {
-                before = prev;
-                prev = v[j] + p * prev;
-                v[j] = prev;
-            }
-#pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j)
-            if (k0 + j < n) c[(k0 + j) * s] = v[j];
-    }
+    walk(c + s, s, n - 1, true, [&](float x) { return prev = x + p * prev; }, never);
+    const float before = c[max(n - 2, 0) * s];
     float next = (p / (p * p - 1.0f)) * (p * before + prev);
     c[(n - 1) * s] = next;
-    for (int k0 = n - 2; k0 >= 0; k0 -= PF_BATCH) {
-        float v[PF_BATCH];
-#pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 - j >= 0 ? c[(k0 - j) * s] : 0.0f;
-#pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j)
-            if (k0 - j >= 0) {
-                next = p * (next - v[j]);
-                v[j] = next;
-            }
-#pragma unroll
-        for (int j = 0; j < PF_BATCH; ++j)
-            if (k0 - j >= 0) c[(k0 - j) * s] = v[j];
-    }
+    walk(c + (n - 2) * s, -s, n - 1, true, [&](float x) { return next = p * (next - x); }, never);
 }
 
 __device__ __forceinline__ float prefilter_scale(float v)
@@ -127,7 +144,7 @@ __device__ __forceinline__ float prefilter_scale(float v)
 // x lines.  The minimum and maximum follow the reference's rule that the
 // lower clamp bound is at most 0 (interpolator.cxx:109-112); the last block
 // to finish reduces the blocks' values.
-__global__ void __launch_bounds__(PF_NT) k_prefilter_x(PrefilterPass a)
+__global__ void __launch_bounds__(PF_NT, PF_MINB) k_prefilter_x(PrefilterPass a)
 {
     extern __shared__ float sl[];
     __shared__ float2 wmm[PF_NW];
@@ -137,20 +154,27 @@ __global__ void __launch_bounds__(PF_NT) k_prefilter_x(PrefilterPass a)
     const int l0 = blockIdx.x * a.lb, nl = min(a.lb, a.nlines - l0);
     const float *src = a.in + size_t(l0) * n;
     float mn = INFINITY, mx = -INFINITY;
-    for (int l = w; l < nl; l += PF_NW) {
+    // (two lines of a warp at a time: more loads in flight)
+    for (int l = w; l < nl; l += 2 * PF_NW) {
         const float *row = src + size_t(l) * n;
         float *c = sl + l * pitch;
+        const bool two = l + PF_NW < nl;
         for (int k0 = lane; k0 < n; k0 += 32 * PF_BATCH) {
-            float v[PF_BATCH];
+            float v[2][PF_BATCH];
 #pragma unroll
-            for (int j = 0; j < PF_BATCH; ++j) v[j] = k0 + 32 * j < n ? __ldg(row + k0 + 32 * j) : 0.0f;
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < PF_BATCH; ++j)
-                if (k0 + 32 * j < n) {
-                    mn = fminf(mn, v[j]);
-                    mx = fmaxf(mx, v[j]);
-                    c[k0 + 32 * j] = prefilter_scale(v[j]);
-                }
+                for (int j = 0; j < PF_BATCH; ++j)
+                    v[i][j] = k0 + 32 * j < n && (i == 0 || two) ? __ldg(row + size_t(i) * PF_NW * n + k0 + 32 * j) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < PF_BATCH; ++j)
+                    if (k0 + 32 * j < n && (i == 0 || two)) {
+                        mn = fminf(mn, v[i][j]);
+                        mx = fmaxf(mx, v[i][j]);
+                        c[i * PF_NW * pitch + k0 + 32 * j] = prefilter_scale(v[i][j]);
+                    }
         }
     }
 #pragma unroll
@@ -211,7 +235,7 @@ __global__ void __launch_bounds__(PF_NT) k_prefilter_x(PrefilterPass a)
 // line, of the row across the plane's rows (3D) and of the columns within
 // PAD_H of the image's x borders
 template <bool PAD>
-__global__ void __launch_bounds__(PF_NT) k_prefilter_cols(PrefilterPass a)
+__global__ void __launch_bounds__(PF_NT, PF_MINB) k_prefilter_cols(PrefilterPass a)
 {
     extern __shared__ float sl[];
     __shared__ int images[2 * PAD_H + 1];   // PAD, 3D: the padded rows that hold this row
@@ -221,13 +245,13 @@ __global__ void __launch_bounds__(PF_NT) k_prefilter_cols(PrefilterPass a)
     const int l = t & (lb - 1), g = t / lb, ng = PF_NT / lb;
     const size_t base = size_t(blockIdx.y) * a.bstride + xb + l;
     if (l < nl)
-        for (int k0 = g; k0 < n; k0 += ng * PF_BATCH) {
-            float v[PF_BATCH];
+        for (int k0 = g; k0 < n; k0 += ng * 2 * PF_BATCH) {
+            float v[2 * PF_BATCH];
 #pragma unroll
-            for (int j = 0; j < PF_BATCH; ++j)
+            for (int j = 0; j < 2 * PF_BATCH; ++j)
                 v[j] = k0 + ng * j < n ? __ldcg(a.in + base + size_t(k0 + ng * j) * a.estride) : 0.0f;
 #pragma unroll
-            for (int j = 0; j < PF_BATCH; ++j)
+            for (int j = 0; j < 2 * PF_BATCH; ++j)
                 if (k0 + ng * j < n) sl[(k0 + ng * j) * lb + l] = prefilter_scale(v[j]);
         }
     if (PAD && t >= PF_NT - 32) {   // the last warp has no line
@@ -243,19 +267,39 @@ __global__ void __launch_bounds__(PF_NT) k_prefilter_cols(PrefilterPass a)
     __syncthreads();
     if (t < nl) prefilter_line(sl + t, n, lb);
     __syncthreads();
-    if (l < nl) {
+    if (!PAD) {
+        if (l < nl) {
 #pragma unroll 4
-        for (int k = g; k < n; k += ng) a.out[base + size_t(k) * a.estride] = sl[k * lb + l];
-    }
-    if (!PAD) return;
-    const int nimg = nimages, np = n + 2 * PAD_H, nx = a.nlines;
-    if (l < nl)
-#pragma unroll 2
-        for (int kp = g; kp < np; kp += ng) {
-            const float v = sl[mirror_fold(kp - PAD_H, n) * lb + l];
-            float *row = a.pad + size_t(kp) * a.pad_estride + PAD_H + xb + l;
-            for (int r = 0; r < nimg; ++r) row[size_t(images[r]) * a.pad_pitch] = v;
+            for (int k = g; k < n; k += ng) a.out[base + size_t(k) * a.estride] = sl[k * lb + l];
         }
+        return;
+    }
+    const int nimg = nimages, np = n + 2 * PAD_H, nx = a.nlines;
+    if (l < nl) {
+        // the coefficients, and each in the padded row of its own (most rows
+        // have no other image)
+        float *const col = a.pad + PAD_H + xb + l;
+        float *const own = col + size_t(PAD_H) * a.pad_estride + size_t(images[0]) * a.pad_pitch;
+#pragma unroll 4
+        for (int k = g; k < n; k += ng) {
+            const float v = sl[k * lb + l];
+            a.out[base + size_t(k) * a.estride] = v;
+            own[size_t(k) * a.pad_estride] = v;
+        }
+        // the other rows that hold this one
+        if (nimg > 1)
+            for (int k = g; k < n; k += ng) {
+                const float v = sl[k * lb + l];
+                for (int r = 1; r < nimg; ++r)
+                    col[size_t(k + PAD_H) * a.pad_estride + size_t(images[r]) * a.pad_pitch] = v;
+            }
+        // the halo along the line
+        for (int h = g; h < 2 * PAD_H; h += ng) {
+            const int kp = h < PAD_H ? h : n + h;
+            const float v = sl[mirror_fold(kp - PAD_H, n) * lb + l];
+            for (int r = 0; r < nimg; ++r) col[size_t(kp) * a.pad_estride + size_t(images[r]) * a.pad_pitch] = v;
+        }
+    }
     // the x halo's columns whose source lies in this block, and the zeros
     // that fill the padded rows to their pitch (written by the last block)
     const int j = t & 31, w = t >> 5;
