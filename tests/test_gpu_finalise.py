@@ -53,3 +53,27 @@ def test_the_cost_does_not_depend_on_who_finalises_it(size, cost):
     assert fc == ci
     if cost == "ssd":
         assert lv.value(p)[0] == ci
+
+
+@pytest.mark.parametrize("cost", ["ssd", "ncc"])
+@pytest.mark.parametrize("size", [(70, 41), (40, 20, 17)])
+def test_value_from_host_memory(size, cost, monkeypatch):
+    """parameters and costs in the caller's host memory or copied: the same
+    bits; non-finite parameters are refused, the level stays usable"""
+    import mia_gb300 as M
+    from mia_gb300 import _lib
+    lv, mov, ref, p, kw = _level(size, 8.0, cost)
+    monkeypatch.setenv("MGR_HOST_COPY", "1")
+    staged = M.Level(size, **kw)
+    monkeypatch.delenv("MGR_HOST_COPY")
+    staged.set_images(mov, ref)
+    want = staged.value(p)
+    assert lv.value(p) == want
+    for bad in (np.nan, np.inf):
+        q = p.copy()
+        q[-1] = bad
+        for level in (lv, staged):
+            with pytest.raises(_lib.MgrError):
+                level.value(q)
+            assert level.value(p) == want
+    assert lv.evaluate(p)[:2] == staged.evaluate(p)[:2]

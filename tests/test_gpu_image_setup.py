@@ -83,3 +83,10 @@ def test_new_images_on_a_kept_level(size):
     o = O.Level(size, precision=O.PREC_F64, **kw)
     o.set_images(c, d)
     assert abs(got[0] - o.evaluate(p)[0]) <= 1e-5 * abs(got[0])
+
+
+# the recursion walks a line in batches of 8 values
+@pytest.mark.parametrize("size", [(8, 9, 10), (11, 16, 17), (18, 19, 24), (25, 26, 27), (10, 9), (17, 18), (26, 33)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_line_lengths_about_the_batches(size):
+    test_whole_voxel_shifts(size)
