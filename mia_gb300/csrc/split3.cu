@@ -19,7 +19,8 @@
 //       gather costs shared-memory wavefronts instead of L1 lines; each
 //       thread samples two planes per step (two independent tap chains in
 //       flight); the warped image is written and the SSD / NCC sums are
-//       accumulated; the last block finalises the cost.
+//       accumulated (finalised after the kernel, a batch of NCC pairs by the
+//       last block).
 //   k_adjoint3<TZ>    central differences of the warped image (x and y
 //       neighbours from a ring of planes in shared memory, z neighbours
 //       carried in registers; mia/3d/image.cc:347-466), the SSD /
