@@ -568,17 +568,21 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         qgrid[0] = std::min(int(titems.size()), split3_queue_grid(cost, 0, sm_warp));
         qgrid[1] = std::min(int(titems.size()), split3_queue_grid(cost, 1, sm_adj));
     }
+    // 3D NCC: the force constants between the warp and adjoint kernels
+    const bool fin = dim == 3 && cost != MGR_COST_SSD;
     auto step = [&]() {
         launch_pdl(pdl, k_min_propose, mgrid, dim3(MT), 0, st, d_states, d_vecs, mz, d_active, msc);
         if (queue) {
             launch_split3_queue(cost, d_args, d_titems, int(titems.size()), d_active, d_queue, qgrid[0], sm_warp,
                                 0, pdl, st);
+            if (fin) launch_finalise3_batch(d_args, np, d_active, pdl, st);
             launch_split3_queue(cost, d_args, d_titems, int(titems.size()), d_active, d_queue + 2, qgrid[1], sm_adj,
                                 1, pdl, st);
         } else {
             if (!launch_split_batch(dim, cost, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
                                     d_active, sm_warp, 0, pdl, st))
                 throw std::invalid_argument("tile shape not compiled in");
+            if (fin) launch_finalise3_batch(d_args, np, d_active, pdl, st);
             launch_split_batch(dim, cost, tile[0], tile[1], tile[2], d_args, d_titems, int(titems.size()),
                                d_active, sm_adj, 1, pdl, st);
         }
@@ -591,7 +595,7 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     // kernel attributes are set outside the capture
     prepare_split_batch(dim, cost, tile[0], tile[1], tile[2], sm_warp, sm_adj);
     cudaGraphExec_t exec = nullptr;
-    const unsigned kernels_per_chunk = unsigned(chunk) * 5 + 1;
+    const unsigned kernels_per_chunk = unsigned(chunk) * (fin ? 6 : 5) + 1;
     tr_setup.stop();
     if (use_graphs) {
         TraceScope tr("batch: graph capture", st);

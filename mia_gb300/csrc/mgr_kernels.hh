@@ -108,9 +108,8 @@ struct EvalArgs {
     // (the warp blocks then end without a device-wide fence and last-block
     // reduction): an SSD cost by the gather's last block (the adjoint takes
     // its force scale from the settings), an NCC cost by k_finalise3, which
-    // launch_warp3 queues right after the warp kernel (2D: SSD only); 0: the
-    // warp kernel's last block finalises the cost (3D: only a batch's NCC
-    // kernel can, a single evaluation's is followed by k_finalise3)
+    // launch_warp3 queues right after the warp kernel (2D: SSD only); 0: 2D,
+    // the warp kernel's last block finalises the cost, 3D, k_finalise3
     int defer_cost;
     // 1: the split path's adjoint and gather kernels (3D: the warp kernel,
     // too) are launched with programmatic stream serialisation (each may start while the one
@@ -165,6 +164,8 @@ void launch_gather3(const EvalArgs &a, int with_gradient, int dense, cudaStream_
 void prepare_split3_batch(int cost, size_t sm_warp, size_t sm_adj);
 void launch_split3_batch(int cost, const EvalArgs *args, const int2 *items, int nitems, const int *active, size_t sm,
                          int which, bool pdl, cudaStream_t st);
+// NCC: the pairs' costs after a batch's warp kernel
+void launch_finalise3_batch(const EvalArgs *args, int npairs, const int *active, bool pdl, cudaStream_t st);
 void launch_gather3_batch(const EvalArgs *args, const int2 *items, int nitems, const int *active, const int *nblocks,
                           bool pdl, cudaStream_t st);
 

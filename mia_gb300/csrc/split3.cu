@@ -19,8 +19,7 @@
 //       gather costs shared-memory wavefronts instead of L1 lines; each
 //       thread samples two planes per step (two independent tap chains in
 //       flight); the warped image is written and the SSD / NCC sums are
-//       accumulated (finalised after the kernel, a batch of NCC pairs by the
-//       last block).
+//       accumulated (the cost is finalised after the kernel).
 //   k_adjoint3<TZ>    central differences of the warped image (x and y
 //       neighbours from a ring of planes in shared memory, z neighbours
 //       carried in registers; mia/3d/image.cc:347-466), the SSD /
@@ -100,7 +99,7 @@ constexpr unsigned FULL = 0xffffffffu;
 // the SSD sum, every other one unrounded: the sums differ in the last bits,
 // and a batch's line searches would take other steps
 template <int TZ, int COST, bool BATCH>
-__device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, int bz, int ntiles, int tile)
+__device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, int bz, int tile)
 {
     constexpr int NW = NT3 / 32;
     constexpr int NPAIR = RING_N / 2;                      // the ring's slots are filled in pairs of planes
@@ -110,7 +109,6 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
     // [RING_N][RING_Y][RING_X] ring (the tensor copies want a 128-byte
     // aligned destination), then C and Tx
     extern __shared__ __align__(128) float sm3[];
-    __shared__ double red[5 * NW];
     __shared__ float wsum[5][NW];
     __shared__ float csc[2];   // NCC centres (converted once per block)
     __shared__ int zs[TZ];
@@ -121,7 +119,6 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
     __shared__ unsigned rdone[NPAIR];     // warps done with the slots' current planes
     __shared__ int nissued;               // pairs of planes whose copies were issued
     __shared__ volatile int ring_failed;  // a wait of this block gave up
-    __shared__ bool is_last;
     const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
     const int nx = a.n[0], ny = a.n[1], nz = a.n[2];
     const int x0 = bx * TX3, y0 = by * TY3, z0 = bz * TZ;
@@ -561,17 +558,9 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             for (int w = 0; w < NW; ++w) v += widen(wsum[tid][w]);
         a.tile_sums[size_t(tile) * 5 + tid] = v;
     }
-    // SSD costs are finalised by the gather, a single evaluation's NCC cost by
-    // k_finalise3: only a batch's NCC kernel has a last-block pass (its code
-    // alone costs the others 1 %: 383x351x317 SSD 662 -> 654 us)
-    if (!BATCH || COST == MGR_COST_SSD) return;
-    __syncthreads();
-    if (tid == 0) is_last = arrive_last(&a.counters[0], ntiles);
-    __syncthreads();
-    if (is_last) {
-        reduce_tile_sums(a, ntiles, size_t(nx) * ny * nz, red);
-        if (tid == 0) a.counters[0] = 0;
-    }
+    // (the cost is finalised from the tile sums after this kernel: an SSD cost
+    // by the gather, an NCC cost by k_finalise3; a last-block pass here, even
+    // one that is not taken, cost 383x351x317 SSD 662 instead of 654 us)
 }
 
 // ---------------------------------------------------------------------
@@ -1167,7 +1156,7 @@ template <int TZ, int COST>
 __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3(const __grid_constant__ EvalArgs a)
 {
     const int tile = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    warp3_body<TZ, COST, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x * gridDim.y * gridDim.z, tile);
+    warp3_body<TZ, COST, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, tile);
 }
 
 template <int TZ>
@@ -1183,9 +1172,8 @@ __global__ void MGR_GATHER_BOUNDS k_gather3(EvalArgs a, int with_gradient, int i
 }
 
 // The NCC cost and force constants from the warp kernel's tile sums, one
-// block of NT3 threads: the reduction the warp kernel's last block makes
-// otherwise (same striding, same order), so that the warp blocks end
-// without a device-wide fence.  The adjoint kernel after it reads the
+// block of NT3 threads, so that the warp blocks end without a device-wide
+// fence.  The adjoint kernel after it reads the
 // constants.
 __global__ void __launch_bounds__(NT3) k_finalise3(EvalArgs a)
 {
@@ -1195,13 +1183,24 @@ __global__ void __launch_bounds__(NT3) k_finalise3(EvalArgs a)
     reduce_tile_sums(a, a.ax[0].nt * a.ax[1].nt * a.ax[2].nt, size_t(a.n[0]) * a.n[1] * a.n[2], red);
 }
 
-__device__ __forceinline__ void decode_tile3(const EvalArgs &a, int t, int &bx, int &by, int &bz, int &nt)
+// the same for every running pair of a batch, a block each
+__global__ void __launch_bounds__(NT3) k_finalise3_batch(const EvalArgs *__restrict__ args,
+                                                         const int *__restrict__ active)
 {
-    const int ntx = a.ax[0].nt, nty = a.ax[1].nt, ntz = a.ax[2].nt;
+    __shared__ double red[5 * (NT3 / 32)];
+    pdl_wait();
+    pdl_trigger();
+    if (!active[blockIdx.x]) return;
+    const EvalArgs &a = args[blockIdx.x];
+    reduce_tile_sums(a, a.ax[0].nt * a.ax[1].nt * a.ax[2].nt, size_t(a.n[0]) * a.n[1] * a.n[2], red);
+}
+
+__device__ __forceinline__ void decode_tile3(const EvalArgs &a, int t, int &bx, int &by, int &bz)
+{
+    const int ntx = a.ax[0].nt, nty = a.ax[1].nt;
     bx = t % ntx;
     by = (t / ntx) % nty;
     bz = t / (ntx * nty);
-    nt = ntx * nty * ntz;
 }
 
 template <int TZ, int COST>
@@ -1213,9 +1212,9 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_batch(const EvalAr
     pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     const EvalArgs &a = args[it.x];
-    int bx, by, bz, nt;
-    decode_tile3(a, it.y, bx, by, bz, nt);
-    warp3_body<TZ, COST, true>(a, bx, by, bz, nt, it.y);
+    int bx, by, bz;
+    decode_tile3(a, it.y, bx, by, bz);
+    warp3_body<TZ, COST, true>(a, bx, by, bz, it.y);
 }
 
 template <int TZ>
@@ -1226,8 +1225,8 @@ __global__ void MGR_ADJ_BOUNDS k_adjoint3_batch(const EvalArgs *__restrict__ arg
     pdl_wait();   // the minimizer sets the flags
     if (!active[it.x]) return;
     const EvalArgs &a = args[it.x];
-    int bx, by, bz, nt;
-    decode_tile3(a, it.y, bx, by, bz, nt);
+    int bx, by, bz;
+    decode_tile3(a, it.y, bx, by, bz);
     adjoint3_body<TZ>(a, bx, by, bz, it.y);
 }
 
@@ -1271,9 +1270,9 @@ __global__ void __launch_bounds__(NT3, MGR_WARP_MINB) k_warp3_queue(const EvalAr
     while (next_item(queue, nitems, items, it, slot)) {
         if (!active[it.x]) continue;
         const EvalArgs &a = args[it.x];
-        int bx, by, bz, nt;
-        decode_tile3(a, it.y, bx, by, bz, nt);
-        warp3_body<TZ, COST, true>(a, bx, by, bz, nt, it.y);
+        int bx, by, bz;
+        decode_tile3(a, it.y, bx, by, bz);
+        warp3_body<TZ, COST, true>(a, bx, by, bz, it.y);
     }
     queue_done(queue);
 }
@@ -1290,8 +1289,8 @@ __global__ void MGR_ADJ_BOUNDS k_adjoint3_queue(const EvalArgs *__restrict__ arg
     while (next_item(queue, nitems, items, it, slot)) {
         if (!active[it.x]) continue;
         const EvalArgs &a = args[it.x];
-        int bx, by, bz, nt;
-        decode_tile3(a, it.y, bx, by, bz, nt);
+        int bx, by, bz;
+        decode_tile3(a, it.y, bx, by, bz);
         adjoint3_body<TZ>(a, bx, by, bz, it.y);
     }
     queue_done(queue);
@@ -1507,6 +1506,12 @@ void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int 
         launch_pdl(pdl, warp3_queue_kernel(cost), dim3(grid), dim3(NT3), sm, st, args, items, nitems, active, queue);
     else
         launch_pdl(pdl, k_adjoint3_queue<BATCH_TZ>, dim3(grid), dim3(AT3), sm, st, args, items, nitems, active, queue);
+    count_launch();
+}
+
+void launch_finalise3_batch(const EvalArgs *args, int npairs, const int *active, bool pdl, cudaStream_t st)
+{
+    launch_pdl(pdl, k_finalise3_batch, dim3(npairs), dim3(NT3), 0, st, args, active);
     count_launch();
 }
 
