@@ -112,7 +112,7 @@ void alloc_together(DevBuf<unsigned char> &slab, cudaStream_t s, Each each)
 // host blob and uploaded with one copy; `off` are byte offsets into it
 struct AxisDev {
     AxisHost h;
-    size_t off[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};   // fs, as, rows, ftile0, atile0, gtile, fw, aw, glist, glen
+    size_t off[11] = {};   // fs, as, rows, ftile0, atile0, gtile, fw, aw, glist, glen, win
     const unsigned char *base = nullptr;
 
     template <class T>
@@ -135,6 +135,7 @@ struct AxisDev {
         off[7] = pack(blob, h.aw);
         off[8] = pack(blob, h.glist);
         off[9] = pack(blob, h.glen);
+        off[10] = pack(blob, h.win);
     }
     Axis view() const
     {
@@ -149,6 +150,7 @@ struct AxisDev {
         a.aw = reinterpret_cast<const float4 *>(base + off[7]);
         a.glist = reinterpret_cast<const int *>(base + off[8]);
         a.glen = reinterpret_cast<const int *>(base + off[9]);
+        a.win = reinterpret_cast<const int2 *>(base + off[10]);
         a.n = h.n;
         a.nc = h.nc;
         a.t = h.t;

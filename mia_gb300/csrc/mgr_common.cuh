@@ -374,6 +374,7 @@ struct Axis {
     const int2 *gtile;  // per coefficient: tiles [lo, hi] whose adjoint footprint holds it
     const int *glist;   // per coefficient: GATHER_LMAX offsets into the partial slots, this axis' part
     const int *glen;    // per coefficient: entries of glist (-1: longer than GATHER_LMAX)
+    const int2 *win;    // per coefficient: voxels [lo, hi) whose four adjoint coefficients include it
     int n;              // voxels
     int nc;             // coefficients
     int t;              // tile length (voxels)

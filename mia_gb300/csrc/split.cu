@@ -261,20 +261,12 @@ __device__ __forceinline__ void adjoint2_body(const EvalArgs &a, int bx, int by,
         if ((e & 3) == 0) asy[e / 4] = Y.as[yc] - ay0;
     }
     // the tile's voxels whose four coefficients include one (none beyond the
-    // grid): those that it has a weight for, and the voxel before them if the
-    // last of its four is this one with weight 0 (an infinite force is felt
-    // there all the same)
+    // grid)
     for (int o = tid; o < AXc + AYc; o += NT) {
         const bool isx = o < AXc;
         const Axis &A = isx ? X : Y;
         const int c = isx ? ax0 + o : ay0 + o - AXc, v0 = isx ? x0 : y0, e = isx ? ex : ey;
-        int2 r = make_int2(0, 0);
-        if (c < A.nc) {
-            r = A.rows[c];
-            const int n = isx ? nx : ny;
-            r = r.y > 0 ? make_int2(r.x, r.x + r.y) : make_int2(n, n);
-            if (r.x > 0 && A.as[r.x - 1] + 3 >= c) --r.x;
-        }
+        const int2 r = c < A.nc ? A.win[c] : make_int2(0, 0);
         rx[o] = make_int2(max(r.x - v0, 0), min(r.y - v0, e));
     }
     const int xx = tid % TX, yy0 = tid / TX;

@@ -126,6 +126,17 @@ void build_axis(AxisHost &ax, int n, int nc, int tile)
             ax.aw[size_t(i) * 4 + k] = p.second;
         }
     }
+    // The voxels that a coefficient gets a sum from: those whose window of
+    // four holds it, the weights of 0 included (an infinite force is felt
+    // there all the same).  Starts do not decrease, so they are one range,
+    // empty where the grid is so fine that windows leave coefficients out.
+    ax.win.assign(size_t(nc) * 2, 0);
+    for (int o = 0, lo = 0, hi = 0; o < nc; ++o) {
+        while (lo < n && ax.as[lo] + 3 < o) ++lo;
+        while (hi < n && ax.as[hi] <= o) ++hi;
+        ax.win[size_t(o) * 2] = lo;
+        ax.win[size_t(o) * 2 + 1] = std::max(lo, hi);
+    }
     // tile footprints
     ax.ftile0.resize(ax.nt);
     ax.atile0.resize(ax.nt);

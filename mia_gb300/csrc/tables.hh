@@ -14,6 +14,7 @@ struct AxisHost {
     std::vector<int> as;       // n
     std::vector<float> aw;     // n x 4
     std::vector<int> rows;     // nc x (first, len)
+    std::vector<int> win;      // nc x (lo, hi): the voxels lo <= i < hi whose window as[i] .. as[i] + 3 holds it
     std::vector<int> ftile0;   // nt
     std::vector<int> atile0;   // nt
     std::vector<int> gtile;    // nc x (lo, hi)

@@ -131,3 +131,25 @@ def test_an_infinite_force_reaches_the_four_coefficients_of_each_axis(at):
         lv.set_path("split", tile)
         g = np.asarray(lv.evaluate(p)[2]).reshape(ncy, ncx, 2)
         np.testing.assert_array_equal(~np.isfinite(g).all(axis=2), want, err_msg=str(tile))
+
+
+# grids with several coefficients per voxel, up to windows of four that leave
+# coefficients out between them (five per voxel)
+@pytest.mark.parametrize("cost", ["ssd", "ncc"])
+@pytest.mark.parametrize("size,csize", [((8, 16), (40, 80)), ((9, 7), (45, 10)), ((33, 20), (110, 62)),
+                                        ((40, 33), (163, 130))])
+def test_grids_finer_than_the_voxels(size, csize, cost):
+    import mia_gb300 as M
+    from mia_gb300 import synth
+    from oracle import oracle as O
+    kw = dict(csize=csize, cost=cost)
+    lv, o = M.Level(size, **kw), O.Level(size, precision=O.PREC_F64, **kw)
+    mov, ref = _pair(size, 3)
+    lv.set_images(mov, ref)
+    o.set_images(mov, ref)
+    p = synth.smooth_params(lv.csize, 1.0, seed=7)
+    oi, _, ogi, _ = o.evaluate(p)
+    for tile in TILES:
+        lv.set_path("split", tile)
+        ci, _, gi, _, _ = lv.evaluate(p)
+        assert abs(ci - oi) <= 1e-5 * abs(oi) and _rel(gi, ogi) < 1e-4, tile
