@@ -187,23 +187,20 @@ namespace mgr {
 // A new coefficient grid on a level whose images stay (the second pass of a
 // registration level after refine): parameter buffers, tables and penalty
 // are rebuilt, the prefiltered images are kept.  All work is queued on the
-// level's stream.
+// level's stream.  A failure leaves the level as it was.
 void level_set_grid(mgr_level *L, const int csize[3], const int tile[3])
 {
     ck(cudaSetDevice(L->device), "cudaSetDevice");   // (callers may be helper threads)
     const int D = L->d.dim;
+    int g[3] = {1, 1, 1};
     for (int k = 0; k < D; ++k) {
         if (csize[k] <= 3) throw std::invalid_argument("coefficient grid must be larger than 3 per axis");
-        L->nc[k] = csize[k];
-        L->d.csize[k] = csize[k];
+        g[k] = csize[k];
     }
-    L->ncoef = size_t(L->nc[0]) * L->nc[1] * L->nc[2];
-    L->nparams = L->ncoef * D;
-    for (int k = 0; k < 3; ++k) L->tile[k] = tile[k];
+    L->reshape(g, tile, L->path);
+    for (int k = 0; k < D; ++k) L->d.csize[k] = g[k];
     L->grad_image.release();
     L->grad_penalty.release();
-    L->build_penalty();
-    L->build_tables();
     check_launch("level set grid");
 }
 mgr_level *level_create_on_images(const mgr_level *S, const int csize[3], cudaStream_t st)
@@ -222,8 +219,6 @@ mgr_level *level_create_on_images(const mgr_level *S, const int csize[3], cudaSt
         L->tile[k] = S->tile[k];
     }
     L->N = S->N;
-    L->ncoef = size_t(L->nc[0]) * L->nc[1] * L->nc[2];
-    L->nparams = L->ncoef * D;
     L->path = S->path;
     L->device = S->device;
     L->coherent = S->coherent;
@@ -232,8 +227,7 @@ mgr_level *level_create_on_images(const mgr_level *S, const int csize[3], cudaSt
     L->images_from = S;
     L->images_set = true;
     L->alloc_state();
-    L->build_penalty();
-    L->build_tables();
+    L->reshape(L->nc, L->tile, L->path);
     check_launch("level create on images");
     return L.release();
 }
@@ -292,12 +286,10 @@ mgr_status mgr::level_create(const mgr_level_desc *desc, int device, void *strea
             }
         }
         L->N = size_t(L->n[0]) * L->n[1] * L->n[2];
-        L->ncoef = size_t(L->nc[0]) * L->nc[1] * L->nc[2];
-        L->nparams = L->ncoef * d.dim;
-        if (tile && L->tile_fits(tile, false))
+        if (tile && L->tile_fits(L->nc, tile, false))
             for (int k = 0; k < 3; ++k) L->tile[k] = tile[k];
         else
-            L->choose_tile();
+            L->choose_tile(L->nc, L->tile);
         L->device = device;
         ck(cudaSetDevice(device), "cudaSetDevice");
         configure_pool(device);
@@ -323,8 +315,7 @@ mgr_status mgr::level_create(const mgr_level_desc *desc, int device, void *strea
         });
         if (d.dim == 3) L->has_tmap = encode_pad_tmap(&L->tmap, L->coef_pad.p, L->n[0], L->n[1], L->n[2]);
         L->alloc_state();
-        L->build_penalty();
-        L->build_tables();
+        L->reshape(L->nc, L->tile, L->path);
         check_launch("level create");
     });
     if (st == MGR_OK) *out = L.release();
@@ -720,9 +711,9 @@ mgr_status mgr_level_set_grid(mgr_level *lvl, const int csize[3])
         }
         if (same) return;
         // the tile follows the new coefficient spacing as at creation
-        for (int k = 0; k < D; ++k) lvl->nc[k] = cs[k];
-        lvl->choose_tile();
-        level_set_grid(lvl, cs, lvl->tile);
+        int t[3];
+        lvl->choose_tile(cs, t);
+        level_set_grid(lvl, cs, t);
         ck(cudaStreamSynchronize(lvl->stream), "set_grid sync");
     });
 }
@@ -750,21 +741,16 @@ mgr_status mgr_level_set_path(mgr_level *lvl, int path, int tile_x, int tile_y, 
         if (!tile_supported(lvl->d.dim, t[0], t[1], t[2]))
             throw std::invalid_argument("tile shape not compiled in (3D: 32x8xTZ, TZ in 4, 8, 12, 16, 20, 24, 32; "
                                         "2D: 32x8, 32x16, 64x8, 64x16, 32x32)");
-        if (!lvl->tile_fits(t, false))
+        if (!lvl->tile_fits(lvl->nc, t, false))
             throw std::invalid_argument("the tile's shared memory does not fit at this coefficient spacing");
-        const bool fused_change = (path == MGR_PATH_FUSED) != (lvl->path == MGR_PATH_FUSED);
-        lvl->path = path;
-        bool changed = fused_change;
-        for (int k = 0; k < 3; ++k)
-            if (t[k] != lvl->tile[k]) {
-                lvl->tile[k] = t[k];
-                changed = true;
-            }
+        bool changed = (path == MGR_PATH_FUSED) != (lvl->path == MGR_PATH_FUSED);
+        for (int k = 0; k < 3; ++k) changed = changed || t[k] != lvl->tile[k];
         if (changed) {
             ck(cudaStreamSynchronize(lvl->stream), "sync");
-            lvl->build_tables();
+            lvl->reshape(lvl->nc, t, path);
             ck(cudaStreamSynchronize(lvl->stream), "sync");
         }
+        lvl->path = path;
         if (path == MGR_PATH_FUSED && fused3_smem(lvl->args(true)) > size_t(227) * 1024) {
             lvl->path = MGR_PATH_SPLIT;
             throw std::invalid_argument("the fused kernel's shared memory does not fit at this coefficient spacing");

@@ -10,6 +10,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/mgr.h"
@@ -72,6 +73,13 @@ struct DevBuf {
         n = count;
         own = false;
     }
+    void swap(DevBuf &o) noexcept
+    {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+        std::swap(st, o.st);
+        std::swap(own, o.own);
+    }
     void alloc(size_t count, cudaStream_t s)
     {
         if (count <= n && p) return;
@@ -91,14 +99,14 @@ struct DevBuf {
 // The buffers that `each` lists (each(f) calls f(buffer, count) for all of
 // them) in one allocation: a level has about twenty, and the cost of a
 // stream-ordered allocation grows with the blocks that the pool holds and the
-// streams they were freed on.
+// streams they were freed on.  The slab is a fresh one: buffers that borrow
+// from another slab keep it until this one has its memory.
 template <class Each>
 void alloc_together(DevBuf<unsigned char> &slab, cudaStream_t s, Each each)
 {
     auto bytes = [](auto &b, size_t count) { return (count * sizeof(*b.p) + 255) & ~size_t(255); };
     size_t total = 0;
     each([&](auto &b, size_t count) { total += bytes(b, count); });
-    slab.release();
     slab.alloc(total, s);
     size_t at = 0;
     each([&](auto &b, size_t count) {
@@ -197,7 +205,6 @@ struct mgr_level {
     bool has_tmap = false;
     int slot = 0;
     bool images_set = false;
-    bool tables_valid = false;
     bool timing = false;
     // 1: events around every kernel (launched one after another); 2: events
     // around the whole evaluation only (kernels overlap as in untimed runs)
@@ -310,17 +317,17 @@ struct mgr_level {
     }
 
     // whether tile t is compiled in and, in 3D, its blocks' shared memory
-    // fits: `strict`, the warp block three to an SM and the adjoint block in
+    // fits on a grid of g coefficients: `strict`, the warp block three to an SM and the adjoint block in
     // 64 KiB (the rule without measurements); else what a launch allows
     // (the autotuner measured the shape, occupancy included)
-    bool tile_fits(const int t[3], bool strict = true) const
+    bool tile_fits(const int g[3], const int t[3], bool strict = true) const
     {
         if (!tile_supported(d.dim, t[0], t[1], t[2])) return false;
         if (d.dim == 2) return true;
         AxisHost hx, hy, hz;
-        build_axis(hx, n[0], nc[0], t[0]);
-        build_axis(hy, n[1], nc[1], t[1]);
-        build_axis(hz, n[2], nc[2], t[2]);
+        build_axis(hx, n[0], g[0], t[0]);
+        build_axis(hy, n[1], g[1], t[1]);
+        build_axis(hz, n[2], g[2], t[2]);
         const size_t w =
             (size_t(3) * hz.fc * hy.fc * (hx.fc + 32) + 32 + size_t(WARP_RING_PLANES) * 16 * 64) * sizeof(float);
         // (split3_smem(a, 1) but for the adjoint's ring, which takes at most
@@ -330,37 +337,32 @@ struct mgr_level {
         return w + 128 <= 200 * 1024 && adj <= 200 * 1024;
     }
 
-    // the tile of the autotuner's nearest case (tune.cc) when a launch
-    // allows it, else 32x16 in 2D and in 3D the deepest z tile (16, 8, 4)
-    // that fits three warp blocks to an SM
-    void choose_tile()
+    // the tile for a grid of g coefficients into t: that of the autotuner's
+    // nearest case (tune.cc) when a launch allows it, else 32x16 in 2D and in
+    // 3D the deepest z tile (16, 8, 4) that fits three warp blocks to an SM
+    void choose_tile(const int g[3], int t[3]) const
     {
-        int t[3];
-        if (tuned_tile(d.dim, n, nc, t) && tile_fits(t, false)) {
-            for (int k = 0; k < 3; ++k) tile[k] = t[k];
-            return;
-        }
-        if (d.dim == 2) {
-            tile[0] = 32;
-            tile[1] = 16;
-            tile[2] = 1;
-            return;
-        }
+        if (tuned_tile(d.dim, n, g, t) && tile_fits(g, t, false)) return;
+        t[0] = 32;
+        t[1] = d.dim == 3 ? 8 : 16;
+        t[2] = 1;
+        if (d.dim == 2) return;
         static const int tzs[3] = {16, 8, 4};
-        for (int k = 0; k < 3; ++k) {
-            const int c[3] = {32, 8, tzs[k]};
-            for (int j = 0; j < 3; ++j) tile[j] = c[j];
-            if (tile_fits(c)) return;
+        for (int z : tzs) {
+            t[2] = z;
+            if (tile_fits(g, t)) return;
         }
     }
 
-    // the per-axis tables of tiles t into A, packed at the end of blob;
-    // returns the number of tiles and sets the partial slot size
-    int build_axis_set(const int t[3], AxisDev (&A)[3], std::vector<unsigned char> &blob, int &slot_size) const
+    // the per-axis tables of tiles t on a grid of g coefficients into A,
+    // packed at the end of blob; returns the number of tiles and sets the
+    // partial slot size
+    int build_axis_set(const int g[3], const int t[3], AxisDev (&A)[3], std::vector<unsigned char> &blob,
+                       int &slot_size) const
     {
         const int D = d.dim;
         AxisDev *ax = A;
-        for (int k = 0; k < D; ++k) build_axis(ax[k].h, n[k], nc[k], t[k]);
+        for (int k = 0; k < D; ++k) build_axis(ax[k].h, n[k], g[k], t[k]);
         {
             // per axis and coefficient: the partial-slot offset parts of the
             // tiles that hold it, slot entry (tx, ty[, tz]) of coefficient
@@ -390,76 +392,100 @@ struct mgr_level {
         return ax[0].h.nt * ax[1].h.nt * (D == 3 ? ax[2].h.nt : 1);
     }
 
-    // the fused kernel's tile: 30 interior voxels in x (32 lanes with the
-    // halo), 8 rows, the level's z tile
-    void fused_tile(int t[3]) const
+    // Moves the level to a grid of g coefficients, the split path's tile t and
+    // a path: the tables (with the penalty's, one upload), the parameter and
+    // gradient buffers and the partials.  All that can fail comes first and
+    // leaves the level as it was; then the new state takes the old one's
+    // place.  It is a fresh allocation: kernels queued earlier may still read
+    // the old one, which is freed in stream order.
+    void reshape(const int g[3], const int t[3], int new_path)
     {
-        t[0] = 30;
-        t[1] = 8;
-        t[2] = tile[2];
-    }
-
-    // the penalty's cells of the grid on the host (3D: translation-invariant;
-    // 2D: boundary-clipped CSR rows, cached across levels of equal grid)
-    void build_penalty()
-    {
-        if (!d.has_penalty) return;
-        const float range[3] = {float(d.size[0]), float(d.size[1]), float(d.dim == 3 ? d.size[2] : 1)};
-        if (d.dim == 3) ptable_host = build_penalty3(nc, range, d.pen_div, d.pen_curl);
-        else penalty2_host = penalty2_cached(nc, range, d.pen_div, d.pen_curl);
-    }
-
-    // Everything that depends on the coefficient grid and the tile: the
-    // tables (with the penalty's, one upload), the parameter and gradient
-    // buffers, the partials.  In a fresh allocation: kernels queued earlier
-    // may still read the old one, which is freed in stream order.
-    void build_tables()
-    {
-        std::vector<unsigned char> blob;
-        const int ntiles = build_axis_set(tile, ax, blob, slot);
-        size_t part = size_t(ntiles) * slot, sums = size_t(ntiles);
-        if (path == MGR_PATH_FUSED) {
-            std::vector<unsigned char> blob_f;
-            int t[3];
-            fused_tile(t);
-            const int ntf = build_axis_set(t, axf, blob_f, slot_f);
-            part = std::max(part, size_t(ntf) * slot_f);
+        const int D = d.dim;
+        AxisDev A[3], AF[3];
+        std::vector<unsigned char> blob, blob_f;
+        int sl = 0, sl_f = 0;
+        const int ntiles = build_axis_set(g, t, A, blob, sl);
+        size_t part = size_t(ntiles) * sl, sums = size_t(ntiles);
+        if (new_path == MGR_PATH_FUSED) {
+            // the fused kernel's tile: 30 interior voxels in x (32 lanes with
+            // the halo), 8 rows, the level's z tile
+            const int tf[3] = {30, 8, t[2]};
+            const int ntf = build_axis_set(g, tf, AF, blob_f, sl_f);
+            part = std::max(part, size_t(ntf) * sl_f);
             sums = std::max(sums, size_t(ntf));
-            axis_tables_f.release();
-            axis_tables_f.upload(blob_f, stream);
-            for (int k = 0; k < d.dim; ++k) axf[k].base = axis_tables_f.p;
         }
+        // the penalty's cells (3D: translation-invariant; 2D:
+        // boundary-clipped CSR rows, cached across levels of equal grid)
+        const bool new_grid = !slab_grid.p || g[0] != nc[0] || g[1] != nc[1] || g[2] != nc[2];
+        std::vector<float> cells3;
+        std::shared_ptr<const Penalty2Table> cells2 = penalty2_host;
+        if (d.has_penalty && new_grid) {
+            const float range[3] = {float(d.size[0]), float(d.size[1]), float(D == 3 ? d.size[2] : 1)};
+            if (D == 3) cells3 = build_penalty3(g, range, d.pen_div, d.pen_curl);
+            else cells2 = penalty2_cached(g, range, d.pen_div, d.pen_curl);
+        }
+        const std::vector<float> &p3 = new_grid ? cells3 : ptable_host;
         size_t at_pen[3] = {0, 0, 0};
-        if (d.has_penalty && d.dim == 3) {
-            at_pen[0] = AxisDev::pack(blob, ptable_host);
+        if (d.has_penalty && D == 3) {
+            at_pen[0] = AxisDev::pack(blob, p3);
         } else if (d.has_penalty) {
-            at_pen[0] = AxisDev::pack(blob, penalty2_host->rowptr);
-            at_pen[1] = AxisDev::pack(blob, penalty2_host->col);
-            at_pen[2] = AxisDev::pack(blob, penalty2_host->val);
+            at_pen[0] = AxisDev::pack(blob, cells2->rowptr);
+            at_pen[1] = AxisDev::pack(blob, cells2->col);
+            at_pen[2] = AxisDev::pack(blob, cells2->val);
         }
         EvalArgs sizes{};   // what the counts below depend on
-        sizes.dim = d.dim;
-        for (int k = 0; k < 3; ++k) sizes.nc[k] = nc[k];
-        const size_t plain_blocks = (N + 255) / 256;
-        alloc_together(slab_grid, stream, [&](auto buf) {
-            buf(params, nparams);
-            buf(params_f, nparams);
-            buf(grad_total, nparams);
-            buf(axis_tables, blob.size());
-            buf(partial, part);
-            buf(tile_sums, std::max<size_t>(sums, plain_blocks) * 5);
-            buf(pen_part, size_t(gather_blocks(sizes)) + 1);
+        sizes.dim = D;
+        for (int k = 0; k < 3; ++k) sizes.nc[k] = g[k];
+        const size_t ncoefs = size_t(g[0]) * g[1] * g[2], np = ncoefs * D, plain_blocks = (N + 255) / 256;
+        struct {
+            DevBuf<unsigned char> slab, tables, tables_f;
+            DevBuf<double> params, grad_total, tile_sums, pen_part;
+            DevBuf<float> params_f, partial;
+        } to;
+        alloc_together(to.slab, stream, [&](auto buf) {
+            buf(to.params, np);
+            buf(to.params_f, np);
+            buf(to.grad_total, np);
+            buf(to.tables, blob.size());
+            buf(to.partial, part);
+            buf(to.tile_sums, std::max<size_t>(sums, plain_blocks) * 5);
+            buf(to.pen_part, size_t(gather_blocks(sizes)) + 1);
         });
-        axis_tables.upload(blob, stream);
-        for (int k = 0; k < d.dim; ++k) ax[k].base = axis_tables.p;
-        if (d.has_penalty && d.dim == 3) {
+        to.tables.upload(blob, stream);
+        to.tables_f.upload(blob_f, stream);
+
+        // nothing fails from here on
+        slab_grid.swap(to.slab);
+        params.swap(to.params);
+        params_f.swap(to.params_f);
+        grad_total.swap(to.grad_total);
+        axis_tables.swap(to.tables);
+        axis_tables_f.swap(to.tables_f);
+        partial.swap(to.partial);
+        tile_sums.swap(to.tile_sums);
+        pen_part.swap(to.pen_part);
+        for (int k = 0; k < 3; ++k) {
+            A[k].base = axis_tables.p;
+            AF[k].base = axis_tables_f.p;
+            ax[k] = std::move(A[k]);
+            axf[k] = std::move(AF[k]);
+            nc[k] = g[k];
+            tile[k] = t[k];
+        }
+        slot = sl;
+        slot_f = sl_f;
+        ncoef = ncoefs;
+        nparams = np;
+        path = new_path;
+        if (new_grid) ptable_host = std::move(cells3);
+        penalty2_host = std::move(cells2);
+        if (d.has_penalty && D == 3) {
             ptable.borrow(axis_tables.p + at_pen[0], ptable_host.size());
         } else if (d.has_penalty) {
             pen_rowptr.borrow(axis_tables.p + at_pen[0], penalty2_host->rowptr.size());
             pen_col.borrow(axis_tables.p + at_pen[1], penalty2_host->col.size());
             pen_val.borrow(axis_tables.p + at_pen[2], penalty2_host->val.size());
         }
-        tables_valid = true;
     }
 
     // counters and scalars, zero; means of the images

@@ -105,3 +105,77 @@ def test_every_allocation_failure_is_reported_and_the_library_stays_usable(name)
         L.mgr_debug_fail_allocation(0)
     assert failures > 0
     assert _same(run(), want)
+
+
+def _changes():
+    """name: (level arguments, first grid, the change)"""
+    def other_tile(lv, tiles):
+        lv.set_path("split", [t for t in tiles if t != lv.tile[:len(t)]][0])
+
+    return {
+        "grid3d": (dict(size=(22, 18, 14), cost="ssd"), (8, 7, 6), lambda lv: lv.set_grid((15, 12, 10))),
+        "grid2d": (dict(size=(48, 40), cost="ncc"), (9, 8), lambda lv: lv.set_grid((20, 17))),
+        "tile3d": (dict(size=(40, 20, 36), cost="ncc"), (8, 7, 6), lambda lv: other_tile(lv, [(32, 8, 4), (32, 8, 8)])),
+        "tile2d": (dict(size=(80, 70), cost="ssd"), (9, 8), lambda lv: other_tile(lv, [(64, 8), (32, 32)])),
+        "fused": (dict(size=(40, 20, 36), cost="ssd"), (8, 7, 6), lambda lv: lv.set_path("fused")),
+    }
+
+
+@pytest.mark.parametrize("name", ["grid3d", "grid2d", "tile3d", "tile2d", "fused"])
+def test_a_change_without_memory_leaves_the_level_as_it_was(name):
+    """set_grid and set_path on a level in use, each of their allocations
+    failed in turn: the level keeps its grid and tile and gives the values it
+    gave, bit for bit, also with a second level made in between (which would
+    get memory that the first had given up); the same change without a
+    failure then gives what it gives a fresh level."""
+    import mia_gb300 as M
+    from mia_gb300 import _lib
+    from mia_gb300 import synth
+    L = _lib.lib()
+    kw, grid, change = _changes()[name]
+    size, cost = kw["size"], kw["cost"]
+    ref = synth.blob_phantom(size[::-1], 6, sigma=(3.0, 8.0), seed=2)
+    mov = np.roll(ref, 1, axis=-1)
+
+    def make():
+        lv = M.Level(size, csize=grid, cost=cost, penalty_weight=2.0)
+        lv.set_images(mov, ref)
+        return lv
+
+    def values(lv):
+        p = synth.smooth_params(lv.csize, 0.8, seed=4)
+        v = lv.value(p)
+        _, f = lv.force(p)
+        return [*lv.evaluate(p), v[0], v[1], lv.warp(p), f, lv.translate(f)]
+
+    fresh = make()
+    before = values(fresh)
+    change(fresh)
+    after = values(fresh)
+    fresh.close()
+    lv = make()
+    tile = lv.tile
+    values(lv)
+    failures = 0
+    try:
+        for k in range(1, 50):
+            _lib.check(L.mgr_debug_fail_allocation(k))
+            try:
+                change(lv)
+                break
+            except _lib.MgrError as e:
+                assert e.status == _lib.MGR_ERR_OOM, (k, e.status, str(e))
+                failures += 1
+            finally:
+                _lib.check(L.mgr_debug_fail_allocation(0))
+            assert lv.csize == grid and lv.tile == tile
+            other = make()
+            assert _same(values(lv), before) and _same(values(other), before), k
+            other.close()
+        else:
+            pytest.fail("more than 50 allocations")
+    finally:
+        L.mgr_debug_fail_allocation(0)
+    assert failures > 0
+    assert _same(values(lv), after)
+    lv.close()
