@@ -975,10 +975,10 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                     // sizes; the coefficients of the pass-0 result (r.x) are
                     // refined on the device for all growing pairs at once and
                     // stay there for the next pass (the host copy is only
-                    // resized: the pass's readback refreshes it).  Grids
-                    // with an axis of fewer than 4 coefficients are refined
-                    // on the host.
-                    // The refined parameters go to one buffer, pair after pair.
+                    // resized: the pass's readback refreshes it).  (No
+                    // level has an axis of fewer than 4 coefficients: its
+                    // creation refuses them.)  The refined parameters go to
+                    // one buffer, pair after pair.
                     std::vector<RefineJobSpec> jobs;
                     std::vector<std::array<int, 3>> grown(pairs.size());
                     size_t total = 0;
@@ -993,7 +993,6 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                     }
                     auto xnew = std::make_shared<DevBuf<double>>();
                     xnew->alloc(total, st);
-                    std::vector<std::vector<double>> on_host;   // kept until the stream has been waited for
                     size_t at = 0;
                     for (size_t i = 0; i < pairs.size(); ++i) {
                         PairRun &r = *pairs[i];
@@ -1001,24 +1000,15 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                         const int *ncn = grown[i].data();
                         double *const to = xnew->p + at;
                         const size_t n = size_t(ncn[0]) * ncn[1] * ncn[2] * dim;
-                        bool small = false;
-                        for (int k = 0; k < dim; ++k) small |= r.csize[k] < 4 || ncn[k] < 4;
-                        if (small) {
-                            refine_params(dim, r.csize, ncn, r.params);
-                            on_host.push_back(r.params);
-                            ck(cudaMemcpyAsync(to, on_host.back().data(), n * sizeof(double), cudaMemcpyHostToDevice, st),
-                               "refined parameters");
-                        } else {
-                            RefineJobSpec j;
-                            for (int k = 0; k < 3; ++k) {
-                                j.nc_old[k] = r.csize[k];
-                                j.nc_new[k] = ncn[k];
-                            }
-                            j.in = r.x;
-                            j.out = to;
-                            jobs.push_back(j);
-                            r.params.resize(n);
+                        RefineJobSpec j;
+                        for (int k = 0; k < 3; ++k) {
+                            j.nc_old[k] = r.csize[k];
+                            j.nc_new[k] = ncn[k];
                         }
+                        j.in = r.x;
+                        j.out = to;
+                        jobs.push_back(j);
+                        r.params.resize(n);
                         at += n;
                     }
                     if (!jobs.empty()) refine_params_device(dim, jobs, st);
