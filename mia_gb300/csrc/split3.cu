@@ -119,6 +119,7 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
     __shared__ unsigned rdone[NPAIR];     // warps done with the slots' current planes
     __shared__ int nissued;               // pairs of planes whose copies were issued
     __shared__ volatile int ring_failed;  // a wait of this block gave up
+    __shared__ int launch_failed;         // one of this launch had, when this block started
     const Axis &X = a.ax[0], &Y = a.ax[1], &Z = a.ax[2];
     const int nx = a.n[0], ny = a.n[1], nz = a.n[2];
     const int x0 = bx * TX3, y0 = by * TY3, z0 = bz * TZ;
@@ -189,6 +190,9 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             rdone[k] = 0;
         }
         ring_failed = 0;
+        // (read once: another block may raise it meanwhile, and all threads
+        // of this one take the same way)
+        launch_failed = *(volatile unsigned *)&a.counters[6] != 0u;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
@@ -304,7 +308,7 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
         // afterwards), later blocks read their taps from global memory, so
         // that a stalled copy engine costs one wait limit per launch, not
         // one per block
-        bool ok = a.has_tmap != 0 && *(volatile unsigned *)&a.counters[6] == 0u && (smem_u32(sm3) & 127u) == 0u;
+        bool ok = a.has_tmap != 0 && launch_failed == 0 && (smem_u32(sm3) & 127u) == 0u;
         float m = 0.0f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -437,6 +441,9 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
                     ring_failed = 1;
                     atomicOr(&a.counters[6], 1u);
                 }
+                // lanes of this warp whose waits did not give up walk on, and
+                // wait for this one wherever they release planes
+                for (; t < ez && t + RING_N < nplanes; t += 2) __syncwarp();
                 break;
             }
             const float2x px = pack2(px0 - ua0, px0 - ub0), py = pack2(py0 - ua1, py0 - ub1);
