@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(PF_NT, PF_MINB) k_prefilter_x(PrefilterPass a)
             mx = fmaxf(mx, wmm[k].y);
         }
         if (0.0f < mn) mn = 0.0f;
+        if (mx < mn) mx = mn;   // an image of NaN alone: its samples are the lower bound
         a.minmax[0] = mn;
         a.minmax[1] = mx;
         *a.counter = 0;

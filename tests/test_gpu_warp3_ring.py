@@ -68,3 +68,35 @@ def test_displacements_that_are_not_numbers(value):
         cost.append(d_c.cpu().numpy()[0])
     assert np.isfinite(cost[0])
     assert abs(cost[1] - cost[0]) <= 1e-5 * cost[0]
+
+
+@pytest.mark.parametrize("hole", ["all", "one"])
+def test_a_moving_image_that_is_not_a_number(hole):
+    """the device entry point takes images as they are: voxels without a
+    value are sampled as the lower bound of the clamp (at most 0), in the
+    ring as in the plain path, also where the image has no value at all"""
+    import torch
+
+    import mia_gb300 as M
+    from mia_gb300 import synth
+    size = (70, 20, 24)
+    rng = np.random.default_rng(8)
+    mov, ref = rng.uniform(1.0, 2.0, (2, *size[::-1])).astype(np.float32)
+    if hole == "all":
+        mov[:] = np.nan
+    else:
+        mov[7, 9, 30] = np.nan
+    d_mov, d_ref = torch.from_numpy(mov).cuda(), torch.from_numpy(ref).cuda()
+    lv = M.Level(size, rate=6.0, cost="ssd")
+    torch.cuda.synchronize()
+    lv.set_images_device(d_mov.data_ptr(), d_ref.data_ptr())
+    p = synth.smooth_params(lv.csize, 1.0, seed=2)
+    warped, cost = [], []
+    for path in ("plain", "split"):
+        lv.set_path(path)
+        cost.append(lv.evaluate(p)[0])
+        warped.append(lv.warp(p))
+    assert np.isfinite(cost[0]) and abs(cost[1] - cost[0]) <= 1e-5 * cost[0]
+    np.testing.assert_array_equal(warped[1], warped[0])
+    if hole == "all":
+        assert np.all(warped[1] == 0.0)
