@@ -251,12 +251,13 @@ unsigned long long mgr_allocation_count(void) { return g_allocs.load(); }
 
 mgr_status mgr_level_create(const mgr_level_desc *desc, int device, void *stream, mgr_level **out)
 {
-    return level_create(desc, device, stream, nullptr, out);
+    return level_create(desc, device, stream, nullptr, false, out);
 }
 
 }  // extern "C"
 
-mgr_status mgr::level_create(const mgr_level_desc *desc, int device, void *stream, const int *tile, mgr_level **out)
+mgr_status mgr::level_create(const mgr_level_desc *desc, int device, void *stream, const int *tile, bool strict,
+                             mgr_level **out)
 {
     if (!desc || !out) return fail(MGR_ERR_ARG, "null argument");
     *out = nullptr;
@@ -286,7 +287,7 @@ mgr_status mgr::level_create(const mgr_level_desc *desc, int device, void *strea
             }
         }
         L->N = size_t(L->n[0]) * L->n[1] * L->n[2];
-        if (tile && L->tile_fits(L->nc, tile, false))
+        if (tile && L->tile_fits(L->nc, tile, strict))
             for (int k = 0; k < 3; ++k) L->tile[k] = tile[k];
         else
             L->choose_tile(L->nc, L->tile);

@@ -910,7 +910,7 @@ mgr_status register_batch(int npairs, const mgr_level_desc *descs, int levels, c
                         }
                         mgr_level *L = nullptr;
                         const int *tile = level_tile[shift].data();
-                        ckm(level_create(&d, device, sp, tile, &L));
+                        ckm(level_create(&d, device, sp, tile, false, &L));
                         r.made[shift] = L;
                         // (a tile that level_create has not taken is refused here)
                         ckm(mgr_level_set_path(L, MGR_PATH_SPLIT, tile[0], tile[1], tile[2]));

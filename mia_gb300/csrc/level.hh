@@ -515,9 +515,10 @@ inline void registration_tile(int dim, int t[3])
     t[1] = dim == 3 ? 8 : 16;
     t[2] = dim == 3 ? 16 : 1;
 }
-// mgr_level_create, with the split path's tile when tile is given (and
-// fits: else the level keeps the one it would choose)
-mgr_status level_create(const mgr_level_desc *desc, int device, void *stream, const int *tile, mgr_level **out);
+// mgr_level_create, with the split path's tile when tile is given (and fits,
+// by the strict rule or not: else the level keeps the one it would choose)
+mgr_status level_create(const mgr_level_desc *desc, int device, void *stream, const int *tile, bool strict,
+                        mgr_level **out);
 // mgr_level_set_images_device without the final stream synchronisation
 void level_set_images_async(mgr_level *L, const float *d_src, const float *d_ref);
 // a new coefficient grid (and tile) on a level, images kept

@@ -95,9 +95,8 @@ double register_pair_device(const mgr_level_desc &full, int levels, const mgr_mi
             LevelHandle lv;
             int t[3];
             registration_tile(dim, t);
-            ckm(level_create(&d, device, st, nullptr, &lv.h));
-            if (lv.h->tile_fits(lv.h->nc, t)) ckm(mgr_level_set_path(lv.h, path, t[0], t[1], t[2]));
-            else ckm(mgr_level_set_path(lv.h, path, 0, 0, 0));
+            ckm(level_create(&d, device, st, t, true, &lv.h));
+            ckm(mgr_level_set_path(lv.h, path, 0, 0, 0));   // (the tile it was created with)
             level_set_images_async(lv.h, to[0], to[1]);
             tr_lvl.stop();
             TraceScope tr_min("pair: minimizer", st);
