@@ -461,7 +461,6 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
     std::vector<int2> titems, gitems;
     std::vector<int> nblocks(np);
     size_t sm_warp = 0, sm_adj = 0, max_params = 0;
-    int has_pen = 0;
     const int cost = pairs[members[0]]->full.cost;   // (the same for all pairs of a batch)
     // the pairs' parameters: in the refine pass in place, else one upload
     std::vector<size_t> off(np + 1, 0);
@@ -509,7 +508,6 @@ void run_pass(std::vector<std::unique_ptr<PairRun>> &pairs, const mgr_minimizer_
         for (int q = 0; q < nblocks[k]; ++q) gitems.push_back(make_int2(k, q));
         sm_warp = std::max(sm_warp, split_smem(a, 0));
         sm_adj = std::max(sm_adj, split_smem(a, 1));
-        has_pen |= a.has_penalty;
         max_params = std::max(max_params, n);
     }
     if (std::max(sm_warp, sm_adj) > 200 * 1024)

@@ -303,7 +303,6 @@ struct mgr_level {
         a.pen_grad_w = (d.pen_corrected ? 1.0 : -1.0) * a.pen_weight;
         a.pen_grad_wf = float(a.pen_grad_w);
         a.cost_wf = float(a.cost_weight);
-        a.pen_equal_w = d.pen_div == d.pen_curl;
         a.ptable = ptable.p;
         a.pen_rowptr = pen_rowptr.p;
         a.pen_col = pen_col.p;

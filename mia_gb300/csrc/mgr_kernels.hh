@@ -86,7 +86,6 @@ struct EvalArgs {
     // the gather's weights as float (3D; FP64 instructions are slow)
     float pen_grad_wf;     // pen_grad_w
     float cost_wf;         // cost_weight
-    int pen_equal_w;       // div == curl (multiply skips the cross terms)
     const float *ptable;   // 3D: 9x9x9 cells x 6 floats (xx, xy, yy, yz, zz, xz)
     const int *pen_rowptr; // 2D: CSR rows of the boundary-clipped matrix
     const int *pen_col;
