@@ -336,15 +336,28 @@ def final_cost_report(res, plain_out, oracle):
             in_b += db <= 1e-4 * abs(fo) or abs(r[2] - f64) <= 1e-4 * abs(f64)
             per.append({"pair": k, "batched": r[2], "plain": q[2], "oracle": fo, "oracle_f64": f64,
                         "oracle_perturbation_spread": spread, "batched_rel": db / abs(fo),
-                        "batched_rel_vs_f64": abs(r[2] - f64) / abs(f64), "plain_rel": dp / abs(fo)})
+                        "batched_rel_vs_f64": abs(r[2] - f64) / abs(f64), "plain_rel": dp / abs(fo),
+                        "of_tolerance": db / max(tol, 1e-300)})
         rep["vs_oracle"] = {"rule": "|final - oracle| <= max(1e-4 |oracle|, |oracle_f64 - oracle|, 3 x oracle spread "
                                     "under a 1e-7 perturbation of the moving image)",
                             "batched_pairs_passing": int(ok_b), "plain_pairs_passing": int(ok_p), "pairs": len(per),
                             "batched_within_1e-4_of_oracle_or_oracle_f64": int(in_b),
                             "max_batched_rel": float(max(p["batched_rel"] for p in per)),
                             "max_batched_rel_vs_f64": float(max(p["batched_rel_vs_f64"] for p in per)),
-                            "per_pair": per}
+                            # (all of them would make the line longer than what reads it keeps)
+                            "worst_pairs": sorted(per, key=lambda p: -p["of_tolerance"])[:3]}
     return rep
+
+
+def print_line(line):
+    """the result line, numbers at eight significant digits"""
+    def short(v):
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        if isinstance(v, (list, tuple)):
+            return [short(x) for x in v]
+        return float("%.8g" % v) if isinstance(v, float) else v
+    print(json.dumps(short(line)))
 
 
 def measure_batch(name, steps, warmup, device, cpu_seconds=0.0, clocks=None, profile_region=False,
@@ -524,7 +537,7 @@ def run_batch(args):
     line.update({k: v for k, v in r.items() if k not in ("value", "unit", "ms_per_step")})
     line["timing"] = "wall clock of the whole batched registration, device synchronised on both sides"
     line["clocks"] = clk.summary()
-    print(json.dumps(line))
+    print_line(line)
     return 0
 
 
@@ -559,7 +572,7 @@ def run_reference(args):
                          "sample": "%d full evaluations of %s" % (args.steps, "x".join(map(str, size)))},
         "e2e": {"value": v, "unit": "Mvoxel/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
-    print(json.dumps(line))
+    print_line(line)
     return 0
 
 
@@ -584,7 +597,7 @@ def run_reference_batch(args):
             "cpu_baseline": {"value": v, "unit": "pairs/s", "cores": threads, "kind": "port",
                              "sample": "%d pair registrations, %.1f s per step at most" % (counts, per_step)},
             "e2e": {"value": v, "unit": "pairs/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line))
+    print_line(line)
     return 0
 
 
@@ -759,7 +772,7 @@ def run_gpu(args):
             r["clocks"] = bclk.summary()
             r["steps"], r["warmup"] = 3, 2
             line["batched"][bname] = r
-    print(json.dumps(line))
+    print_line(line)
     return 0
 
 
