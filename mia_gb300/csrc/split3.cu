@@ -559,6 +559,11 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
                 break;
             }
     }
+    // a persistent block's next item initialises the barriers again, for which
+    // they have to be invalidated first
+    if (BATCH && tid == 0)
+        for (int k = 0; k < NPAIR; ++k)
+            asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&mbar[k])) : "memory");
     if (tid < 5) {
         double v = 0.0;
         if (tid < ncomp)
