@@ -503,11 +503,12 @@ struct mgr_level {
 namespace mgr {
 // The tile of the registration drivers' split path, per pair (register.cu)
 // and batched (batch.cu), so that both run the same kernels in the same
-// order: 32x8x16 in 3D, 32x16 in 2D.  The autotuner's table times single
-// evaluations, where the tile sets the latency of one launch; in the batch
-// every launch carries all pairs and the deeper tile's lower per-item
-// overhead wins (60-frame 2D series: 1733-1778 pairs/s with 32x16 against
-// 1389-1415 with the tuned 32x8; the 3D cohort the same either way).
+// order: 32x8x16 in 3D, 32x16 in 2D (but for the last bits of a 3D SSD tile
+// that does not fit the tap ring, warp3_body's BATCH).  The autotuner's table
+// times single evaluations, where the tile sets the latency of one launch; in
+// the batch every launch carries all pairs and the deeper tile's lower
+// per-item overhead wins (60-frame 2D series: 1733-1778 pairs/s with 32x16
+// against 1389-1415 with the tuned 32x8; the 3D cohort the same either way).
 inline void registration_tile(int dim, int t[3])
 {
     t[0] = 32;

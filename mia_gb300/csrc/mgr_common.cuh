@@ -226,7 +226,9 @@ __device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c)
 // (at once for a kernel launched without the attribute).  Before it a kernel
 // reads only the level's fixed tables.  pdl_trigger, issued by every block
 // after its pdl_wait, lets the next kernel be launched: so no kernel starts
-// before the one two places back in the stream has completed.
+// before the one two places back in the stream has completed.  A kernel that
+// triggers without a wait (the parameters' conversion) must be launched
+// without the attribute, in plain stream order.
 __device__ __forceinline__ void pdl_wait()
 {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");

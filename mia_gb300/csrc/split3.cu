@@ -30,7 +30,7 @@
 //       and y in shared memory (the reference contracts y before x; the
 //       order changes only the rounding, and x first keeps the intermediate
 //       small); the result goes to the tile's partial slot (no atomics).
-//   k_gather3         per 4x4x4 block of coefficients: the fixed-order sum of
+//   k_gather3         per 4x4x2 block of coefficients: the fixed-order sum of
 //       the partial slots that hold each coefficient, the divcurl stencil
 //       (C3DPPDivcurlMatrixImpl::evaluate / multiply,
 //       mia/3d/ppmatrix.cc:292-599) over a shared-memory copy of the
@@ -1079,7 +1079,7 @@ __device__ __forceinline__ void gather3_body(const EvalArgs &a, int with_gradien
     pacc[w][11][lane] = S2;
     __syncthreads();
     // the warps' partials of each quantity summed in a fixed order (FP32,
-    // warp k % GSUB sums quantity k into row 0), then warp 0 combines them
+    // warp k % GSUB sums quantity k into row 0), which the warps below combine
     // (the outputs are widened to double at the store)
     for (int k = w; k < GNQ; k += GSUB) {
         float t = pacc[0][k][lane];
@@ -1320,7 +1320,9 @@ __global__ void MGR_GATHER_BOUNDS k_gather3_batch(const EvalArgs *__restrict__ a
 
 // float copy of the parameters (the warp and gather kernels read them as
 // float, as the reference's spline evaluation does; FP64 conversions are
-// slow on this GPU, so they are done once per evaluation)
+// slow on this GPU, so they are done once per evaluation).  It and
+// k_params_host let the next kernel start without a wait of their own: they
+// are only ever launched in plain stream order (launch_params_f32).
 __global__ void __launch_bounds__(256) k_params_f32(const double *__restrict__ p, float *__restrict__ f, size_t n)
 {
     pdl_trigger();   // the warp kernel may start its set-up (it waits for this kernel)

@@ -100,3 +100,25 @@ def test_a_moving_image_that_is_not_a_number(hole):
     np.testing.assert_array_equal(warped[1], warped[0])
     if hole == "all":
         assert np.all(warped[1] == 0.0)
+
+
+@pytest.mark.parametrize("size", [(40, 24, 20), (70, 33, 21), (36, 41, 50)])
+def test_batch_and_single_sums_of_tiles_outside_the_ring(size):
+    """Images whose last x tile is narrow: its box leaves the padded copy, so
+    its planes are sampled after the walk, and a batch adds their squares
+    rounded, a single evaluation does not.  Over one minimizer step from the
+    same start both take the same step (an SSD force does not depend on the
+    sum), so the parameters have the same bits; each sum is off by at most 16
+    additions per thread and 5 tree levels of 2^-24 relative (all terms are
+    positive), so the costs differ by at most 2 * 22 * 2^-24."""
+    from mia_gb300 import registration as R
+    from mia_gb300 import synth
+    ref = synth.blob_phantom(size[::-1], 8, sigma=(3.0, 6.0), seed=6)
+    mov = np.roll(ref, 1, axis=2).astype(np.float32)
+    mz = R.minimizer("gsl", maxiter=1, step=0.1)
+    kw = dict(cost="ssd", penalty_weight=1.0)
+    one = R.register_pair(mov, ref, 6.0, 1, mz, path="split", **kw)
+    both = R.register_batch([(mov, ref), (mov, ref)], 6.0, 1, mz, **kw)
+    for b in both:
+        np.testing.assert_array_equal(b[0], one[0])
+        assert b[3] == one[3] and abs(b[2] - one[2]) <= 44 * 2.0 ** -24 * abs(one[2])
