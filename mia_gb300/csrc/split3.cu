@@ -147,6 +147,10 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
     // the parameters' float copy comes from the kernel before this one
     pdl_wait();
     pdl_trigger();
+    // whether a wait of this launch has given up (read once: another block may
+    // raise the flag meanwhile, and all threads of this one take the same way)
+    unsigned flag = 0u;
+    if (tid == 0) flag = *(volatile unsigned *)&a.counters[6];
     float *C = sm3 + RING_N * RING_PLANE;  // [3][FZ][FY][FX]
     float *Tx = C + 3 * FZ * FY * FX;      // [3][FZ][FY][32]
     // coefficient footprint: rows (iz, iy) of 3 FX consecutive floats
@@ -190,9 +194,7 @@ __device__ __forceinline__ void warp3_body(const EvalArgs &a, int bx, int by, in
             rdone[k] = 0;
         }
         ring_failed = 0;
-        // (read once: another block may raise it meanwhile, and all threads
-        // of this one take the same way)
-        launch_failed = *(volatile unsigned *)&a.counters[6] != 0u;
+        launch_failed = flag != 0u;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
