@@ -104,7 +104,8 @@ mgr_status mgr_level_csize(const mgr_level *lvl, int csize[3], size_t *nparams);
    keeps for the next level's size (:399-412, before that level's
    set_size).  A grid equal to the current one changes nothing.  Returns
    after the rebuild; parameters and gradients of later calls have the new
-   size. */
+   size.  A call that fails (MGR_ERR_OOM, for instance) leaves the level with
+   the grid it had. */
 mgr_status mgr_level_set_grid(mgr_level *lvl, const int csize[3]);
 
 /* Replaces: C3DImageFullCost::do_reinit + TCost::set_reference
@@ -166,7 +167,8 @@ mgr_status mgr_level_force(mgr_level *lvl, const double *params, float *force,
 mgr_status mgr_level_translate(mgr_level *lvl, const float *force, double *grad);
 
 /* Select the evaluation strategy (MGR_PATH_*) and, for MGR_PATH_SPLIT, the
-   tile shape (0 = autotuned default).  Compiled shapes: 3D 32 x 8 x TZ with
+   tile shape (0 = the level's present one; MGR_ERR_OOM leaves the level as
+   it was).  Compiled shapes: 3D 32 x 8 x TZ with
    TZ in {4, 8, 12, 16, 20, 24, 32}; 2D 32 x 8, 32 x 16, 64 x 8, 64 x 16,
    32 x 32; any other shape is MGR_ERR_ARG.  Has no counterpart in the
    reference: it chooses between implementations of the same result. */

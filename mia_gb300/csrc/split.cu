@@ -26,7 +26,8 @@
 // the other end: there the warp kernel's FP64 sums and the adjoint kernel's
 // shared-memory reads were the time; with four threads per sum, component
 // pairs and whole lines per thread 26 -> 22 and 15.7 -> 11.6 us, evaluations
-// one after another 26.6 -> 21.9 us (96x96 SSD 30.7 -> 30.1).
+// one after another 26.6 -> 21.9 us (96x96 SSD 30.7 -> 30.1); the adjoint's
+// voxel ranges from a table instead of two dependent loads 21.8 -> 21.4 us.
 #include "mgr_cost.cuh"
 #include "mgr_launch.hh"
 
