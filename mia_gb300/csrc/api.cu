@@ -72,15 +72,20 @@ void raise_smem_limit(const void *kernel, size_t bytes)
     int device = 0;
     cudaGetDevice(&device);
     std::lock_guard<std::mutex> lk(mu);
+    Limit *have = nullptr;
     for (auto &l : set)
-        if (l.kernel == kernel && l.device == device) {
-            if (l.bytes >= bytes) return;
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-            l.bytes = bytes;
-            return;
-        }
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-    set.push_back({kernel, device, bytes});
+        if (l.kernel == kernel && l.device == device) have = &l;
+    if (have && have->bytes >= bytes) return;
+    // a size that no block can have: reported here, as a later successful call
+    // would clear the error, and not noted, so that the kernel's later
+    // launches raise the limit as far as they need
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        ck(e, "shared memory of a block");
+    }
+    if (have) have->bytes = bytes;
+    else set.push_back({kernel, device, bytes});
 }
 
 // phase trace (MGR_TRACE=1)
@@ -422,17 +427,26 @@ static void evaluate_in_place(mgr_level *L, const double *params, bool with_grad
     a.params_host = params;
     double *hc = L->host_small();
     a.host_out = hc;
-    if (with_gradient) {
-        if (grad_total) a.grad_total = grad_total;
-        a.grad_image = grad_image;
-        a.grad_penalty = grad_penalty;
-        run_image_term(L, a, true);
-    } else {
-        a.defer_cost = L->can_defer();
-        launch_warp(a, L->stream);
-        launch_gather(a, 0, L->stream);
+    try {
+        if (with_gradient) {
+            if (grad_total) a.grad_total = grad_total;
+            a.grad_image = grad_image;
+            a.grad_penalty = grad_penalty;
+            run_image_term(L, a, true);
+        } else {
+            a.defer_cost = L->can_defer();
+            launch_warp(a, L->stream);
+            launch_gather(a, 0, L->stream);
+        }
+        check_launch("evaluate kernels");
+    } catch (...) {
+        // what was queued before a launch that failed reads the caller's
+        // memory: not after this call; the gather, which would have cleared
+        // the flag of non-finite parameters, has not run
+        cudaMemsetAsync(L->counters.p + 7, 0, sizeof(unsigned), L->stream);
+        cudaStreamSynchronize(L->stream);
+        throw;
     }
-    check_launch("evaluate kernels");
     ck(cudaStreamSynchronize(L->stream), "evaluate sync");
     unsigned flags[2];
     std::memcpy(flags, hc + 2, sizeof flags);

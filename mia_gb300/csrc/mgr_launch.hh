@@ -3,11 +3,15 @@
 
 #include <cuda_runtime.h>
 
+#include <stdexcept>
+#include <string>
+
 namespace mgr {
 
 // A launch that may start while the kernel before it in the stream is still
 // running (the kernel waits in pdl_wait before it reads that kernel's
-// outputs), or a plain stream-ordered launch.
+// outputs), or a plain stream-ordered launch.  A launch that fails is reported
+// at once: no kernel after it runs on what it would have written.
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                        Args... args)
@@ -22,7 +26,11 @@ inline void launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        throw std::runtime_error(std::string("kernel launch: ") + cudaGetErrorString(e));
+    }
 }
 
 }  // namespace mgr

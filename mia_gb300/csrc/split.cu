@@ -529,8 +529,9 @@ static void launch_batch_tile(const EvalArgs *args, const int2 *items, int nitem
 template <int TX, int TY>
 static void prepare_batch_tile(size_t sm_warp, size_t sm_adj)
 {
-    cudaFuncSetAttribute(k_warp2_batch<TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_warp));
-    cudaFuncSetAttribute(k_adjoint2_batch<TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm_adj));
+    // (only ever raised: another thread's batch may be running with more)
+    raise_smem_limit(reinterpret_cast<const void *>(k_warp2_batch<TX, TY>), sm_warp);
+    raise_smem_limit(reinterpret_cast<const void *>(k_adjoint2_batch<TX, TY>), sm_adj);
 }
 
 void prepare_split_batch(int dim, int cost, int tx, int ty, int tz, size_t sm_warp, size_t sm_adj)
