@@ -744,9 +744,6 @@ mgr_status mgr_level_set_path(mgr_level *lvl, int path, int tile_x, int tile_y, 
             if (lvl->d.dim != 3 || lvl->d.cost != MGR_COST_SSD)
                 throw std::invalid_argument("the fused path evaluates 3D SSD only");
             if (lvl->images_from) throw StateError("the fused path needs the level's own images");
-            for (int k = 0; k < 3; ++k)
-                if (lvl->nc[k] - 3 > lvl->n[k] - 1)
-                    throw std::invalid_argument("the fused path needs a coefficient spacing of at least one voxel");
         }
         // the shape is checked before anything changes: a refused call
         // leaves the level as it was

@@ -25,6 +25,7 @@
 // image's sums (mia/3d/cost/ncc.cc:88-128), which a single pass only knows
 // when every tile has finished.
 #include <algorithm>
+#include <stdexcept>
 #include <string>
 
 #include "../../include/mgr.h"
@@ -506,11 +507,6 @@ size_t fused3_smem(const EvalArgs &a)
     return (az + std::max(walk, ay)) * sizeof(float);
 }
 
-bool tile_supported_fused3(int tx, int ty, int tz)
-{
-    return tx == FTX && ty == FTY && (tz == 4 || tz == 8 || tz == 16 || tz == 32);
-}
-
 namespace {
 template <int TZ>
 void launch_fused3_z(const EvalArgs &a, int with_gradient, size_t sm, cudaStream_t st)
@@ -524,11 +520,16 @@ void launch_fused3(const EvalArgs &a, int with_gradient, cudaStream_t st)
 {
     launch_params_f32(a, st);
     const size_t sm = fused3_smem(a);
+    // (the tables are made for this length: no other kernel may run on them)
     switch (a.ax[2].t) {
     case 4: launch_fused3_z<4>(a, with_gradient, sm, st); break;
     case 8: launch_fused3_z<8>(a, with_gradient, sm, st); break;
+    case 12: launch_fused3_z<12>(a, with_gradient, sm, st); break;
+    case 16: launch_fused3_z<16>(a, with_gradient, sm, st); break;
+    case 20: launch_fused3_z<20>(a, with_gradient, sm, st); break;
+    case 24: launch_fused3_z<24>(a, with_gradient, sm, st); break;
     case 32: launch_fused3_z<32>(a, with_gradient, sm, st); break;
-    default: launch_fused3_z<16>(a, with_gradient, sm, st); break;
+    default: throw std::invalid_argument("fused kernel: z tile not compiled in");
     }
     count_launch();
 }

@@ -406,6 +406,10 @@ struct mgr_level {
         const int ntiles = build_axis_set(g, t, A, blob, sl);
         size_t part = size_t(ntiles) * sl, sums = size_t(ntiles);
         if (new_path == MGR_PATH_FUSED) {
+            // (its footprints count on it)
+            for (int k = 0; k < D; ++k)
+                if (g[k] - 3 > n[k] - 1)
+                    throw std::invalid_argument("the fused path needs a coefficient spacing of at least one voxel");
             // the fused kernel's tile: 30 interior voxels in x (32 lanes with
             // the halo), 8 rows, the level's z tile
             const int tf[3] = {30, 8, t[2]};

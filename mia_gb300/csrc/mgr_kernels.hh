@@ -155,7 +155,6 @@ void launch_split3_queue(int cost, const EvalArgs *args, const int2 *items, int 
                          int grid, size_t sm, int which, bool pdl, cudaStream_t st);
 // the fused SSD kernel (fused3.cu): warp, force and adjoint in one pass per
 // 30 x 8 x TZ tile; with_gradient = 0 sums the cost only
-bool tile_supported_fused3(int tx, int ty, int tz);
 size_t fused3_smem(const EvalArgs &a);
 void launch_fused3(const EvalArgs &a, int with_gradient, cudaStream_t st);
 int gather3_blocks(const EvalArgs &a);

@@ -81,3 +81,51 @@ def test_fused_path_is_3d_ssd_only():
     lv2 = M.Level((64, 48), rate=4.0)
     with pytest.raises(_lib.MgrError):
         lv2.set_path("fused")
+
+
+@pytest.mark.parametrize("tz", [4, 8, 12, 16, 20, 24, 32])
+@pytest.mark.parametrize("size,rate", [((49, 10, 25), (9.99, 6.67, 3.97)), ((61, 37, 70), 5.0)])
+def test_every_z_tile_of_the_level(size, rate, tz):
+    """the fused kernel with each z tile that a level can have, the lengths
+    between the powers of two included (partial last tiles, one plane)"""
+    import mia_gb300 as M
+    from mia_gb300 import synth
+    mov, ref = _pair(size[::-1], seed=7)
+    kw = dict(rate=rate, cost="ssd", penalty_weight=1.0)
+    lv = M.Level(size, **kw)
+    lv.set_images(mov, ref)
+    o = O.Level(size, precision=O.PREC_F64, **kw)
+    o.set_images(mov, ref)
+    p = synth.smooth_params(lv.csize, 1.5, seed=3)
+    lv.set_path("split", (32, 8, tz))
+    lv.set_path("fused")
+    assert lv.tile[2] == tz
+    ci, cp, gi, gp, _ = lv.evaluate(p)
+    oi, op, ogi, ogp = o.evaluate(p)
+    assert _rel(ci, oi) <= 1e-5 and _rel(cp, op) <= 1e-5
+    assert _rel_l2(gi, ogi) <= 1e-4 and _rel_l2(gp, ogp) <= 1e-4
+    lv.close()
+
+
+def test_a_fused_level_refuses_a_grid_finer_than_the_voxels():
+    import mia_gb300 as M
+    from mia_gb300 import _lib
+    from mia_gb300 import synth
+    size = (40, 24, 20)
+    mov, ref = _pair(size[::-1], seed=2)
+    lv = M.Level(size, csize=(9, 8, 7), cost="ssd")
+    lv.set_images(mov, ref)
+    lv.set_path("fused")
+    p = synth.smooth_params(lv.csize, 1.0, seed=1)
+    want = lv.evaluate(p)
+    with pytest.raises(_lib.MgrError) as e:
+        lv.set_grid((9, 8, 23))   # 20 intervals on 19
+    assert e.value.status == _lib.MGR_ERR_ARG and lv.csize == (9, 8, 7)
+    for x, y in zip(lv.evaluate(p), want):
+        np.testing.assert_array_equal(x, y)
+    lv.set_grid((9, 8, 22))
+    q = synth.smooth_params(lv.csize, 1.0, seed=2)
+    fused = lv.evaluate(q)
+    lv.set_path("split")
+    assert _rel(lv.evaluate(q)[0], fused[0]) <= 1e-5
+    lv.close()
