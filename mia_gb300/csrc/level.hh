@@ -428,10 +428,17 @@ struct mgr_level {
             else cells2 = penalty2_cached(g, range, d.pen_div, d.pen_curl);
         }
         const std::vector<float> &p3 = new_grid ? cells3 : ptable_host;
+        // 2D cells are many on large grids (49 per coefficient, 20 bytes each):
+        // from 256 KB on they are uploaded from the cached table as it is, as
+        // packing them costs more than the three uploads it saves.  A level
+        // made with them packed / apart: 88 / 93 us at 165 KB (192x160, rate
+        // 16), 115 / 116 at 318 KB, 176 / 154 at 714 KB, 637 / 385 at 4.3 MB
+        // (1024x1024)
+        const bool apart = d.has_penalty && D == 2 && cells2->col.size() * 20 >= 256 * 1024;
         size_t at_pen[3] = {0, 0, 0};
         if (d.has_penalty && D == 3) {
             at_pen[0] = AxisDev::pack(blob, p3);
-        } else if (d.has_penalty) {
+        } else if (d.has_penalty && !apart) {
             at_pen[0] = AxisDev::pack(blob, cells2->rowptr);
             at_pen[1] = AxisDev::pack(blob, cells2->col);
             at_pen[2] = AxisDev::pack(blob, cells2->val);
@@ -443,7 +450,8 @@ struct mgr_level {
         struct {
             DevBuf<unsigned char> slab, tables, tables_f;
             DevBuf<double> params, grad_total, tile_sums, pen_part;
-            DevBuf<float> params_f, partial;
+            DevBuf<float> params_f, partial, pen_val;
+            DevBuf<int> pen_rowptr, pen_col;
         } to;
         alloc_together(to.slab, stream, [&](auto buf) {
             buf(to.params, np);
@@ -453,8 +461,16 @@ struct mgr_level {
             buf(to.partial, part);
             buf(to.tile_sums, std::max<size_t>(sums, plain_blocks) * 5);
             buf(to.pen_part, size_t(gather_blocks(sizes)) + 1);
+            buf(to.pen_rowptr, apart ? cells2->rowptr.size() : 0);
+            buf(to.pen_col, apart ? cells2->col.size() : 0);
+            buf(to.pen_val, apart ? cells2->val.size() : 0);
         });
         to.tables.upload(blob, stream);
+        if (apart) {
+            to.pen_rowptr.upload(cells2->rowptr, stream);
+            to.pen_col.upload(cells2->col, stream);
+            to.pen_val.upload(cells2->val, stream);
+        }
         to.tables_f.upload(blob_f, stream);
 
         // nothing fails from here on
@@ -482,7 +498,11 @@ struct mgr_level {
         path = new_path;
         if (new_grid) ptable_host = std::move(cells3);
         penalty2_host = std::move(cells2);
-        if (d.has_penalty && D == 3) {
+        if (apart) {
+            pen_rowptr.swap(to.pen_rowptr);
+            pen_col.swap(to.pen_col);
+            pen_val.swap(to.pen_val);
+        } else if (d.has_penalty && D == 3) {
             ptable.borrow(axis_tables.p + at_pen[0], ptable_host.size());
         } else if (d.has_penalty) {
             pen_rowptr.borrow(axis_tables.p + at_pen[0], penalty2_host->rowptr.size());
